@@ -87,6 +87,7 @@ namespace
         st |= dalloc(c, &m.ref, n);
         st |= dalloc(c, &m.hc, n);
         st |= dalloc(c, &m.hc2, n);
+        st |= dalloc(c, &m.pred, n);
         st |= dalloc(c, &m.rank, n);
         st |= dalloc(c, &m.wl_ref, n);
         st |= dalloc(c, &m.wl_cells, n);
@@ -108,6 +109,7 @@ namespace
         dfree(m.ref);
         dfree(m.hc);
         dfree(m.hc2);
+        dfree(m.pred);
         dfree(m.rank);
         dfree(m.wl_ref);
         dfree(m.wl_cells);
@@ -141,10 +143,10 @@ namespace
         {
             cudaEventDestroy(e);
         }
-        dfree(c.d_ite);
-        if (c.h_ite)
+        dfree(c.d_setup);
+        if (c.h_setup)
         {
-            cudaFreeHost(c.h_ite);
+            cudaFreeHost(c.h_setup);
         }
         free_mesh(c.mesh[0]);
         free_mesh(c.mesh[1]);
@@ -153,19 +155,16 @@ namespace
         dfree(c.t2);
         dfree(c.t3);
         dfree(c.rf);
-        dfree(c.cf);
+        for (uint32_t** bm : {&c.tk, &c.tc, &c.tr, &c.above, &c.ref_above, &c.par_above})
+        {
+            dfree(*bm);
+        }
         dfree(c.detail);
-        dfree(c.tag);
         dfree(c.block_sums);
         dfree(c.d_counts);
         dfree(c.d_flags);
-        dfree(c.d_eps);
         dfree(c.d_absmax);
         dfree(c.g.err);
-        if (c.h_eps)
-        {
-            cudaFreeHost(c.h_eps);
-        }
         dfree(h->staging);
         if (c.h_counts)
         {
@@ -404,13 +403,13 @@ extern "C"
             return fail(SG_ERR_CUDA, "sg_mesh_create: no CUDA device");
         }
         {
-            // device memory of the mesh (two meshes of 10 word arrays, 6 scratch bitmaps, the dense detail and tag
-            // slabs) and of one field with its update_fields buffer, against the free memory of the device: a
+            // device memory of the mesh (two meshes of 11 word arrays, 5 scratch and 6 tag bitmaps, the dense detail
+            // slab) and of one field with its update_fields buffer, against the free memory of the device: a
             // configuration that cannot fit is refused here rather than by a failing allocation midway
             const sg::Geom gg    = sg::make_geom(dim, min_level, max_level);
             const double words   = static_cast<double>(gg.total_words);
             const double cap     = 32.0 * words;
-            const double mesh_b  = (2.0 * 10.0 + 6.0) * 4.0 * words + 9.0 * cap;
+            const double mesh_b  = (2.0 * 11.0 + 5.0 + 6.0) * 4.0 * words + 8.0 * cap;
             const double field_b = 16.0 * cap;
             size_t free_b = 0, total_b = 0;
             if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess)
@@ -491,22 +490,22 @@ extern "C"
         st |= dalloc(c, &c.t2, nw);
         st |= dalloc(c, &c.t3, nw);
         st |= dalloc(c, &c.rf, nw);
-        st |= dalloc(c, &c.cf, nw);
+        for (uint32_t** bm : {&c.tk, &c.tc, &c.tr, &c.above, &c.ref_above, &c.par_above})
+        {
+            st |= dalloc(c, bm, nw);
+        }
         st |= dalloc(c, &c.detail, static_cast<size_t>(c.capacity));
-        st |= dalloc(c, &c.tag, static_cast<size_t>(c.capacity));
         c.n_scan_blocks = (c.g.total_words + 4095) / 4096;
         st |= dalloc(c, &c.block_sums, 4 * static_cast<size_t>(c.n_scan_blocks) + 4);
         st |= dalloc(c, &c.d_counts, static_cast<size_t>(sg::COUNTS));
         st |= dalloc(c, &c.d_flags, 8);
         st |= dalloc(c, &c.d_adapt, static_cast<size_t>(sg::A_COUNT));
-        st |= dalloc(c, &c.d_ite, 1);
-        st |= dalloc(c, &c.d_eps, sg::EPS_VELOCITY + 3);
+        st |= dalloc(c, &c.d_setup, 1);
         st |= dalloc(c, &c.d_absmax, 1);
         st |= dalloc(c, &c.g.err, 1);
         if (!st)
         {
-            if (cudaMallocHost(reinterpret_cast<void**>(&c.h_ite), sizeof(int)) != cudaSuccess
-                || cudaMallocHost(reinterpret_cast<void**>(&c.h_eps), 3 * sg::MAXLEV * sizeof(double)) != cudaSuccess
+            if (cudaMallocHost(reinterpret_cast<void**>(&c.h_setup), sizeof(sg::PassSetup)) != cudaSuccess
                 || cudaMallocHost(reinterpret_cast<void**>(&c.h_counts), sg::COUNTS * sizeof(long long)) != cudaSuccess
                 || cudaMallocHost(reinterpret_cast<void**>(&c.h_flags), 8 * sizeof(int)) != cudaSuccess
                 || cudaMallocHost(reinterpret_cast<void**>(&c.h_adapt), sg::A_COUNT * sizeof(int)) != cudaSuccess)
@@ -527,13 +526,16 @@ extern "C"
         for (int k = 0; k < 2; ++k)
         {
             sg::DeviceMesh& mk = c.mesh[k];
-            for (uint32_t* bm : {mk.cells, mk.cag, mk.proj, mk.uni, mk.ref, mk.hc, mk.hc2})
+            for (uint32_t* bm : {mk.cells, mk.cag, mk.proj, mk.uni, mk.ref, mk.hc, mk.hc2, mk.pred})
             {
                 cudaMemsetAsync(bm, 0, nw * 4, c.stream);
             }
         }
         cudaMemsetAsync(c.detail, 0, static_cast<size_t>(c.capacity) * sizeof(double), c.stream);
-        cudaMemsetAsync(c.tag, 0, static_cast<size_t>(c.capacity), c.stream);
+        for (uint32_t* bm : {c.tk, c.tc, c.tr, c.above, c.ref_above, c.par_above})
+        {
+            cudaMemsetAsync(bm, 0, nw * 4, c.stream);
+        }
         k_box_cells<<<sg::grid_for(c.g.lv[max_level].nwords), 256, 0, c.stream>>>(c.g, max_level, c.m().cells);
         st = sg::check(c, "initial cells");
         if (!st)
@@ -1437,7 +1439,8 @@ extern "C"
             // one dense detail slab per adapted field; the contents are rebuilt by every pass
             cudaStreamSynchronize(c.stream);
             dfree(c.detail);
-            if (dalloc(c, &c.detail, static_cast<size_t>(c.capacity) * static_cast<size_t>(n)))
+            dfree(c.d_absmax);
+            if (dalloc(c, &c.detail, static_cast<size_t>(c.capacity) * static_cast<size_t>(n)) || dalloc(c, &c.d_absmax, static_cast<size_t>(n)))
             {
                 c.detail_comps = 0;
                 return from_ctx(c, SG_ERR_CUDA);
@@ -1576,7 +1579,7 @@ extern "C"
         {
             return from_ctx(c, SG_ERR_CUDA);
         }
-        int st = sg::gather_compact(c, c.m(), c.detail, h->staging);
+        int st = sg::gather_details(c, c.m(), h->staging);
         if (st)
         {
             return from_ctx(c, st);
@@ -1597,7 +1600,8 @@ extern "C"
         {
             return fail(SG_ERR_ARG, "sg_tag_download: null argument");
         }
-        sg::Ctx& c = u->mesh->ctx;
+        sg_mesh_s* h = u->mesh;
+        sg::Ctx& c   = h->ctx;
         if (int st = sg::host_counts(c, c.m()))
         {
             return from_ctx(c, st);
@@ -1606,26 +1610,19 @@ extern "C"
         {
             return fail(SG_ERR_ARG, "sg_tag_download: size differs from the reference mesh");
         }
-        HostMesh hm;
-        if (int st = pull(c, c.m().ref, hm, true))
+        if (stage(h, (n + 7) / 8))
+        {
+            return from_ctx(c, SG_ERR_CUDA);
+        }
+        uint8_t* bytes = reinterpret_cast<uint8_t*>(h->staging);
+        if (int st = sg::tag_bytes(c, c.m(), bytes))
         {
             return from_ctx(c, st);
         }
-        std::vector<uint8_t> dense(static_cast<size_t>(c.capacity));
-        cudaMemcpyAsync(dense.data(), c.tag, dense.size(), cudaMemcpyDeviceToHost, c.stream);
+        cudaMemcpyAsync(values, bytes, static_cast<size_t>(n), cudaMemcpyDeviceToHost, c.stream);
         if (cudaStreamSynchronize(c.stream) != cudaSuccess)
         {
             return from_ctx(c, sg::check(c, "tag download"));
-        }
-        for (long long w = 0; w < c.g.total_words; ++w)
-        {
-            uint32_t v = hm.ref[w];
-            while (v)
-            {
-                const int b = __builtin_ctz(v);
-                v &= v - 1;
-                values[host_ref_index(hm, w, b)] = dense[static_cast<size_t>(32 * w + b)];
-            }
         }
         return SG_OK;
     }

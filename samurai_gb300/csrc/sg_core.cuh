@@ -137,7 +137,7 @@ namespace sg
 
     __device__ __forceinline__ bool test(const uint32_t* bm, const Pos& p)
     {
-        return p.w >= 0 && ((__ldg(bm + p.w) >> p.b) & 1u);
+        return p.w >= 0 && ((*(bm + p.w) >> p.b) & 1u);
     }
 
     __device__ __forceinline__ bool test(const uint32_t* bm, const Geom& g, int l, int x, int y, int z)
@@ -193,7 +193,7 @@ namespace sg
     // storage index in samurai's reference numbering
     __device__ __forceinline__ long long ref_index(const uint32_t* ref, const int* rank, const Pos& p)
     {
-        return static_cast<long long>(__ldg(rank + p.w)) + __popc(__ldg(ref + p.w) & ((1u << p.b) - 1u));
+        return static_cast<long long>(*(rank + p.w)) + __popc(*(ref + p.w) & ((1u << p.b) - 1u));
     }
 
     // ------------------------------------------------------- bit kernels
@@ -267,8 +267,8 @@ namespace sg
                 const long long frow = (g.dim == 2) ? ry : static_cast<long long>(rz) * F.R + ry;
                 const long long base = F.woff + frow * F.W;
                 const int k0         = 2 * wi - 1;
-                const uint32_t lo    = (k0 >= 0 && k0 < F.W) ? __ldg(fine + base + k0) : 0u;
-                const uint32_t hi    = (k0 + 1 >= 0 && k0 + 1 < F.W) ? __ldg(fine + base + k0 + 1) : 0u;
+                const uint32_t lo    = (k0 >= 0 && k0 < F.W) ? *(fine + base + k0) : 0u;
+                const uint32_t hi    = (k0 + 1 >= 0 && k0 + 1 < F.W) ? *(fine + base + k0 + 1) : 0u;
                 out |= compress_pairs(lo, hi);
             }
         }
@@ -306,7 +306,7 @@ namespace sg
             return 0u;
         }
         const long long crow = (g.dim == 2) ? ry : static_cast<long long>(rz) * C.R + ry;
-        const uint32_t cw    = __ldg(coarse + C.woff + crow * C.W + wc);
+        const uint32_t cw    = *(coarse + C.woff + crow * C.W + wc);
         return spread16(((k + 1) & 1) ? (cw >> 16) : cw);
     }
 
@@ -382,7 +382,7 @@ namespace sg
     __device__ __forceinline__ uint32_t self_or_ancestor(const Geom& g, const uint32_t* bm, int l, long long row, int wi, int lstop)
     {
         const LevelGeom& L = g.lv[l];
-        uint32_t acc       = __ldg(bm + L.woff + row * L.W + wi);
+        uint32_t acc       = *(bm + L.woff + row * L.W + wi);
         int y, z;
         if (g.dim == 2)
         {
@@ -461,9 +461,9 @@ namespace sg
                 continue;
             }
             const long long base = L.woff + ((g.dim == 2) ? y2 : static_cast<long long>(rz) * L.R + y2) * L.W;
-            const uint32_t mid   = __ldg(src + base + wi);
-            const uint32_t left  = wi > 0 ? __ldg(src + base + wi - 1) : 0u;
-            const uint32_t right = wi + 1 < L.W ? __ldg(src + base + wi + 1) : 0u;
+            const uint32_t mid   = *(src + base + wi);
+            const uint32_t left  = wi > 0 ? *(src + base + wi - 1) : 0u;
+            const uint32_t right = wi + 1 < L.W ? *(src + base + wi + 1) : 0u;
             out |= dilate_x(left, mid, right, r);
         }
         return out;

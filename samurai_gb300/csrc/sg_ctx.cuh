@@ -31,6 +31,7 @@ namespace sg
         uint32_t* ref   = nullptr; // MRMeshId::reference (all_cells)
         uint32_t* hc    = nullptr; // cells[l+1].on(l): cells with a leaf child
         uint32_t* hc2   = nullptr; // cells[l+2].on(l)
+        uint32_t* pred  = nullptr; // prediction ghosts: reference cells in the box that are neither leaves nor projections
         int* rank       = nullptr; // exclusive popcount prefix of ref
         int* wl_ref     = nullptr; // indices of the non-empty reference words, ascending
         int* wl_cells   = nullptr; // indices of the non-empty leaf-cell words, ascending
@@ -74,6 +75,14 @@ namespace sg
         F_DIFFER = 2, // new leaf cells differ from the current ones
         F_GRADX = 3,  // scratch for extra graduation passes
         F_COUNT = 8
+    };
+
+    // the Harten pass index and the criteria thresholds of a pass, per level:
+    // eps_l, 2^(reg+dim) eps_l and that over 2^dim (mr/criteria.hpp:31-111)
+    struct PassSetup
+    {
+        double eps[3 * MAXLEV];
+        int ite;
     };
 
     // Named phase timers with samurai's scope names (timers.hpp:111-1036;
@@ -131,19 +140,19 @@ namespace sg
         KernelTrace trace;
         MeshCfg cfg;
         Geom g{};                // geometry: kernels take it by value as a __grid_constant__ parameter
-        double* d_eps = nullptr; // per-level thresholds of the criteria (3 x MAXLEV)
-        unsigned long long* d_absmax = nullptr; // bits of max |u| over the leaf cells (relative details)
+        PassSetup* d_setup = nullptr; // thresholds and index of the Harten pass in flight
+        PassSetup* h_setup = nullptr; // pinned staging
+        unsigned long long* d_absmax = nullptr; // bits of max |u| over the leaf cells, per adapted field (relative details)
         int detail_comps             = 1;       // dense detail slabs allocated (one per adapted field)
         bool rel_detail = false;                // the Harten pass in flight divides the details by max |u|
         bool refine_boundary = false;           // args::refine_boundary: keep the boundary cells of max_level
-        double* h_eps = nullptr; // pinned staging of d_eps
         cudaStream_t stream = nullptr;
         int device          = -1; // the device current at creation: every buffer of the mesh lives there
         // streams that capture the bodies of conditional graph nodes (one per nesting depth)
         static constexpr int CAPTURE_DEPTH = 4;
         cudaStream_t cap_streams[CAPTURE_DEPTH] = {};
         int cap_depth = 0;
-        bool level_pairs = true; // tag finalisation two levels per launch (k_maximum2)
+        bool level_pairs = true; // launch shape: kept for callers and tuning files, the tag finalisation needs no pairs
         int* d_adapt  = nullptr; // device state of a graphed adaptation (AdaptSlot)
         int* h_adapt  = nullptr; // pinned mirror of d_adapt
         bool graphed_adapt = true; // the whole adaptation as one graph with conditional nodes
@@ -155,11 +164,16 @@ namespace sg
         uint32_t* t1 = nullptr;
         uint32_t* t2 = nullptr;
         uint32_t* t3 = nullptr;
-        uint32_t* rf = nullptr; // refine flags of leaf cells
-        uint32_t* cf = nullptr; // coarsen (and not keep) flags of leaf cells
-        // adaptation fields (dense layout)
-        double* detail = nullptr;
-        uint8_t* tag   = nullptr;
+        uint32_t* rf = nullptr; // the reference before the projection cells' children
+        // adaptation: the dense details (one slab per adapted field), and as bitmaps the tags and the cells
+        // whose detail passes the thresholds of coarsening, refinement and of their own children
+        double* detail      = nullptr;
+        uint32_t* tk        = nullptr; // tagged keep
+        uint32_t* tc        = nullptr; // tagged coarsen
+        uint32_t* tr        = nullptr; // tagged refine
+        uint32_t* above     = nullptr;
+        uint32_t* ref_above = nullptr;
+        uint32_t* par_above = nullptr;
         // scan scratch
         long long* block_sums = nullptr;
         long long n_scan_blocks = 0;
@@ -169,14 +183,11 @@ namespace sg
         int* d_flags        = nullptr;
         int* h_flags        = nullptr; // pinned mirror
         long long capacity  = 0;       // dense elements per field (32 * total_words)
-        int* d_ite          = nullptr; // Harten pass index seen by the detail/criteria kernels
-        int* h_ite          = nullptr; // pinned staging
         bool use_graphs     = true;    // replay captured launch sequences
         unsigned long long mesh_version = 1; // bumped at every change of the current mesh
         int fuse_top        = -1;      // levels 0..fuse_top are small enough for one-block mesh chains
         int fuse_top_field  = -1;      // the same for the FP64 field chains
         int fuse_top_max    = -1;      // the same for the tag-finalisation chain
-        const int* guard    = nullptr; // device flag: word launches do nothing while it is 0
         long long max_blocks = 152LL * 8; // grid limit of the one-warp-per-word launches, in blocks of 8 warps (x4 for one thread per word)
         int block            = 256;       // threads per block of the FP64 list kernels
         long long fuse_words_mesh  = 0; // one-block chain limits (words per level) behind fuse_top, fuse_top_field, fuse_top_max
@@ -221,14 +232,15 @@ namespace sg
 
     // kernels and drivers (sg_mesh.cu / sg_field.cu)
     int build_mesh(Ctx& c, DeviceMesh& m);           // from m.cells; asynchronous
-    int scan_rank(Ctx& c, DeviceMesh& m);            // rank, word lists, counters; asynchronous
     int host_counts(Ctx& c, DeviceMesh& m);          // synchronises and refreshes nb_ref / nb_cells
     int update_ghost_mr(Ctx& c, DeviceField& f);     // update_ghost_mr(u)
     int adapt(Ctx& c, DeviceField& f, double eps, double regularity, int* n_harten, bool relative_detail = false);
     int upwind(Ctx& c, DeviceField& u, DeviceField& unp1, const double* a, double dt, int scheme);
-    int upwind_on(Ctx& c, const DeviceMesh& m, const double* ud, double* unp1d, const double* a, double dt, int scheme, bool baked);
+    int upwind_on(Ctx& c, const DeviceMesh& m, const double* ud, double* unp1d, const double* a, double dt, int scheme);
     int step(Ctx& c, DeviceField& u, DeviceField& unp1, double eps, double regularity, const double* a, double dt, int scheme, int* n_harten);
     int gather_compact(Ctx& c, const DeviceMesh& m, const double* dense, double* compact);
+    int gather_details(Ctx& c, const DeviceMesh& m, double* compact); // the details of the last pass (first field)
+    int tag_bytes(Ctx& c, const DeviceMesh& m, uint8_t* compact);     // its tags: keep 1, coarsen 2, refine 4
     cudaError_t launch_gather(Ctx& c, const DeviceMesh& m, const double* dense, double* compact); // no error text
     cudaError_t read_device_error(Ctx& c, int* v);                                                  // reads and clears
     int scatter_compact(Ctx& c, const DeviceMesh& m, const double* compact, double* dense);
@@ -289,9 +301,6 @@ namespace sg
     // and the tag finalisation are not fused: their cells wait on memory, and
     // one block serialises that latency (measured slower than one launch per
     // level even at 1K-2K words), so their limit is 0.
-    // device thresholds buffer: [eps | fine | coarse] x MAXLEV, then a velocity
-    constexpr int EPS_VELOCITY = 3 * MAXLEV;
-
     constexpr long long FUSE_WORDS       = 1024;
     constexpr long long FUSE_WORDS_FIELD = 0;
     constexpr long long FUSE_WORDS_MAX   = 0;

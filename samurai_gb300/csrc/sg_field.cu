@@ -9,8 +9,7 @@
 #include <functional>
 #include <type_traits>
 
-#include "sg_access.cuh"
-#include "sg_ctx.cuh"
+#include "sg_phase_dev.cuh"
 
 namespace sg
 {
@@ -30,641 +29,10 @@ namespace sg
         return SG_OK;
     }
 
-    int new_cells_from_tags(Ctx& c, const DeviceMesh& m, uint32_t* nc);
-    int graduate(Ctx& c, uint32_t* nc, int* iterations);
-    int grad_pass(Ctx& c, uint32_t* nc, int slot, const int* guard);
-    int bitmaps_differ(Ctx& c, const uint32_t* a, const uint32_t* b, int slot);
+    int graduate(Ctx& c, DeviceMesh& m, DeviceMesh& nm, int* iterations);
 
     namespace
     {
-        constexpr int BLOCK = 256;
-
-        // One warp per listed word, lane b on bit b.  The list holds the
-        // non-empty words of a superset (reference or leaf cells) in
-        // ascending order; word_of(w) narrows it to the subset a kernel acts
-        // on.  Consecutive cells of a word are consecutive doubles, so every
-        // field access of a warp is one 256-byte segment.  A null list means
-        // every word of [begin, end): the dense range of small levels, which
-        // a launch covers with one warp per word without loading the list
-        // or its offsets (two dependent loads fewer at the head of the
-        // launch; word_of is zero on the words the list leaves out).
-        template <class WordF, class CellF>
-        __device__ __forceinline__ void warp_list(const int* list, long long begin, long long end, long long warp0, long long nwarps, WordF word_of,
-                                                  CellF cell)
-        {
-            const int lane = threadIdx.x & 31;
-            for (long long i = begin + warp0; i < end; i += nwarps)
-            {
-                const long long w = list ? __ldg(list + i) : i;
-                const uint32_t v  = word_of(w);
-                if ((v >> lane) & 1u)
-                {
-                    cell(w, lane);
-                }
-            }
-        }
-
-        // Compacted traversal for the FP64-heavy kernels.  On the traversal
-        // above a warp works on one word and the lanes of its empty bits idle
-        // while the others issue FP64 instructions, which the narrow FP64 pipe
-        // executes for the whole warp (42 % of the lanes of the leaf-cell
-        // words of the 2D max_level-12 workload hold a cell).  Here a warp
-        // takes ch consecutive words of the list, ranks their set bits with a
-        // warp prefix sum and processes them 32 at a time, one per lane.
-        // item(valid, w, b) is called by every lane of the warp (so that it
-        // may shuffle); only lanes with valid set hold an item, bit b of word w.
-        constexpr unsigned FULL_MASK = 0xffffffffu;
-
-        // words per warp: the largest power of two (<= 32) that still leaves
-        // every warp of the launch a chunk; 1 on lists shorter than two words
-        // per warp, where the launch is latency-bound and the compaction does
-        // not pay
-        __device__ __forceinline__ int items_chunk(long long n, long long nwarps)
-        {
-            const long long per = n / (nwarps > 0 ? nwarps : 1);
-            int ch              = 1;
-            while (ch < 32 && 2 * ch <= per)
-            {
-                ch <<= 1;
-            }
-            return ch;
-        }
-
-        template <class WordF, class ItemF>
-        __device__ __forceinline__ void warp_items(const int* list, long long begin, long long end, long long warp0, long long nwarps, int ch,
-                                                   WordF word_of, ItemF item)
-        {
-            const int lane = threadIdx.x & 31;
-            for (long long c0 = begin + warp0 * ch; c0 < end; c0 += nwarps * ch)
-            {
-                long long w = 0;
-                uint32_t m  = 0u;
-                if (lane < ch && c0 + lane < end)
-                {
-                    w = list ? __ldg(list + c0 + lane) : c0 + lane;
-                    m = word_of(w);
-                }
-                int incl = __popc(m); // inclusive prefix of the item counts over the lanes
-                for (int o = 1; o < 32; o <<= 1)
-                {
-                    const int t = __shfl_up_sync(FULL_MASK, incl, o);
-                    if (lane >= o)
-                    {
-                        incl += t;
-                    }
-                }
-                const int total = __shfl_sync(FULL_MASK, incl, 31);
-                for (int base = 0; base < total; base += 32)
-                {
-                    const int j = base + lane;
-                    // the word of item j: the first lane whose inclusive prefix exceeds j
-                    int lo_k = 0, hi_k = 31;
-                    for (int s = 0; s < 5; ++s)
-                    {
-                        const int mid = (lo_k + hi_k) >> 1;
-                        if (__shfl_sync(FULL_MASK, incl, mid) > j)
-                        {
-                            hi_k = mid;
-                        }
-                        else
-                        {
-                            lo_k = mid + 1;
-                        }
-                    }
-                    const long long wk = __shfl_sync(FULL_MASK, w, lo_k);
-                    const uint32_t mk  = __shfl_sync(FULL_MASK, m, lo_k);
-                    const int before   = __shfl_sync(FULL_MASK, incl, lo_k) - __popc(mk);
-                    const bool valid   = j < total;
-                    // position of set bit number r (from 0) of mk
-                    int r = valid ? j - before : 0, pos = 0;
-                    uint32_t x = mk;
-                    for (int sh = 16; sh > 0; sh >>= 1)
-                    {
-                        const int cnt = __popc(x & ((1u << sh) - 1u));
-                        if (r >= cnt)
-                        {
-                            r -= cnt;
-                            x >>= sh;
-                            pos += sh;
-                        }
-                    }
-                    item(valid, wk, pos);
-                }
-            }
-        }
-
-        // warp_list with the compacted traversal where the list is long enough:
-        // cell(w, b) for every set bit
-        template <class WordF, class CellF>
-        __device__ __forceinline__ void warp_list_compact(const int* list, long long begin, long long end, long long warp0, long long nwarps,
-                                                          WordF word_of, CellF cell)
-        {
-            const int ch = items_chunk(end - begin, nwarps);
-            if (ch == 1)
-            {
-                warp_list(list, begin, end, warp0, nwarps, word_of, cell);
-                return;
-            }
-            warp_items(list, begin, end, warp0, nwarps, ch, word_of,
-                       [&](bool valid, long long w, int b)
-                       {
-                           if (valid)
-                           {
-                               cell(w, b);
-                           }
-                       });
-        }
-
-        __device__ __forceinline__ long long warp_id()
-        {
-            return (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
-        }
-
-        __device__ __forceinline__ long long warp_count()
-        {
-            return (static_cast<long long>(gridDim.x) * blockDim.x) >> 5;
-        }
-
-
-        // The prediction coefficients interp_coeffs<3> (numeric/prediction.hpp:32-36)
-        // of tap t in {0,1,2} for a child of parity q are 1 at t = 1 and
-        // +-1/8 at t = 0, 2 (negative at t = 0 for odd children, at t = 2 for
-        // even ones); products over the axes are +-8^-k, k = off-centre taps.
-
-        // Element of a cell that the reference algorithm guarantees to be in
-        // the stored box.  A position outside it (a bug or an invalid mesh)
-        // is recorded in the device error word and redirected to element 0,
-        // so that no access leaves the allocation.
-        __device__ __forceinline__ long long elem_at(const Geom& g, int l, int x, int y, int z)
-        {
-            const Pos p = pos_of(g, l, x, y, z);
-            if (p.w < 0)
-            {
-                atomicOr(g.err, 1);
-                return 0;
-            }
-            return elem(p);
-        }
-
-        // x * 2^-s (0 < s < 64), exactly, without the FP64 pipe when it can: for
-        // a normal x whose product stays normal the product is x with its
-        // exponent lowered by s (what the multiplication rounds to, since it is
-        // exact); zeros keep their bits; other values take the multiplication.
-        __device__ __forceinline__ double scale_down(double x, int s)
-        {
-            const long long b = __double_as_longlong(x);
-            const int e       = static_cast<int>((b >> 52) & 0x7FF);
-            if (e > s && e < 0x7FF)
-            {
-                return __longlong_as_double(b - (static_cast<long long>(s) << 52));
-            }
-            if ((static_cast<unsigned long long>(b) << 1) == 0)
-            {
-                return x;
-            }
-            return x * __longlong_as_double(static_cast<long long>(1023 - s) << 52);
-        }
-
-        // x * 8^-k: the prediction coefficients' magnitudes
-        __device__ __forceinline__ double scale8(double x, int k)
-        {
-            return scale_down(x, 3 * k);
-        }
-
-        template <int CAP>
-        __device__ __forceinline__ LinForm<CAP> scale_down(const LinForm<CAP>& x, int s)
-        {
-            return x * (1.0 / static_cast<double>(1LL << s));
-        }
-
-        // -x when neg, by the sign bit (exact, no FP64 operation)
-        __device__ __forceinline__ double negate_if(bool neg, double x)
-        {
-            return __longlong_as_double(__double_as_longlong(x) ^ (static_cast<long long>(neg) << 63));
-        }
-
-        template <int CAP>
-        __device__ __forceinline__ LinForm<CAP> scale8(const LinForm<CAP>& x, int k)
-        {
-            return x * (k == 1 ? 0.125 : (k == 2 ? 0.015625 : 0.001953125));
-        }
-
-        template <int CAP>
-        __device__ __forceinline__ LinForm<CAP> negate_if(bool neg, const LinForm<CAP>& x)
-        {
-            return neg ? -x : x;
-        }
-
-        // A box of cells [x0, x0+n) x [y0, y0+n) x [z0, z0+n) at level l as a base
-        // element and strides: both corners are checked against the stored
-        // box (a violation is recorded and every access goes to element 0)
-        struct Box3
-        {
-            long long base, sy, sz;
-        };
-
-        template <int DIM>
-        __device__ __forceinline__ Box3 box_at(const Geom& g, int l, int x0, int y0, int z0, int n)
-        {
-            const Pos lo = pos_of(g, l, x0, y0, DIM == 3 ? z0 : 0);
-            const Pos hi = pos_of(g, l, x0 + n - 1, y0 + n - 1, DIM == 3 ? z0 + n - 1 : 0);
-            if (lo.w < 0 || hi.w < 0)
-            {
-                atomicOr(g.err, 1);
-                return {0, 0, 0};
-            }
-            const LevelGeom& L = g.lv[l];
-            return {elem(lo), 32LL * L.W, 32LL * L.W * L.R};
-        }
-
-        // prediction_op<order,false> for one fine cell (numeric/prediction.hpp:286-361)
-        template <int DIM, class A>
-        __device__ __forceinline__ typename A::V predict_one(const Geom& g, const A& u, int l, int x, int y, int z, int order)
-        {
-            const int px = x >> 1, py = y >> 1, pz = z >> 1;
-            if (order == 0)
-            {
-                return u.get(elem_at(g, l - 1, px, py, pz));
-            }
-            // acc + u * coeff with coeff = ((1 * cx) * cy) * cz = +-8^-k (k = axes
-            // with an off-centre tap): u * coeff is +-(u * 8^-k) bit for bit
-            // (power-of-two scaling is exact) and acc + (-m) is acc - m
-            typename A::V acc = A::konst(0.);
-            const int qx = x & 1, qy = y & 1, qz = z & 1;
-            const Box3 bx     = box_at<DIM>(g, l - 1, px - 1, py - 1, pz - 1, 3);
-#pragma unroll
-            for (int sz = 0; sz < (DIM == 3 ? 3 : 1); ++sz)
-            {
-#pragma unroll
-                for (int sy = 0; sy < 3; ++sy)
-                {
-                    const long long base = bx.base + sy * bx.sy + sz * bx.sz;
-#pragma unroll
-                    for (int sx = 0; sx < 3; ++sx)
-                    {
-                        const int k      = (sx != 1) + (sy != 1) + (DIM == 3 && sz != 1);
-                        const bool neg   = ((sx == 0 && qx) || (sx == 2 && !qx)) ^ ((sy == 0 && qy) || (sy == 2 && !qy))
-                                         ^ (DIM == 3 && ((sz == 0 && qz) || (sz == 2 && !qz)));
-                        const typename A::V v = u.get(base + sx);
-                        // acc + u * coeff == acc + (+-m): one FP64 addition per tap
-                        const typename A::V m = k == 0 ? v : scale8(v, k);
-                        acc                   = acc + negate_if(neg, m);
-                    }
-                }
-            }
-            return acc;
-        }
-
-        // projection_op_ (numeric/projection.hpp:15-65)
-        template <int DIM, class A>
-        __device__ __forceinline__ typename A::V project_one(const Geom& g, const A& u, int lf, int x, int y, int z)
-        {
-            typename A::V sum = A::konst(0.);
-            const Box3 bx     = box_at<DIM>(g, lf, 2 * x, 2 * y, 2 * z, 2);
-#pragma unroll
-            for (int sz = 0; sz < (DIM == 3 ? 2 : 1); ++sz)
-            {
-#pragma unroll
-                for (int sy = 0; sy < 2; ++sy)
-                {
-                    const long long e = bx.base + sy * bx.sy + sz * bx.sz;
-                    sum               = sum + (u.get(e) + u.get(e + 1));
-                }
-            }
-            // sum * (1 / 2^dim)
-            return scale_down(sum, DIM);
-        }
-
-        // ----------------------------------------------------------- tags
-        __global__ void k_tag_init(const __grid_constant__ Geom gp, const int* wl, const long long* lo, const uint32_t* ref, const uint32_t* cells,
-                                   uint8_t* tag, double* det)
-        {
-            warp_list(wl, lo[LO_REF], lo[LO_REF + gp.nlev], warp_id(), warp_count(), [&](long long w) { return ref[w]; },
-                      [&](long long w, int b)
-                      {
-                          const long long e = 32 * w + b;
-                          tag[e]            = static_cast<uint8_t>((cells[w] >> b) & 1u);
-                          det[e]            = 0.;
-                      });
-        }
-
-        // ----------------------------------------------------- outer ghosts
-        // k-th diagonal direction in for_each_diagonal_direction order
-        // (stencil.hpp:338-349): first coordinate fastest, at least two
-        // non-zero components
-        __device__ __forceinline__ void diagonal_dir(int dim, int k, int* d)
-        {
-            int found = 0;
-            const int nz = (dim == 3) ? 3 : 1;
-            for (int t = 0; t < 9 * nz; ++t)
-            {
-                const int x = t % 3 - 1, y = (t / 3) % 3 - 1, z = (dim == 3) ? t / 9 - 1 : 0;
-                if ((x != 0) + (y != 0) + (z != 0) > 1)
-                {
-                    if (found == k)
-                    {
-                        d[0] = x;
-                        d[1] = y;
-                        d[2] = z;
-                        return;
-                    }
-                    ++found;
-                }
-            }
-            d[0] = d[1] = d[2] = 0;
-        }
-
-        // PolynomialExtrapolation of the second ghost layer (bc/polynomial_extrapolation.hpp:22-92, stencil of 4
-        // cells along d from c - d): u(c + 2d) = u(c - d) - 3 u(c) + 3 u(c + d), in the reference's operation order
-        template <class A>
-        __device__ __forceinline__ void extrapolate_layer2(const Geom& g, int l, const int* c, const int* d, const A& u)
-        {
-            const int z = g.dim == 3;
-            const long long em = elem_at(g, l, c[0] - d[0], c[1] - d[1], z ? c[2] - d[2] : 0);
-            const long long e0 = elem_at(g, l, c[0], c[1], z ? c[2] : 0);
-            const long long e1 = elem_at(g, l, c[0] + d[0], c[1] + d[1], z ? c[2] + d[2] : 0);
-            const long long e2 = elem_at(g, l, c[0] + 2 * d[0], c[1] + 2 * d[1], z ? c[2] + 2 * d[2] : 0);
-            u.put(e2, (u.get(em) - u.get(e0) * 3.0) + u.get(e1) * 3.0);
-        }
-
-        // update_outer_corners_by_polynomial_extrapolation (bc/apply_field_bc.hpp:371-505) followed by
-        // project_corner_below (algorithm/update_outer_ghost.hpp:268-337), one block per diagonal direction d:
-        // layer 1 copies the corner leaf, layer 2 (ghost width 2) extrapolates along d, then the other ghosts
-        // of the corner block copy the diagonal ones (the off-diagonal copies).  parts: 1 the corners, 2 their
-        // projection below, 3 both (the projection reads the corners, after a block barrier).
-        template <class A>
-        __device__ void corner_role(const Geom& g, const int* d, int l, const uint32_t* cells, const uint32_t* ref, const A& u, int parts = 3)
-        {
-            if (crosses_periodic(g, d))
-            {
-                return; // no corner across a periodic axis (the test is uniform over the block)
-            }
-            const int n = g.lv[l].n;
-            int nfree   = 0;
-            for (int k = 0; k < g.dim; ++k)
-            {
-                nfree += (d[k] == 0);
-            }
-            const long long npos = (nfree == 0) ? 1 : n; // 3D edges have one free axis
-            for (long long t = threadIdx.x; (parts & 1) && t < npos; t += blockDim.x)
-            {
-                int c[3];
-                for (int k = 0; k < 3; ++k)
-                {
-                    c[k] = (k < g.dim) ? (d[k] > 0 ? n - 1 : (d[k] < 0 ? 0 : static_cast<int>(t))) : 0;
-                }
-                const Pos pc = pos_of(g, l, c[0], c[1], c[2]);
-                if (test(cells, pc))
-                {
-                    const long long eg = elem_at(g, l, c[0] + d[0], c[1] + d[1], g.dim == 3 ? c[2] + d[2] : 0);
-                    u.put(eg, u.get(elem(pc)));
-                    if (g.ghost_width >= 2)
-                    {
-                        if (test(ref, g, l, c[0] + 2 * d[0], c[1] + 2 * d[1], g.dim == 3 ? c[2] + 2 * d[2] : 0))
-                        {
-                            extrapolate_layer2(g, l, c, d, u);
-                        }
-                        // off-diagonal copies: from c + k d (k = 1, 2) to c + k d + delta, delta moving the
-                        // non-zero components after the first by g - (k - 1), g in [0, 2), not all zero
-                        int nz[3], nnz = 0;
-                        for (int k = 0; k < g.dim; ++k)
-                        {
-                            if (d[k] != 0)
-                            {
-                                nz[nnz++] = k;
-                            }
-                        }
-                        const int combos = nnz == 3 ? 4 : 2;
-                        for (int k = 1; k <= 2; ++k)
-                        {
-                            const int sx = c[0] + k * d[0], sy = c[1] + k * d[1], sz = g.dim == 3 ? c[2] + k * d[2] : 0;
-                            const long long es = elem_at(g, l, sx, sy, sz);
-                            for (int combo = 0; combo < combos; ++combo)
-                            {
-                                int delta[3] = {0, 0, 0};
-                                bool source  = true;
-                                int tmp      = combo;
-                                for (int p = 1; p < nnz; ++p)
-                                {
-                                    const int dp = (tmp % 2) - (k - 1);
-                                    tmp /= 2;
-                                    delta[nz[p]] += dp * d[nz[p]];
-                                    source = source && dp == 0;
-                                }
-                                if (!source)
-                                {
-                                    u.put(elem_at(g, l, sx + delta[0], sy + delta[1], sz + delta[2]), u.get(es));
-                                }
-                            }
-                        }
-                    }
-                }
-            }
-            if (parts != 3)
-            {
-                if (!(parts & 2))
-                {
-                    return;
-                }
-            }
-            else
-            {
-                __syncthreads();
-            }
-            for (int dl = 1; dl <= 2; ++dl)
-            {
-                const int pl = l - dl;
-                if (pl < 0)
-                {
-                    break;
-                }
-                const int npl          = g.lv[pl].n;
-                const long long npos_c = (nfree == 0) ? 1 : npl;
-                for (long long t = threadIdx.x; t < npos_c; t += blockDim.x)
-                {
-                    int gc[3], ch[3];
-                    for (int k = 0; k < 3; ++k)
-                    {
-                        if (k >= g.dim)
-                        {
-                            gc[k] = ch[k] = 0;
-                            continue;
-                        }
-                        gc[k] = d[k] > 0 ? npl : (d[k] < 0 ? -1 : static_cast<int>(t));
-                        ch[k] = (gc[k] << dl) + (d[k] == -1 ? ((1 << dl) - 1) : 0);
-                    }
-                    const Pos pg = pos_of(g, pl, gc[0], gc[1], gc[2]);
-                    const Pos pf = pos_of(g, l, ch[0], ch[1], ch[2]);
-                    if (test(ref, pg) && test(ref, pf))
-                    {
-                        u.put(elem(pg), u.get(elem(pf)));
-                    }
-                }
-            }
-        }
-
-        // face position helper: direction index k in 0..2*dim-1 is
-        // (+e0,-e0,+e1,-e1,...) (stencil.hpp:301-317)
-        __device__ __forceinline__ void face_cell(const Geom& g, int l, int k, long long t, int* in, int* dir)
-        {
-            const int axis = k >> 1;
-            const int sgn  = (k & 1) ? -1 : 1;
-            const int n    = g.lv[l].n;
-            const int f0 = static_cast<int>(t % n), f1 = static_cast<int>(t / n);
-            // the free coordinates fill the non-normal axes in order
-            dir[0] = dir[1] = dir[2] = 0;
-            in[2]                    = 0;
-            if (axis == 0)
-            {
-                in[0] = sgn > 0 ? n - 1 : 0;
-                in[1] = f0;
-                in[2] = (g.dim == 3) ? f1 : 0;
-            }
-            else if (axis == 1)
-            {
-                in[0] = f0;
-                in[1] = sgn > 0 ? n - 1 : 0;
-                in[2] = (g.dim == 3) ? f1 : 0;
-            }
-            else
-            {
-                in[0] = f0;
-                in[1] = f1;
-                in[2] = sgn > 0 ? n - 1 : 0;
-            }
-            dir[axis] = sgn;
-        }
-
-        struct GhostLevelArgs
-        {
-            int l;
-            int do_corners;
-            int do_project;   // project_bc: level < max_level
-            int do_dirichlet; // apply_field_bc: level >= min_level and a BC is attached
-            int do_predict;   // predict_bc: min_level <= level < max_level
-            double value;
-            int nb_corner;    // blocks of the corner role
-            int nb_face;      // blocks of the face role
-            long long nfaces; // face positions (2*dim directions)
-            int do_proj;      // project the reference of level l onto proj_cells[l-1]
-            int corner_parts; // corner_role parts run by the corner blocks
-            int do_dirichlet_layer2; // the second ghost layer next to non-leaf boundary cells (level >= min_level, a BC)
-        };
-
-        // One launch per level of the top-down pass of update_ghost_mr
-        // (algorithm/update_ghost_mr.hpp:206-222).  Within a level the
-        // reference's operations touch disjoint cells and read only cells
-        // finalised earlier, so they run concurrently as block roles:
-        //  - corners: outer corners and their projection two levels down;
-        //  - faces: per Cartesian direction, the Dirichlet ghost 2v - u
-        //    (bc/dirichlet.hpp:22-29) then predict_bc to level l+1
-        //    (update_outer_ghost.hpp:195-266) by the same thread, or project_bc
-        //    (update_outer_ghost.hpp:20-155) next to union cells;
-        //  - projection of the reference cells of level l onto proj_cells[l-1]
-        //    (numeric/projection.hpp:15-65).
-        template <int DIM, class A>
-        __device__ __forceinline__ void face_work(const Geom& g, const GhostLevelArgs& a, long long t, const uint32_t* cells, const uint32_t* uni,
-                                                  const uint32_t* ref, const A& u)
-        {
-            const int l        = a.l;
-            const int n        = g.lv[l].n;
-            const long long nf = (DIM == 2) ? n : static_cast<long long>(n) * n;
-            const int k        = static_cast<int>(t / nf);
-            int in[3], dir[3];
-            face_cell(g, l, k, t - k * nf, in, dir);
-            if (crosses_periodic(g, dir))
-            {
-                return; // a periodic axis has no boundary
-            }
-            const Pos pi = pos_of(g, l, in[0], in[1], in[2]);
-            const int gx = in[0] + dir[0], gy = in[1] + dir[1], gz = in[2] + dir[2];
-            if ((a.do_dirichlet || a.do_predict) && test(cells, pi))
-            {
-                const long long eg = elem_at(g, l, gx, gy, gz);
-                typename A::V v;
-                if (a.do_dirichlet)
-                {
-                    v = A::konst(2 * a.value) - u.get(elem(pi));
-                    u.put(eg, v);
-                    // update_further_ghosts_by_polynomial_extrapolation (bc/apply_field_bc.hpp:531-593), ghost
-                    // width 2: the second layer beyond a boundary leaf, where it is a reference cell
-                    if (g.ghost_width >= 2 && test(ref, g, l, gx + dir[0], gy + dir[1], gz + dir[2]))
-                    {
-                        extrapolate_layer2(g, l, in, dir, u);
-                    }
-                }
-                else
-                {
-                    v = u.get(eg);
-                }
-                if (a.do_predict)
-                {
-                    for (int sz = 0; sz < (DIM == 3 ? 2 : 1); ++sz)
-                    {
-                        for (int sy = 0; sy < 2; ++sy)
-                        {
-                            for (int sx = 0; sx < 2; ++sx)
-                            {
-                                const Pos pf = pos_of(g, l + 1, 2 * gx + sx, 2 * gy + sy, DIM == 3 ? 2 * gz + sz : 0);
-                                if (test(ref, pf))
-                                {
-                                    u.put(elem(pf), v);
-                                }
-                            }
-                        }
-                    }
-                }
-            }
-            else if (a.do_project && test(uni, pi))
-            {
-                const Pos pg = pos_of(g, l, gx, gy, gz);
-                if (!test(ref, pg))
-                {
-                    return;
-                }
-                typename A::V sum = A::konst(0.);
-                int nch           = 0;
-                for (int dl = 1; dl <= 2 && nch == 0 && l + dl < g.nlev; ++dl)
-                {
-                    const int lc = l + dl;
-                    const int m  = 1 << dl;
-                    for (int sz = 0; sz < (DIM == 3 ? m : 1); ++sz)
-                    {
-                        for (int sy = 0; sy < m; ++sy)
-                        {
-                            for (int sx = 0; sx < m; ++sx)
-                            {
-                                const Pos pc = pos_of(g, lc, gx * m + sx, gy * m + sy, DIM == 3 ? gz * m + sz : 0);
-                                if (test(ref, pc))
-                                {
-                                    sum = sum + u.get(elem(pc));
-                                    ++nch;
-                                }
-                            }
-                        }
-                    }
-                }
-                u.put(elem(pg), nch > 0 ? sum / static_cast<double>(nch) : A::konst(0.));
-                // the second ghost layer beyond a boundary cell that is not a leaf but has finer leaves
-                // (apply_extrapolation_bc_ghosts, bc/apply_field_bc.hpp:196-214), ghost width 2
-                if (g.ghost_width >= 2 && a.do_dirichlet_layer2 && test(ref, g, l, gx + dir[0], gy + dir[1], gz + dir[2]))
-                {
-                    extrapolate_layer2(g, l, in, dir, u);
-                }
-            }
-        }
-
-        template <class A>
-        struct IsRev
-        {
-            static constexpr bool value = false;
-        };
-        template <int CAP>
-        struct IsRev<RevAcc<CAP>>
-        {
-            static constexpr bool value = true;
-        };
-
         // The transposes of one projection and one prediction, written out instead of through linear forms: the
         // weights are those the forms would carry (2^-dim for each child; +-8^-k for each tap of the order-1
         // stencil, the signs and k as in predict_one), so the adjoint is the same operator, without building a form
@@ -731,699 +99,50 @@ namespace sg
             }
         }
 
-        // projection of the reference cells of level l onto proj_cells[l-1]
-        // (numeric/projection.hpp:15-65), warps warp0, warp0+nwarps, ...
-        template <int DIM, class A>
-        __device__ __forceinline__ void project_level(const Geom& g, int l, const int* wl_ref, const long long* lo, const uint32_t* proj, const uint32_t* ref,
-                                                      const A& u, long long warp0, long long nwarps)
-        {
-            const int lc = l - 1;
-            const LevelGeom& C = g.lv[lc];
-            warp_list_compact(lo ? wl_ref : nullptr, lo ? lo[LO_REF + lc] : C.woff, lo ? lo[LO_REF + lc + 1] : C.woff + C.nwords, warp0, nwarps,
-                      [&](long long w)
-                      {
-                          const WordLoc loc = word_loc(g, lc, w);
-                          return proj[w] & coarsen_word(g, ref, lc, loc.row, loc.wi);
-                      },
-                      [&](long long w, int b)
-                      {
-                          const Cell c = cell_of(g, lc, w, b);
-                          if constexpr (IsRev<A>::value)
-                          {
-                              project_transpose<DIM>(g, u, 32 * w + b, l, c.x, c.y, c.z);
-                          }
-                          else
-                          {
-                              u.put(32 * w + b, project_one<DIM>(g, u, l, c.x, c.y, c.z));
-                          }
-                      });
-        }
-
-        // prediction of the ghosts of level l from level l-1
-        // (algorithm/update_ghost_mr.hpp:224-233)
-        template <int DIM, class A>
-        __device__ __forceinline__ void predict_level(const Geom& g, int l, int order, const int* wl_ref, const long long* lo, const uint32_t* cells,
-                                                      const uint32_t* proj, const uint32_t* ref, const A& u, long long warp0, long long nwarps)
-        {
-            const LevelGeom& L = g.lv[l];
-            warp_list_compact(lo ? wl_ref : nullptr, lo ? lo[LO_REF + l] : L.woff, lo ? lo[LO_REF + l + 1] : L.woff + L.nwords, warp0, nwarps,
-                      [&](long long w)
-                      {
-                          const WordLoc loc = word_loc(g, l, w);
-                          return ref[w] & ~(cells[w] | proj[w]) & box_mask(g, l, loc.row, loc.wi, 0, 0) & refine_word(g, ref, l, loc.row, loc.wi);
-                      },
-                      [&](long long w, int b)
-                      {
-                          const Cell c = cell_of(g, l, w, b);
-                          if constexpr (IsRev<A>::value)
-                          {
-                              predict_transpose<DIM>(g, u, 32 * w + b, l, c.x, c.y, c.z, order);
-                          }
-                          else
-                          {
-                              u.put(32 * w + b, predict_one<DIM>(g, u, l, c.x, c.y, c.z, order));
-                          }
-                      });
-        }
-
-        // One launch per level of the top-down pass of update_ghost_mr
-        // (algorithm/update_ghost_mr.hpp:206-222).  Within a level the
-        // reference's operations touch disjoint cells and read only cells
-        // finalised earlier, so they run concurrently as block roles:
-        //  - corners: outer corners and their projection two levels down;
-        //  - faces: per Cartesian direction, the Dirichlet ghost 2v - u
-        //    (bc/dirichlet.hpp:22-29) then predict_bc to level l+1
-        //    (update_outer_ghost.hpp:195-266) by the same thread, or project_bc
-        //    (update_outer_ghost.hpp:20-155) next to union cells;
-        //  - projection of the reference cells of level l onto proj_cells[l-1].
-        template <int DIM, class A>
-        __global__ void k_ghost_level(const __grid_constant__ Geom gp, GhostLevelArgs a, const int* wl_ref, const long long* lo, const uint32_t* cells,
-                                      const uint32_t* uni, const uint32_t* proj, const uint32_t* ref, A u)
+        // The launches of the transposed ghost update: one per level and role, so
+        // that no launch reads what it writes.
+        // top-down, level l: corners (parts 1), faces and the projection onto level l-1; or the corners'
+        // projection below alone (parts 2)
+        template <int DIM, int CAP>
+        __global__ void k_ghost_reverse(const __grid_constant__ Geom gp, int l, int parts, int nb, int has_bc, MeshPtrs m, RevAcc<CAP> u)
         {
             const Geom& g = gp;
-            const int l   = a.l;
-            if (static_cast<int>(blockIdx.x) < a.nb_corner)
+            if (static_cast<int>(blockIdx.x) < nb)
             {
-                int d[3];
-                diagonal_dir(DIM, static_cast<int>(blockIdx.x), d);
-                corner_role(g, d, l, cells, ref, u, a.corner_parts);
-                return;
-            }
-            if (static_cast<int>(blockIdx.x) < a.nb_corner + a.nb_face)
-            {
-                const long long t = static_cast<long long>(blockIdx.x - a.nb_corner) * blockDim.x + threadIdx.x;
-                if (t < a.nfaces)
+                const long long nc    = l >= g.min_level ? corner_count<DIM>(g, l) : 0;
+                const long long total = (parts & 1) ? boundary_count<DIM>(g, l) : nc;
+                for (long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += static_cast<long long>(nb) * blockDim.x)
                 {
-                    face_work<DIM>(g, a, t, cells, uni, ref, u);
-                }
-                return;
-            }
-            if (!a.do_proj)
-            {
-                return;
-            }
-            const long long rb     = static_cast<long long>(blockIdx.x - a.nb_corner - a.nb_face);
-            const long long warp0  = (rb * blockDim.x + threadIdx.x) >> 5;
-            const long long nwarps = (static_cast<long long>(gridDim.x - a.nb_corner - a.nb_face) * blockDim.x) >> 5;
-            project_level<DIM>(g, l, wl_ref, lo, proj, ref, u, warp0, nwarps);
-        }
-
-        // iterate_over_periodic_ghosts (algorithm/update_periodic.hpp:27-140) on
-        // axis d, one side: side 0 pairs the ghosts of [n, n + gw) with [0, gw),
-        // side 1 those of [-gw, 0) with [n - gw, n); the other axes span
-        // [-gw, n + gw).  Only pairs of two reference cells count.  Work item t
-        // of the side: gw * (n + 2 gw)^(dim-1) of them.
-        __device__ __forceinline__ bool periodic_pair(const Geom& g, int l, int d, int side, long long t, const uint32_t* ref, long long* eg,
-                                                      long long* ei)
-        {
-            const int n = g.lv[l].n, gw = g.ghost_width, span = n + 2 * gw;
-            int c[3]    = {0, 0, 0};
-            c[d]        = (side == 0 ? n : -gw) + static_cast<int>(t % gw);
-            long long r = t / gw;
-            for (int k = 0; k < g.dim; ++k)
-            {
-                if (k != d)
-                {
-                    c[k] = -gw + static_cast<int>(r % span);
-                    r /= span;
-                }
-            }
-            int q[3] = {c[0], c[1], c[2]};
-            q[d] += side == 0 ? -n : n;
-            const Pos pg = pos_of(g, l, c[0], c[1], c[2]);
-            const Pos pi = pos_of(g, l, q[0], q[1], q[2]);
-            if (!test(ref, pg) || !test(ref, pi))
-            {
-                return false;
-            }
-            *eg = elem(pg);
-            *ei = elem(pi);
-            return true;
-        }
-
-        inline long long periodic_side_items(const Geom& g, int l)
-        {
-            const long long span = g.lv[l].n + 2 * g.ghost_width;
-            return g.ghost_width * (g.dim == 2 ? span : span * span);
-        }
-
-        // update_ghost_periodic(level, field) (algorithm/update_periodic.hpp:19-25)
-        // on one axis: both sides at once (they read inner cells and write
-        // outer ghosts, so no item reads what another writes)
-        __global__ void k_periodic_copy(const __grid_constant__ Geom gp, int l, int d, long long per_side, const uint32_t* ref, double* u)
-        {
-            const Geom& g     = gp;
-            const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (t >= 2 * per_side)
-            {
-                return;
-            }
-            const int side = t >= per_side ? 1 : 0;
-            long long eg, ei;
-            if (periodic_pair(g, l, d, side, t - side * per_side, ref, &eg, &ei))
-            {
-                u[eg] = u[ei];
-            }
-        }
-
-        // update_tag_periodic(level, tag) (algorithm/update_periodic.hpp:178-300)
-        // on one axis and side: both cells of a pair take the union of their tags
-        __global__ void k_periodic_tag(const __grid_constant__ Geom gp, int l, int d, int side, long long per_side, const uint32_t* ref, uint8_t* tag)
-        {
-            const Geom& g     = gp;
-            const long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-            if (t >= per_side)
-            {
-                return;
-            }
-            long long eg, ei;
-            if (periodic_pair(g, l, d, side, t, ref, &eg, &ei))
-            {
-                tag[eg] |= tag[ei];
-                tag[ei] |= tag[eg];
-            }
-        }
-
-        // the periodic ghost copies of one level, axis after axis (a later axis
-        // reads the ghosts an earlier one wrote: the corners)
-        void periodic_copies(Ctx& c, const DeviceMesh& m, int l, double* u)
-        {
-            const Geom& g = c.g;
-            if (!g.periodic || l < 0 || l >= g.nlev)
-            {
-                return;
-            }
-            const long long per = periodic_side_items(g, l);
-            for (int d = 0; d < g.dim; ++d)
-            {
-                if ((g.periodic >> d) & 1)
-                {
-                    k_periodic_copy<<<static_cast<int>((2 * per + BLOCK - 1) / BLOCK), BLOCK, 0, c.stream>>>(c.g, l, d, per, m.ref, u);
-                    launched(c, "periodic_copy");
-                }
-            }
-        }
-
-        void periodic_tags(Ctx& c, const DeviceMesh& m, int l)
-        {
-            const Geom& g = c.g;
-            if (!g.periodic || l < 0 || l >= g.nlev)
-            {
-                return;
-            }
-            const long long per = periodic_side_items(g, l);
-            for (int d = 0; d < g.dim; ++d)
-            {
-                if ((g.periodic >> d) & 1)
-                {
-                    for (int side = 0; side < 2; ++side)
+                    if (t < nc)
                     {
-                        k_periodic_tag<<<static_cast<int>((per + BLOCK - 1) / BLOCK), BLOCK, 0, c.stream>>>(c.g, l, d, side, per, m.ref, c.tag);
-                        launched(c, "periodic_tag");
+                        corner_item<DIM>(g, l, t, m.cells, m.ref, u, parts);
+                    }
+                    else
+                    {
+                        const FaceArgs a{l, l < g.max_level, l >= g.min_level && has_bc, l >= g.min_level && l < g.max_level};
+                        face_item<DIM>(g, a, t - nc, m.cells, m.uni, m.ref, u, 0.);
                     }
                 }
+                return;
             }
+            project_items<DIM>(g, l, m.wl_ref, m.lo, m.proj, static_cast<int>(((blockIdx.x - nb) * blockDim.x + threadIdx.x) >> 5),
+                               static_cast<int>(((gridDim.x - nb) * blockDim.x) >> 5),
+                               [&](long long w, int b, const Cell& c) { project_transpose<DIM>(g, u, 32 * w + b, l, c.x, c.y, c.z); });
         }
 
-        struct GhostChainArgs
-        {
-            int l_hi, l_lo; // levels of the chain, walked from l_hi down to l_lo
-            int lmin;       // lowest level holding reference cells
-            int has_bc;
-            double value;
-        };
-
-        // The small levels of the top-down pass in one block: the roles of
-        // k_ghost_level one level after the other.
-        template <int DIM>
-        __global__ void __launch_bounds__(1024, 1) k_ghost_levels_small(const __grid_constant__ Geom gp, GhostChainArgs ca, const int* wl_ref, const long long* lo, const uint32_t* cells,
-                                             const uint32_t* uni, const uint32_t* proj, const uint32_t* ref, ValAcc u)
-        {
-            const Geom& g         = gp;
-            const int minl        = g.min_level, maxl = g.max_level;
-            const int ndiag       = (DIM == 2) ? 4 : 20;
-            const long long warp0 = threadIdx.x >> 5;
-            const long long nw    = blockDim.x >> 5;
-            for (int l = ca.l_hi; l >= ca.l_lo; --l)
-            {
-                GhostLevelArgs a{};
-                a.l            = l;
-                a.do_project   = l < maxl;
-                a.do_dirichlet = (l >= minl) && ca.has_bc;
-                a.do_dirichlet_layer2 = a.do_dirichlet;
-                a.do_predict   = (l >= minl && l < maxl);
-                a.value        = ca.value;
-                if (l >= minl && l <= maxl)
-                {
-                    for (int k = 0; k < ndiag; ++k)
-                    {
-                        int d[3];
-                        diagonal_dir(DIM, k, d);
-                        corner_role(g, d, l, cells, ref, u);
-                    }
-                }
-                if (a.do_project || a.do_dirichlet || a.do_predict)
-                {
-                    const int n              = g.lv[l].n;
-                    const long long nfaces   = static_cast<long long>(2 * DIM) * ((DIM == 2) ? n : static_cast<long long>(n) * n);
-                    for (long long t = threadIdx.x; t < nfaces; t += blockDim.x)
-                    {
-                        face_work<DIM>(g, a, t, cells, uni, ref, u);
-                    }
-                }
-                if (l > ca.lmin)
-                {
-                    project_level<DIM>(g, l, wl_ref, lo, proj, ref, u, warp0, nw);
-                }
-                __syncthreads();
-            }
-        }
-
-        template <int DIM, class A>
-        __global__ void k_predict(const __grid_constant__ Geom gp, int l, int order, const int* wl_ref, const long long* lo, const uint32_t* cells,
-                                  const uint32_t* proj, const uint32_t* ref, A u)
-        {
-            predict_level<DIM>(gp, l, order, wl_ref, lo, cells, proj, ref, u, warp_id(), warp_count());
-        }
-
-        // the small levels of the bottom-up pass in one block
-        template <int DIM>
-        __global__ void __launch_bounds__(1024, 1) k_predict_small(const __grid_constant__ Geom gp, int l_lo, int l_hi, int order, const int* wl_ref, const long long* lo,
-                                        const uint32_t* cells, const uint32_t* proj, const uint32_t* ref, ValAcc u)
-        {
-            const long long warp0 = threadIdx.x >> 5;
-            const long long nw    = blockDim.x >> 5;
-            for (int l = l_lo; l <= l_hi; ++l)
-            {
-                predict_level<DIM>(gp, l, order, wl_ref, lo, cells, proj, ref, u, warp0, nw);
-                __syncthreads();
-            }
-        }
-
-        // -------------------------------------------------------- details
-        // compute_detail_op (mr/operators.hpp:139-540) on
-        // intersection(all_cells[l], union(cells[l+1], cells[l+2])).on(l)
-        template <int DIM>
-        __global__ void k_detail(const __grid_constant__ Geom gp, int order, const int* wl, const long long* lo, int l0, int l1, const int* d_ite,
-                                 const uint32_t* ref, const uint32_t* hc, const uint32_t* hc2, const double* u, double* det)
+        template <int DIM, int CAP>
+        __global__ void k_predict_reverse(const __grid_constant__ Geom gp, int l, int order, MeshPtrs m, RevAcc<CAP> u)
         {
             const Geom& g = gp;
-            // levels l0 .. min(l1, max_level - ite - 1) (mr/adapt.hpp:310-317)
-            const int le = min(l1, g.max_level - *d_ite - 1);
-            if (le < l0)
-            {
-                return;
-            }
-            warp_list_compact(wl, lo[LO_REF + l0], lo[LO_REF + le + 1], warp_id(), warp_count(), [&](long long w) { return ref[w] & (hc[w] | hc2[w]); },
-                      [&](long long w, int b)
-                      {
-                          const int l    = level_of(g, w);
-                          const Cell c   = cell_of(g, l, w, b);
-                          long long ce[8];
-                          const Box3 cb = box_at<DIM>(g, l + 1, 2 * c.x, 2 * c.y, 2 * c.z, 2);
-                          for (int ch = 0; ch < (1 << DIM); ++ch)
-                          {
-                              ce[ch] = cb.base + (ch & 1) + ((ch >> 1) & 1) * cb.sy + ((ch >> 2) & 1) * cb.sz;
-                          }
-                          if (order == 0)
-                          {
-                              const double uc = u[32 * w + b];
-                              for (int ch = 0; ch < (1 << DIM); ++ch)
-                              {
-                                  det[ce[ch]] = u[ce[ch]] - uc;
-                              }
-                              return;
-                          }
-                          double d[8];
-                          for (int ch = 0; ch < (1 << DIM); ++ch)
-                          {
-                              d[ch] = u[ce[ch]];
-                          }
-                          // d -= cf * src with cf = prod interp1 = +-8^-k (k = axes with
-                          // an off-centre tap): cf * src is +-(src * 8^-k) bit for bit
-                          // (power-of-two scaling is exact), and d - (-m) is d + m, so
-                          // one product per source serves all children
-                          const int nz  = (DIM == 3) ? 3 : 1;
-                          const Box3 sb = box_at<DIM>(g, l, c.x - 1, c.y - 1, c.z - 1, 3);
-#pragma unroll
-                          for (int sz = 0; sz < nz; ++sz)
-                          {
-#pragma unroll
-                              for (int sy = 0; sy < 3; ++sy)
-                              {
-                                  const long long base = sb.base + sy * sb.sy + sz * sb.sz;
-                                  for (int sx = 0; sx < 3; ++sx)
-                                  {
-                                      const double src = u[base + sx];
-                                      const int k      = (sx != 1) + (sy != 1) + (DIM == 3 && sz != 1);
-                                      const double m   = k == 0 ? src : scale8(src, k);
-                                      for (int ch = 0; ch < (1 << DIM); ++ch)
-                                      {
-                                          // interp1(parity, t) < 0: t == 0 on odd children, t == 2 on even ones
-                                          const int px = ch & 1, py = (ch >> 1) & 1, pz = (ch >> 2) & 1;
-                                          const bool neg = ((sx == 0 && px) || (sx == 2 && !px)) ^ ((sy == 0 && py) || (sy == 2 && !py))
-                                                           ^ (DIM == 3 && ((sz == 0 && pz) || (sz == 2 && !pz)));
-                                          d[ch]          = neg ? d[ch] + m : d[ch] - m;
-                                      }
-                                  }
-                              }
-                          }
-                          for (int ch = 0; ch < (1 << DIM); ++ch)
-                          {
-                              det[ce[ch]] = d[ch];
-                          }
-                      });
-        }
-
-        // mr_criteria_op (mr/criteria.hpp:20-113) on
-        // intersection(cells[l], all_cells[l-1]).on(l-1), fine levels l0..l1
-        template <int DIM>
-        __global__ void k_criteria(const __grid_constant__ Geom gp, const double* __restrict__ eps, const int* wl, const long long* lo, int l0, int l1,
-                                   const int* d_ite, const uint32_t* ref, const uint32_t* hc, const double* det, uint8_t* tag, int ncomp,
-                                   long long cstride)
-        {
-            // |detail| above a threshold in one of the components (one per
-            // adapted field, mr/criteria.hpp:45-107)
-            auto above = [&](long long e, double thr)
-            {
-                for (int k = 0; k < ncomp; ++k)
-                {
-                    if (fabs(det[k * cstride + e]) > thr)
-                    {
-                        return true;
-                    }
-                }
-                return false;
-            };
-            const Geom& g = gp;
-            // fine levels l0 .. min(l1, max_level - ite) (mr/adapt.hpp:325-339); the
-            // operator runs on their parents
-            const int le = min(l1, g.max_level - *d_ite);
-            if (le < l0)
-            {
-                return;
-            }
-            warp_list(wl, lo[LO_REF + l0 - 1], lo[LO_REF + le], warp_id(), warp_count(), [&](long long w) { return ref[w] & hc[w]; },
-                      [&](long long w, int b)
-                      {
-                          const int lc  = level_of(g, w);
-                          const int lf  = lc + 1;
-                          const Cell c  = cell_of(g, lc, w, b);
-                          long long fo[8];
-                          const Box3 fb = box_at<DIM>(g, lf, 2 * c.x, 2 * c.y, 2 * c.z, 2);
-                          for (int ch = 0; ch < (1 << DIM); ++ch)
-                          {
-                              fo[ch] = fb.base + (ch & 1) + ((ch >> 1) & 1) * fb.sy + ((ch >> 2) & 1) * fb.sz;
-                          }
-                          if (lf > g.min_level)
-                          {
-                              const bool cond = above(32 * w + b, eps[2 * MAXLEV + lf]);
-                              if (!cond)
-                              {
-                                  bool ok = true;
-                                  for (int ch = 0; ch < (1 << DIM); ++ch)
-                                  {
-                                      if (above(fo[ch], eps[lf]))
-                                      {
-                                          ok = false;
-                                          break;
-                                      }
-                                  }
-                                  if (ok)
-                                  {
-                                      for (int ch = 0; ch < (1 << DIM); ++ch)
-                                      {
-                                          tag[fo[ch]] = 2;
-                                      }
-                                  }
-                              }
-                          }
-                          if (lf < g.max_level)
-                          {
-                              for (int ch = 0; ch < (1 << DIM); ++ch)
-                              {
-                                  if (above(fo[ch], eps[MAXLEV + lf]))
-                                  {
-                                      tag[fo[ch]] |= 4;
-                                  }
-                              }
-                          }
-                      });
-        }
-
-        // compute_relative_detail (mr/rel_detail.hpp:75-111), for a scalar
-        // field: max |u| over the leaf cells (the bits of non-negative doubles
-        // order like the doubles, so an integer atomic max is exact and
-        // independent of the order), then every reference detail times
-        // 1 / max (1 when max is below the machine epsilon)
-        __global__ void k_absmax_init(unsigned long long* m)
-        {
-            *m = static_cast<unsigned long long>(__double_as_longlong(2.2250738585072014e-308)); // numeric_limits<double>::min()
-        }
-
-        __global__ void k_absmax(const int* wl, const long long* lo, int nlev, const uint32_t* cells, const double* u, unsigned long long* m)
-        {
-            const int lane    = threadIdx.x & 31;
-            unsigned long long best = 0;
-            for (long long i = lo[LO_CELLS] + warp_id(); i < lo[LO_CELLS + nlev]; i += warp_count())
-            {
-                const long long w = __ldg(wl + i);
-                if ((__ldg(cells + w) >> lane) & 1u)
-                {
-                    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(fabs(u[32 * w + lane])));
-                    best                       = b > best ? b : best;
-                }
-            }
-            for (int o = 16; o > 0; o >>= 1)
-            {
-                const unsigned long long x = __shfl_xor_sync(0xffffffffu, best, o);
-                best                       = x > best ? x : best;
-            }
-            if (lane == 0 && best)
-            {
-                atomicMax(m, best);
-            }
-        }
-
-        __global__ void k_rel_scale(const int* wl, const long long* lo, int nlev, const uint32_t* ref, const unsigned long long* m, double* det)
-        {
-            double mx = __longlong_as_double(static_cast<long long>(*m));
-            if (mx < 2.220446049250313e-16) // numeric_limits<double>::epsilon()
-            {
-                mx = 1.0;
-            }
-            const double inv = 1. / mx;
-            warp_list(wl, lo[LO_REF], lo[LO_REF + nlev], warp_id(), warp_count(), [&](long long w) { return ref[w]; },
-                      [&](long long w, int b) { det[32 * w + b] *= inv; });
-        }
-
-        // keep_boundary_refined (mr/adapt.hpp:245-274): in each Cartesian
-        // direction, the cells of max_level outside the domain translated by
-        // -max_stencil_radius times the direction (domain_boundary_layer,
-        // boundary.hpp:6-21), i.e. the leaves of max_level within r cells of
-        // the boundary, are tagged keep (the tag is overwritten)
-        __global__ void k_keep_boundary(const __grid_constant__ Geom gp, const int* wl, const long long* lo, const uint32_t* cells, int r, uint8_t* tag)
-        {
-            const Geom& g = gp;
-            const int l   = g.max_level;
-            warp_list(wl, lo[LO_CELLS + l], lo[LO_CELLS + l + 1], warp_id(), warp_count(),
-                      [&](long long w)
-                      {
-                          const WordLoc loc = word_loc(g, l, w);
-                          return cells[w] & ~box_mask(g, l, loc.row, loc.wi, -r, -r);
-                      },
-                      [&](long long w, int b) { tag[32 * w + b] = 1; });
-        }
-
-        // maximum_op (mr/operators.hpp:22-96), children at level l
-        template <int DIM>
-        __device__ __forceinline__ void maximum_level(const Geom& g, int l, const int* wl, const long long* lo, const uint32_t* ref, const uint32_t* hc,
-                                                      uint8_t* tag, long long warp0, long long nwarps)
-        {
-            const int lc = l - 1;
-            const LevelGeom& C = g.lv[lc];
-            warp_list(lo ? wl : nullptr, lo ? lo[LO_REF + lc] : C.woff, lo ? lo[LO_REF + l] : C.woff + C.nwords, warp0, nwarps,
-                      [&](long long w) { return ref[w] & hc[w]; },
-                      [&](long long w, int b)
-                      {
-                          const Cell c  = cell_of(g, lc, w, b);
-                          long long fo[8];
-                          uint8_t keep = 0, coarsen = 2;
-                          const Box3 fb = box_at<DIM>(g, l, 2 * c.x, 2 * c.y, 2 * c.z, 2);
-                          for (int ch = 0; ch < (1 << DIM); ++ch)
-                          {
-                              fo[ch] = fb.base + (ch & 1) + ((ch >> 1) & 1) * fb.sy + ((ch >> 2) & 1) * fb.sz;
-                              const uint8_t t = tag[fo[ch]];
-                              keep |= t & 1;
-                              coarsen &= t & 2;
-                          }
-                          const long long co = 32 * w + b;
-                          if (keep)
-                          {
-                              for (int ch = 0; ch < (1 << DIM); ++ch)
-                              {
-                                  tag[fo[ch]] |= 1;
-                              }
-                              tag[co] |= 1;
-                          }
-                          else if (coarsen)
-                          {
-                              tag[co] |= 1;
-                          }
-                          else
-                          {
-                              for (int ch = 0; ch < (1 << DIM); ++ch)
-                              {
-                                  tag[fo[ch]] &= static_cast<uint8_t>(~2);
-                              }
-                          }
-                      });
-        }
-
-        // byte-wise atomic OR / AND on the tag array (through its 32-bit word)
-        __device__ __forceinline__ void tag_or_atomic(uint8_t* t, unsigned v)
-        {
-            const unsigned long long a = reinterpret_cast<unsigned long long>(t);
-            atomicOr(reinterpret_cast<unsigned*>(a & ~3ull), v << (8 * (a & 3)));
-        }
-
-        __device__ __forceinline__ void tag_and_atomic(uint8_t* t, unsigned v)
-        {
-            const unsigned long long a = reinterpret_cast<unsigned long long>(t);
-            atomicAnd(reinterpret_cast<unsigned*>(a & ~3ull), ~((~v & 0xFFu) << (8 * (a & 3))));
-        }
-
-        // Two consecutive levels of maximum_op in one launch: the operator with children at level l (parents at
-        // l-1) and the one with children at level l-1 (parents at l-2), which in sequence runs after it.  A parent
-        // at l-2 needs the keep bits its children at l-1 carry after the first operator; it derives them itself
-        // from their children at l: keep(p) = keep bit of p, or p is a parent of leaves (reference and hc) whose
-        // children hold a keep bit or are all tagged coarsen.  Those inputs are the same before and after the
-        // first operator's writes (it sets keep bits on all children only when one already holds one, and clears
-        // coarsen bits only when not all hold one), so the two operators' threads run concurrently.  The bytes of
-        // level l-1, written by both, take atomic updates.
-        template <int DIM>
-        __global__ void k_maximum2(const __grid_constant__ Geom gp, int l, const int* wl, const long long* lo, const uint32_t* ref,
-                                   const uint32_t* hc, uint8_t* tag)
-        {
-            const Geom& g      = gp;
-            const long long w1 = g.lv[l - 1].woff; // first word of level l-1
-            const LevelGeom& C = g.lv[l - 1];
-            warp_list(lo ? wl : nullptr, lo ? lo[LO_REF + l - 2] : g.lv[l - 2].woff, lo ? lo[LO_REF + l] : C.woff + C.nwords, warp_id(), warp_count(),
-                      [&](long long w) { return ref[w] & hc[w]; },
-                      [&](long long w, int b)
-                      {
-                          const long long co = 32 * w + b;
-                          if (w >= w1)
-                          {
-                              // parent at l-1, children at l (maximum_op, mr/operators.hpp:22-96)
-                              const Cell c  = cell_of(g, l - 1, w, b);
-                              const Box3 fb = box_at<DIM>(g, l, 2 * c.x, 2 * c.y, 2 * c.z, 2);
-                              long long fo[8];
-                              uint8_t keep = 0, coarsen = 2;
-                              for (int ch = 0; ch < (1 << DIM); ++ch)
-                              {
-                                  fo[ch]          = fb.base + (ch & 1) + ((ch >> 1) & 1) * fb.sy + ((ch >> 2) & 1) * fb.sz;
-                                  const uint8_t t = tag[fo[ch]];
-                                  keep |= t & 1;
-                                  coarsen &= t & 2;
-                              }
-                              if (keep)
-                              {
-                                  for (int ch = 0; ch < (1 << DIM); ++ch)
-                                  {
-                                      tag[fo[ch]] |= 1;
-                                  }
-                                  tag_or_atomic(tag + co, 1u);
-                              }
-                              else if (coarsen)
-                              {
-                                  tag_or_atomic(tag + co, 1u);
-                              }
-                              else
-                              {
-                                  for (int ch = 0; ch < (1 << DIM); ++ch)
-                                  {
-                                      tag[fo[ch]] &= static_cast<uint8_t>(~2);
-                                  }
-                              }
-                              return;
-                          }
-                          // parent at l-2, children p at l-1
-                          const Cell c  = cell_of(g, l - 2, w, b);
-                          const Box3 pb = box_at<DIM>(g, l - 1, 2 * c.x, 2 * c.y, 2 * c.z, 2);
-                          long long po[8];
-                          uint8_t keep = 0, coarsen = 2;
-                          for (int ch = 0; ch < (1 << DIM); ++ch)
-                          {
-                              const int px = 2 * c.x + (ch & 1), py = 2 * c.y + ((ch >> 1) & 1), pz = 2 * c.z + ((ch >> 2) & 1);
-                              po[ch]          = pb.base + (ch & 1) + ((ch >> 1) & 1) * pb.sy + ((ch >> 2) & 1) * pb.sz;
-                              const uint8_t t = tag[po[ch]];
-                              uint8_t k       = t & 1;
-                              const Pos pp    = pos_of(g, l - 1, px, py, DIM == 3 ? pz : 0);
-                              if (!k && test(ref, pp) && test(hc, pp))
-                              {
-                                  // p's own operator: a child's keep bit, or all children tagged coarsen
-                                  const Box3 fb = box_at<DIM>(g, l, 2 * px, 2 * py, 2 * pz, 2);
-                                  uint8_t ck = 0, cc = 2;
-                                  for (int gc = 0; gc < (1 << DIM); ++gc)
-                                  {
-                                      const uint8_t tt = tag[fb.base + (gc & 1) + ((gc >> 1) & 1) * fb.sy + ((gc >> 2) & 1) * fb.sz];
-                                      ck |= tt & 1;
-                                      cc &= tt & 2;
-                                  }
-                                  k = (ck | cc) ? 1 : 0;
-                              }
-                              keep |= k;
-                              coarsen &= t & 2;
-                          }
-                          if (keep)
-                          {
-                              for (int ch = 0; ch < (1 << DIM); ++ch)
-                              {
-                                  tag_or_atomic(tag + po[ch], 1u);
-                              }
-                              tag[co] |= 1;
-                          }
-                          else if (coarsen)
-                          {
-                              tag[co] |= 1;
-                          }
-                          else
-                          {
-                              for (int ch = 0; ch < (1 << DIM); ++ch)
-                              {
-                                  tag_and_atomic(tag + po[ch], static_cast<unsigned>(static_cast<uint8_t>(~2)));
-                              }
-                          }
-                      });
-        }
-
-        template <int DIM>
-        __global__ void k_maximum(const __grid_constant__ Geom gp, int l, const int* wl, const long long* lo, const uint32_t* ref, const uint32_t* hc,
-                                  uint8_t* tag)
-        {
-            maximum_level<DIM>(gp, l, wl, lo, ref, hc, tag, warp_id(), warp_count());
-        }
-
-        // the small levels of the tag finalisation in one block, l_hi down to l_lo
-        template <int DIM>
-        __global__ void __launch_bounds__(1024, 1) k_maximum_small(const __grid_constant__ Geom gp, int l_hi, int l_lo, const int* wl, const long long* lo,
-                                                                   const uint32_t* ref, const uint32_t* hc, uint8_t* tag)
-        {
-            const long long warp0 = threadIdx.x >> 5;
-            const long long nw    = blockDim.x >> 5;
-            for (int l = l_hi; l >= l_lo; --l)
-            {
-                maximum_level<DIM>(gp, l, wl, lo, ref, hc, tag, warp0, nw);
-                __syncthreads();
-            }
+            predict_items<DIM>(g, l, m.wl_ref, m.lo, m.pred, static_cast<int>(warp_id()), static_cast<int>(warp_count()),
+                               [&](long long w, int b, const Cell& c) { predict_transpose<DIM>(g, u, 32 * w + b, l, c.x, c.y, c.z, order); });
         }
 
         // update_fields (algorithm/update_fields.hpp:27-127): copy on
         // reference ∩ new cells, projection on coarsened cells, prediction on
         // refined cells; every other reference entry of the new field is 0.
         template <int DIM, class A>
-        __global__ void k_update_fields(const __grid_constant__ Geom gp, int order, const int* wl, const long long* lo, const uint32_t* nref,
+        __global__ void k_update_fields_reverse(const __grid_constant__ Geom gp, int order, const int* wl, const long long* lo, const uint32_t* nref,
                                         const uint32_t* ncells, const uint32_t* oref, const uint32_t* ocells, const uint32_t* ohc, A uo, A un)
         {
             const Geom& g = gp;
@@ -1484,6 +203,7 @@ namespace sg
 
         struct UpwindArgs
         {
+            double a[3];
             double ha[3]; // .5 * a_d, as the reference's flux forms it
             double hb[3]; // .5 * |a_d|
             double dt;
@@ -1500,7 +220,7 @@ namespace sg
         //    operations, same bits) and passed by a shuffle;
         //  - /dx and dt/dx use dx = 2^-l exactly: x / 2^-l == x * 2^l.
         template <int DIM>
-        __global__ void k_upwind(const __grid_constant__ Geom gp, const int* wl, const long long* lo, const uint32_t* cells, const double* __restrict__ u,
+        __global__ void k_upwind(const __grid_constant__ Geom gp, const int* __restrict__ wl, const long long* __restrict__ lo, const uint32_t* __restrict__ cells, const double* __restrict__ u,
                                  double* __restrict__ unp1, UpwindArgs p)
         {
             const Geom& g  = gp;
@@ -1509,7 +229,7 @@ namespace sg
             // flux is its left neighbour's right flux when that neighbour is the
             // previous lane's cell (the same face, the same expression)
             const long long nb = lo[LO_CELLS], ne = lo[LO_CELLS + g.nlev];
-            warp_items(wl, nb, ne, warp_id(), warp_count(), items_chunk(ne - nb, warp_count()), [&](long long w) { return __ldg(cells + w); },
+            warp_items(wl, nb, ne, warp_id(), warp_count(), items_chunk(ne - nb, warp_count()), [&](long long w) { return cells[w]; },
                            [&](bool valid, long long w, int b)
                            {
                                int l = 0;
@@ -1605,12 +325,12 @@ namespace sg
         // coefficients (a, 0) for a >= 0, (0, a) otherwise; every factor is a
         // power of two.
         template <int DIM>
-        __global__ void k_convection(const __grid_constant__ Geom gp, const int* wl, const long long* lo, const uint32_t* cells, const double* __restrict__ u,
-                                     double* __restrict__ unp1, UpwindArgs p, const double* __restrict__ av)
+        __global__ void k_convection(const __grid_constant__ Geom gp, const int* __restrict__ wl, const long long* __restrict__ lo, const uint32_t* __restrict__ cells, const double* __restrict__ u,
+                                     double* __restrict__ unp1, UpwindArgs p)
         {
             const Geom& g     = gp;
             const long long n = lo[LO_CELLS + g.nlev];
-            warp_list_compact(wl, lo[LO_CELLS], n, warp_id(), warp_count(), [&](long long w) { return __ldg(cells + w); },
+            warp_list_compact(wl, lo[LO_CELLS], n, warp_id(), warp_count(), [&](long long w) { return cells[w]; },
                               [&](long long w, int b)
                               {
                                   const int m        = level_of(g, w);
@@ -1619,12 +339,16 @@ namespace sg
                                   const long long eX = 32 * w + b;
                                   const double uX    = u[eX];
                                   const int nm       = 1 << m;
-                                  auto leaf = [&](int l, const int* q) { return l >= 0 && l <= g.max_level && test(cells, g, l, q[0], q[1], DIM == 3 ? q[2] : 0); };
+                                  auto leaf = [&](int l, const int* q)
+                                  {
+                                      const Pos at = l >= 0 && l <= g.max_level ? pos_of(g, l, q[0], q[1], DIM == 3 ? q[2] : 0) : Pos{-1, 0};
+                                      return at.w >= 0 && ((__ldg(cells + at.w) >> at.b) & 1u);
+                                  };
                                   auto val  = [&](int l, const int* q) { return u[elem_at(g, l, q[0], q[1], DIM == 3 ? q[2] : 0)]; };
                                   double acc = 0.;
                                   for (int d = 0; d < DIM; ++d)
                                   {
-                                      const double a  = av[d];
+                                      const double a  = p.a[d];
                                       const double fl = a >= 0 ? a : 0.;
                                       const double fr = a >= 0 ? 0. : a;
                                       int xp[3] = {c[0], c[1], c[2]}, xm[3] = {c[0], c[1], c[2]};
@@ -1774,6 +498,37 @@ namespace sg
                       [&](long long w, int b) { dense[32 * w + b] = compact[ref_index(ref, rank, Pos{w, b})]; });
         }
 
+        // details in the reference numbering: a cell whose parent the pass did not examine has none (0)
+        template <int DIM>
+        __global__ void k_gather_details(const __grid_constant__ Geom gp, MeshPtrs m, const PassSetup* setup, const double* det, double* compact)
+        {
+            const Geom& g = gp;
+            const int dl0 = max(g.min_level - 1, 0), le = g.max_level - setup->ite - 1;
+            warp_list(m.wl_ref, m.lo[LO_REF], m.lo[LO_REF + g.nlev], warp_id(), warp_count(), [&](long long w) { return m.ref[w]; },
+                      [&](long long w, int b)
+                      {
+                          const int l     = level_down(g, static_cast<int>(w), 0, g.max_level);
+                          bool examined   = false;
+                          if (l - 1 >= dl0 && l - 1 <= le)
+                          {
+                              const Cell c = cell_of(g, l, w, b);
+                              const Pos p  = pos_of(g, l - 1, c.x >> 1, c.y >> 1, DIM == 3 ? c.z >> 1 : 0);
+                              examined     = test(m.ref, p) && (test(m.hc, p) || test(m.hc2, p));
+                          }
+                          compact[ref_index(m.ref, m.rank, Pos{w, b})] = examined ? det[32 * w + b] : 0.;
+                      });
+        }
+
+        __global__ void k_tag_bytes(MeshPtrs m, int nlev, const uint32_t* tk, const uint32_t* tc, const uint32_t* tr, uint8_t* compact)
+        {
+            warp_list(m.wl_ref, m.lo[LO_REF], m.lo[LO_REF + nlev], warp_id(), warp_count(), [&](long long w) { return m.ref[w]; },
+                      [&](long long w, int b)
+                      {
+                          const uint32_t t = ((tk[w] >> b) & 1u) | (((tc[w] >> b) & 1u) << 1) | (((tr[w] >> b) & 1u) << 2);
+                          compact[ref_index(m.ref, m.rank, Pos{w, b})] = static_cast<uint8_t>(t);
+                      });
+        }
+
         __global__ void k_fill(const int* wl, const long long* lo, int nlev, const uint32_t* ref, double* dense, double v)
         {
             warp_list(wl, lo[LO_REF], lo[LO_REF + nlev], warp_id(), warp_count(), [&](long long w) { return ref[w]; }, [&](long long w, int b) { dense[32 * w + b] = v; });
@@ -1799,20 +554,6 @@ namespace sg
         }
     } // namespace
 
-    namespace
-    {
-        // the offsets argument of a level-chain launch over levels l0..l1: null (the dense word range, no list)
-        // when the launch's grid gives every word of those levels a warp of its own, else the mesh's offsets
-        const long long* level_offsets(const Ctx& c, const DeviceMesh& m, int l0, int l1)
-        {
-            const Geom& g       = c.g;
-            const long long wpb = c.block / 32;
-            const long long cap = std::max(1LL, c.max_blocks * 8 / wpb) * wpb;
-            const long long n   = g.lv[l1].woff + g.lv[l1].nwords - g.lv[l0].woff;
-            return n <= cap ? nullptr : m.d_lo;
-        }
-    } // namespace
-
     cudaError_t launch_gather(Ctx& c, const DeviceMesh& m, const double* dense, double* compact)
     {
         k_gather<<<blocks_words(c, 0, c.g.nlev - 1), c.block, 0, c.stream>>>(m.wl_ref, m.d_lo, c.g.nlev, m.ref, m.rank, dense, compact);
@@ -1828,6 +569,27 @@ namespace sg
             return SG_ERR_CUDA;
         }
         return SG_OK;
+    }
+
+    int gather_details(Ctx& c, const DeviceMesh& m, double* compact)
+    {
+        if (c.g.dim == 2)
+        {
+            k_gather_details<2><<<blocks_words(c, 0, c.g.nlev - 1), c.block, 0, c.stream>>>(c.g, mesh_ptrs(m), c.d_setup, c.detail, compact);
+        }
+        else
+        {
+            k_gather_details<3><<<blocks_words(c, 0, c.g.nlev - 1), c.block, 0, c.stream>>>(c.g, mesh_ptrs(m), c.d_setup, c.detail, compact);
+        }
+        launched(c, "gather");
+        return check(c, "gather_details");
+    }
+
+    int tag_bytes(Ctx& c, const DeviceMesh& m, uint8_t* compact)
+    {
+        k_tag_bytes<<<blocks_words(c, 0, c.g.nlev - 1), c.block, 0, c.stream>>>(mesh_ptrs(m), c.g.nlev, c.tk, c.tc, c.tr, compact);
+        launched(c, "gather");
+        return check(c, "tag_bytes");
     }
 
     cudaError_t read_device_error(Ctx& c, int* v)
@@ -2111,24 +873,17 @@ namespace sg
 
     namespace
     {
-        // the Harten pass index and the criteria thresholds of one pass, baked
-        // into a captured graph (the host computes them exactly as for the
-        // staged copies of the per-pass path)
-        struct PassSetup
-        {
-            double eps[3 * MAXLEV];
-            int ite;
-        };
-
-        __global__ void k_pass_setup(PassSetup p, double* d_eps, int* d_ite)
+        // the setup of one pass baked into a captured graph (the host computes
+        // it exactly as for the staged copy of the per-pass path)
+        __global__ void k_pass_setup(PassSetup p, PassSetup* d)
         {
             for (int i = threadIdx.x; i < 3 * MAXLEV; i += blockDim.x)
             {
-                d_eps[i] = p.eps[i];
+                d->eps[i] = p.eps[i];
             }
             if (threadIdx.x == 0)
             {
-                *d_ite = p.ite;
+                d->ite = p.ite;
             }
         }
 
@@ -2272,348 +1027,192 @@ namespace sg
         }
 
         // update_ghost_mr / update_ghost_mr_aggregated (algorithm/update_ghost_mr.hpp:195-270)
-        // as a sequence of launches on accessor u.  ft: levels 0..ft run as
-        // one-block chains (value accessor only; -2 for none).  split: the
-        // corner projection of each level gets a launch of its own, so that
-        // no launch reads what it writes (needed to record the operator).
-        // after() runs after every launch.
-        template <class A, class After>
-        int ghost_launches(Ctx& c, DeviceMesh& m, const A& u, bool has_bc, double bcv, int ft, bool split, After after)
+        // of the sequence's fields.  update_ghost_periodic runs after the boundary
+        // conditions of a level and after its prediction
+        // (update_ghost_mr.hpp:205-234); the copy the reference also makes before
+        // the boundary conditions is overwritten by this one before anything
+        // reads it: the boundary conditions of a serial run read and write no
+        // ghost across a periodic axis.
+        void ghost_phases(Sequence& s)
         {
-            const Geom& g   = c.g;
-            if (g.periodic)
+            const Geom& g  = s.c.g;
+            const int lmin = g.min_level >= 2 ? g.min_level - 2 : 0; // no reference cell below min_level-2
+            auto periodic  = [&](int l)
             {
-                // the periodic copies sit between the levels of both passes: no
-                // level is fused into a one-block chain
-                ft = -2 * MAXLEV;
-            }
-            // update_ghost_periodic after the boundary conditions of a level and
-            // after its prediction (update_ghost_mr.hpp:205-234).  The copy the
-            // reference also makes before the boundary conditions is overwritten
-            // by this one before anything reads it: the boundary conditions of a
-            // serial run read and write no ghost across a periodic axis.
-            auto periodic = [&](int lev)
-            {
-                if constexpr (std::is_same<A, ValAcc>::value)
+                for (int d = 0; d < g.dim; ++d)
                 {
-                    if (g.periodic)
+                    if ((g.periodic >> d) & 1)
                     {
-                        periodic_copies(c, m, lev, u.u);
-                        after();
+                        s.add(OP_PERIODIC_COPY, l, l, d); // a later axis reads the ghosts an earlier one wrote
                     }
                 }
             };
-            const int minl  = c.cfg.min_level;
-            const int maxl  = c.cfg.max_level;
-            const int lmin  = minl >= 2 ? minl - 2 : 0; // no reference cell below min_level-2
-            const int ndiag = (g.dim == 2) ? 4 : 20;
-            int l           = maxl;
-            for (; l >= lmin && l - 1 > ft; --l)
+            for (int l = g.max_level; l >= lmin; --l)
             {
-                GhostLevelArgs a{};
-                a.l            = l;
-                a.do_corners   = (l >= minl && l <= maxl) ? 1 : 0;
-                a.do_project   = l < maxl;
-                a.do_dirichlet = (l >= minl) && has_bc;
-                a.do_dirichlet_layer2 = a.do_dirichlet;
-                a.do_predict   = (l >= minl && l < maxl);
-                a.value        = bcv;
-                a.nb_corner    = a.do_corners ? ndiag : 0;
-                a.corner_parts = split ? 1 : 3;
-                const int n    = g.lv[l].n;
-                a.nfaces       = (a.do_project || a.do_dirichlet || a.do_predict)
-                                     ? static_cast<long long>(2 * g.dim) * ((g.dim == 2) ? n : static_cast<long long>(n) * n)
-                                     : 0;
-                a.nb_face         = static_cast<int>((a.nfaces + c.block - 1) / c.block);
-                a.do_proj         = l > lmin;
-                const int nb_proj = a.do_proj ? blocks_words(c, l - 1, l - 1) : 0;
-                const long long* proj_lo = a.do_proj ? level_offsets(c, m, l - 1, l - 1) : m.d_lo;
-                const int grid    = a.nb_corner + a.nb_face + nb_proj;
-                if (grid > 0)
-                {
-                    if (g.dim == 2)
-                    {
-                        k_ghost_level<2><<<grid, c.block, 0, c.stream>>>(c.g, a, m.wl_ref, proj_lo, m.cells, m.uni, m.proj, m.ref, u);
-                    }
-                    else
-                    {
-                        k_ghost_level<3><<<grid, c.block, 0, c.stream>>>(c.g, a, m.wl_ref, proj_lo, m.cells, m.uni, m.proj, m.ref, u);
-                    }
-                    launched(c, "ghost_level");
-                    after();
-                }
-                if (split && a.nb_corner > 0)
-                {
-                    GhostLevelArgs b = a;
-                    b.corner_parts   = 2;
-                    b.nb_face        = 0;
-                    b.nfaces         = 0;
-                    b.do_proj        = 0;
-                    if (g.dim == 2)
-                    {
-                        k_ghost_level<2><<<b.nb_corner, c.block, 0, c.stream>>>(c.g, b, m.wl_ref, m.d_lo, m.cells, m.uni, m.proj, m.ref, u);
-                    }
-                    else
-                    {
-                        k_ghost_level<3><<<b.nb_corner, c.block, 0, c.stream>>>(c.g, b, m.wl_ref, m.d_lo, m.cells, m.uni, m.proj, m.ref, u);
-                    }
-                    launched(c, "ghost_corner_projection");
-                    after();
-                }
+                s.add(OP_GHOST, l, 0);
                 periodic(l);
             }
-            const int lp0 = lmin > 1 ? lmin : 1;
-            int lp        = lp0;
-            if constexpr (std::is_same<A, ValAcc>::value)
+            for (int l = std::max(lmin, 1); l <= g.max_level; ++l)
             {
-                if (l >= lmin)
+                s.add(OP_PREDICT, l, l);
+                periodic(l);
+            }
+        }
+
+        // the same transposed, launch by launch in forward order (run_reversed turns the captured chain round)
+        template <int DIM>
+        int ghost_reverse_launches(Ctx& c, const DeviceMesh& dm, double* lam, int* overflow, bool has_bc)
+        {
+            const Geom& g    = c.g;
+            const MeshPtrs m = mesh_ptrs(dm);
+            const RevAcc<FormCap<DIM>::value> u{lam, lam, overflow, 1};
+            const int lmin = g.min_level >= 2 ? g.min_level - 2 : 0;
+            for (int l = g.max_level; l >= lmin; --l)
+            {
+                const int nb = static_cast<int>(std::min(16384LL, (boundary_count<DIM>(g, l) + c.block - 1) / c.block));
+                const int np = l > lmin ? blocks_words(c, l - 1, l - 1) : 0;
+                if (nb + np > 0)
                 {
-                    GhostChainArgs ca{l, lmin, lmin, has_bc ? 1 : 0, bcv};
-                    if (g.dim == 2)
-                    {
-                        k_ghost_levels_small<2><<<1, 1024, 0, c.stream>>>(c.g, ca, m.wl_ref, m.d_lo, m.cells, m.uni, m.proj, m.ref, u);
-                    }
-                    else
-                    {
-                        k_ghost_levels_small<3><<<1, 1024, 0, c.stream>>>(c.g, ca, m.wl_ref, m.d_lo, m.cells, m.uni, m.proj, m.ref, u);
-                    }
-                    launched(c, "ghost_levels_small");
-                    after();
+                    k_ghost_reverse<DIM><<<nb + np, c.block, 0, c.stream>>>(c.g, l, 1, nb, has_bc ? 1 : 0, m, u);
+                    launched(c, "ghost_level");
                 }
-                if (lp <= maxl && lp <= ft)
+                if (l >= g.min_level)
                 {
-                    const int e = maxl < ft ? maxl : ft;
-                    if (g.dim == 2)
-                    {
-                        k_predict_small<2><<<1, 1024, 0, c.stream>>>(c.g, lp, e, c.cfg.prediction_radius, m.wl_ref, m.d_lo, m.cells, m.proj, m.ref, u);
-                    }
-                    else
-                    {
-                        k_predict_small<3><<<1, 1024, 0, c.stream>>>(c.g, lp, e, c.cfg.prediction_radius, m.wl_ref, m.d_lo, m.cells, m.proj, m.ref, u);
-                    }
-                    launched(c, "predict_small");
-                    after();
-                    lp = e + 1;
+                    const int ncb = static_cast<int>(std::min(16384LL, (corner_count<DIM>(g, l) + c.block - 1) / c.block));
+                    k_ghost_reverse<DIM><<<ncb, c.block, 0, c.stream>>>(c.g, l, 2, ncb, has_bc ? 1 : 0, m, u);
+                    launched(c, "ghost_corner_projection");
                 }
             }
-            for (; lp <= maxl; ++lp)
+            for (int l = std::max(lmin, 1); l <= g.max_level; ++l)
             {
-                if (g.dim == 2)
-                {
-                    k_predict<2><<<blocks_words(c, lp, lp), c.block, 0, c.stream>>>(c.g, lp, c.cfg.prediction_radius, m.wl_ref, level_offsets(c, m, lp, lp), m.cells, m.proj,
-                                                                                   m.ref, u);
-                }
-                else
-                {
-                    k_predict<3><<<blocks_words(c, lp, lp), c.block, 0, c.stream>>>(c.g, lp, c.cfg.prediction_radius, m.wl_ref, level_offsets(c, m, lp, lp), m.cells, m.proj,
-                                                                                   m.ref, u);
-                }
+                k_predict_reverse<DIM><<<blocks_words(c, l, l), c.block, 0, c.stream>>>(c.g, l, c.cfg.prediction_radius, m, u);
                 launched(c, "predict");
-                after();
-                periodic(lp);
             }
-            return check(c, "update_ghost_mr");
+            return check(c, "update_ghost_mr (transpose)");
+        }
+
+        FieldSlot slot_of(const DeviceField& f)
+        {
+            return {f.data, f.spare, f.bc_value, f.has_bc ? 1 : 0};
+        }
+
+        std::vector<FieldSlot> slots_of(const std::vector<DeviceField*>& fs)
+        {
+            std::vector<FieldSlot> v;
+            for (const DeviceField* f : fs)
+            {
+                v.push_back(slot_of(*f));
+            }
+            return v;
+        }
+
+        // body(first, n) on groups of at most PHASE_FIELDS fields
+        template <class Body>
+        void field_groups(Sequence& s, const std::vector<FieldSlot>& fs, Body body)
+        {
+            for (int k = 0; k < static_cast<int>(fs.size()); k += PHASE_FIELDS)
+            {
+                s.fields(fs.data(), k, std::min(PHASE_FIELDS, static_cast<int>(fs.size()) - k));
+                body();
+            }
         }
 
         int seq_ghost(Ctx& c, DeviceMesh& m, double* u, bool has_bc, double bcv)
         {
             ScopedTimer timer(c, T_GHOST);
-            return ghost_launches(c, m, ValAcc{u}, has_bc, bcv, c.fuse_top_field, false, [] {});
-        }
-
-        // update_fields (algorithm/update_fields.hpp:27-127) from mesh m to nm
-        template <class A>
-        void update_fields_launch(Ctx& c, DeviceMesh& m, DeviceMesh& nm, const A& uo, const A& un)
-        {
-            const Geom& g = c.g;
-            if (g.dim == 2)
-            {
-                k_update_fields<2><<<blocks_words(c, 0, g.nlev - 1), c.block, 0, c.stream>>>(c.g, c.cfg.prediction_radius, nm.wl_ref, nm.d_lo, nm.ref,
-                                                                                            nm.cells, m.ref, m.cells, m.hc, uo, un);
-            }
-            else
-            {
-                k_update_fields<3><<<blocks_words(c, 0, g.nlev - 1), c.block, 0, c.stream>>>(c.g, c.cfg.prediction_radius, nm.wl_ref, nm.d_lo, nm.ref,
-                                                                                            nm.cells, m.ref, m.cells, m.hc, uo, un);
-            }
-            launched(c, "update_fields");
+            Sequence s(c, m, m);
+            const FieldSlot f{u, nullptr, bcv, has_bc ? 1 : 0};
+            s.fields(&f, 0, 1);
+            ghost_phases(s);
+            return s.done("update_ghost_mr");
         }
 
         // Adapt::harten up to the fixed-point test (mr/adapt.hpp:276-375):
-        // tags, ghost update, details, criteria, tag finalisation, new cells,
-        // two graduation passes and the comparison with the current cells.
-        // Reads the pass index and thresholds staged in pinned memory; leaves
-        // the flags in pinned memory.  No host synchronisation.
+        // ghost update, details, tags, new cells, graduation and the comparison
+        // with the current cells.  Reads the pass setup staged in pinned memory;
+        // leaves the flags in pinned memory.  No host synchronisation.
         // The fields fs drive the criteria, one detail component each, the
         // components stored one dense slab after the other.
         int seq_front(Ctx& c, DeviceMesh& m, DeviceMesh& nm, const std::vector<DeviceField*>& fs, const PassSetup* graphed = nullptr)
         {
             const Geom& g  = c.g;
-            const int minl = c.cfg.min_level;
-            const int maxl = c.cfg.max_level;
-            const int nf   = static_cast<int>(fs.size());
-            int st;
+            const int minl = g.min_level;
+            const int maxl = g.max_level;
             if (graphed)
             {
-                k_pass_setup<<<1, 128, 0, c.stream>>>(*graphed, c.d_eps, c.d_ite);
+                k_pass_setup<<<1, 128, 0, c.stream>>>(*graphed, c.d_setup);
                 launched(c, "pass_setup");
             }
             else
             {
-                cudaMemcpyAsync(c.d_ite, c.h_ite, sizeof(int), cudaMemcpyHostToDevice, c.stream);
-                cudaMemcpyAsync(c.d_eps, c.h_eps, 3 * MAXLEV * sizeof(double), cudaMemcpyHostToDevice, c.stream);
+                cudaMemcpyAsync(c.d_setup, c.h_setup, sizeof(PassSetup), cudaMemcpyHostToDevice, c.stream);
             }
-            cudaMemsetAsync(c.d_flags, 0, F_COUNT * sizeof(int), c.stream);
-            k_tag_init<<<blocks_words(c, 0, g.nlev - 1), c.block, 0, c.stream>>>(c.g, m.wl_ref, m.d_lo, m.ref, m.cells, c.tag, c.detail);
-            launched(c, "tag_init");
-            for (int k = 1; k < nf; ++k)
-            {
-                k_fill<<<blocks_words(c, 0, g.nlev - 1), c.block, 0, c.stream>>>(m.wl_ref, m.d_lo, g.nlev, m.ref, c.detail + k * c.capacity, 0.);
-                launched(c, "fill");
-            }
-            if ((st = check(c, "tag_init")))
-            {
-                return st;
-            }
-            for (DeviceField* f : fs)
-            {
-                if ((st = seq_ghost(c, m, f->data, f->has_bc, f->bc_value)))
-                {
-                    return st;
-                }
-            }
+            const std::vector<FieldSlot> slots = slots_of(fs);
+            Sequence s(c, m, nm);
+            s.add(OP_PASS_BEGIN);
+            s.timer_start(T_GHOST);
+            field_groups(s, slots, [&]() { ghost_phases(s); });
+            s.timer_stop(T_GHOST);
 
-            timer_start(c, T_DETAIL);
+            s.timer_start(T_DETAIL);
             const int dl0 = minl > 0 ? minl - 1 : 0;
             const int dl1 = maxl - 1;
-            for (int k = 0; k < nf && dl1 >= dl0; ++k)
+            if (dl1 >= dl0)
             {
-                const double* u = fs[k]->data;
-                double* det     = c.detail + k * c.capacity;
-                if (g.dim == 2)
-                {
-                    k_detail<2><<<blocks_words(c, dl0, dl1), c.block, 0, c.stream>>>(c.g, c.cfg.prediction_radius, m.wl_ref, m.d_lo, dl0, dl1, c.d_ite,
-                                                                                    m.ref, m.hc, m.hc2, u, det);
-                }
-                else
-                {
-                    k_detail<3><<<blocks_words(c, dl0, dl1), c.block, 0, c.stream>>>(c.g, c.cfg.prediction_radius, m.wl_ref, m.d_lo, dl0, dl1, c.d_ite,
-                                                                                    m.ref, m.hc, m.hc2, u, det);
-                }
-                launched(c, "detail");
+                field_groups(s, slots,
+                             [&]()
+                             {
+                                 if (c.rel_detail)
+                                 {
+                                     s.add(OP_ABSMAX_INIT);
+                                     s.add(OP_ABSMAX);
+                                 }
+                                 s.add(OP_DETAIL, dl0, dl1);
+                             });
             }
-            for (int k = 0; k < nf && c.rel_detail; ++k)
-            {
-                k_absmax_init<<<1, 1, 0, c.stream>>>(c.d_absmax);
-                k_absmax<<<blocks_words(c, 0, g.nlev - 1), c.block, 0, c.stream>>>(m.wl_cells, m.d_lo, g.nlev, m.cells, fs[k]->data, c.d_absmax);
-                k_rel_scale<<<blocks_words(c, 0, g.nlev - 1), c.block, 0, c.stream>>>(m.wl_ref, m.d_lo, g.nlev, m.ref, c.d_absmax, c.detail + k * c.capacity);
-                launched(c, "absmax", 3);
-            }
-            timer_stop(c, T_DETAIL);
+            s.timer_stop(T_DETAIL);
 
-            timer_start(c, T_TAG);
-            if (minl >= 1 && maxl >= minl)
-            {
-                if (g.dim == 2)
-                {
-                    k_criteria<2><<<blocks_words(c, minl - 1, maxl - 1), c.block, 0, c.stream>>>(c.g, c.d_eps, m.wl_ref, m.d_lo, minl, maxl, c.d_ite,
-                                                                                                m.ref, m.hc, c.detail, c.tag, nf, c.capacity);
-                }
-                else
-                {
-                    k_criteria<3><<<blocks_words(c, minl - 1, maxl - 1), c.block, 0, c.stream>>>(c.g, c.d_eps, m.wl_ref, m.d_lo, minl, maxl, c.d_ite,
-                                                                                                m.ref, m.hc, c.detail, c.tag, nf, c.capacity);
-                }
-                launched(c, "criteria");
-            }
-            if (c.refine_boundary)
-            {
-                // "refine boundary" (mr/adapt.hpp:341-346), between tag cells and tag finalization
-                k_keep_boundary<<<blocks_words(c, maxl, maxl), c.block, 0, c.stream>>>(c.g, m.wl_cells, m.d_lo, m.cells, c.cfg.max_stencil_radius,
-                                                                                   c.tag);
-                launched(c, "keep_boundary");
-            }
-            timer_stop(c, T_TAG);
+            s.timer_start(T_TAG);
+            s.add(OP_CRITERIA);
+            s.timer_stop(T_TAG);
 
-            timer_start(c, T_FINALIZE);
+            // children at levels maxl .. min_level: below min_level no parent has a leaf child, so the operator has
+            // nothing to do there; periodic axes: update_tag_periodic before each level's operator, and on the
+            // levels below too (mr/adapt.hpp:348-357)
+            s.timer_start(T_FINALIZE);
+            for (int l = maxl; l >= 1; --l)
             {
-                // children at levels maxl .. min_level: below min_level no parent
-                // has a leaf child, so the operator has nothing to do there
-                const int lstop = std::max(1, c.cfg.min_level);
-                int l           = maxl;
-                // periodic axes: update_tag_periodic before each level's operator
-                // (mr/adapt.hpp:348-357), so no level is fused into a one-block chain
-                const int top   = g.periodic ? -2 * MAXLEV : c.fuse_top_max;
-                while (l >= lstop && l - 1 > top)
+                for (int d = 0; d < g.dim; ++d)
                 {
-                    periodic_tags(c, m, l);
-                    if (c.level_pairs && !g.periodic && l - 1 >= lstop && l - 2 > top)
+                    for (int side = 0; side < 2 && ((g.periodic >> d) & 1); ++side)
                     {
-                        // children at levels l and l-1 in one launch
-                        if (g.dim == 2)
-                        {
-                            k_maximum2<2><<<blocks_words(c, l - 2, l - 1), c.block, 0, c.stream>>>(c.g, l, m.wl_ref, level_offsets(c, m, l - 2, l - 1), m.ref, m.hc,
-                                                                                         c.tag);
-                        }
-                        else
-                        {
-                            k_maximum2<3><<<blocks_words(c, l - 2, l - 1), c.block, 0, c.stream>>>(c.g, l, m.wl_ref, level_offsets(c, m, l - 2, l - 1), m.ref, m.hc,
-                                                                                         c.tag);
-                        }
-                        launched(c, "maximum"); // the trace groups the one- and two-level launches
-                        l -= 2;
-                        continue;
+                        s.add(OP_PERIODIC_TAG, l, l, 2 * d + side);
                     }
-                    if (g.dim == 2)
-                    {
-                        k_maximum<2><<<blocks_words(c, l - 1, l - 1), c.block, 0, c.stream>>>(c.g, l, m.wl_ref, level_offsets(c, m, l - 1, l - 1), m.ref, m.hc, c.tag);
-                    }
-                    else
-                    {
-                        k_maximum<3><<<blocks_words(c, l - 1, l - 1), c.block, 0, c.stream>>>(c.g, l, m.wl_ref, level_offsets(c, m, l - 1, l - 1), m.ref, m.hc, c.tag);
-                    }
-                    launched(c, "maximum");
-                    --l;
                 }
-                if (l >= lstop)
+                if (l >= std::max(1, minl))
                 {
-                    if (g.dim == 2)
-                    {
-                        k_maximum_small<2><<<1, 1024, 0, c.stream>>>(c.g, l, lstop, m.wl_ref, m.d_lo, m.ref, m.hc, c.tag);
-                    }
-                    else
-                    {
-                        k_maximum_small<3><<<1, 1024, 0, c.stream>>>(c.g, l, lstop, m.wl_ref, m.d_lo, m.ref, m.hc, c.tag);
-                    }
-                    launched(c, "maximum_small");
-                }
-                // the levels below hold no operator but still exchange their tags
-                for (int lt = lstop - 1; g.periodic && lt >= 1; --lt)
-                {
-                    periodic_tags(c, m, lt);
+                    s.add(OP_MAXIMUM, l, l);
                 }
             }
-            timer_stop(c, T_FINALIZE);
-            if ((st = check(c, "criteria")))
-            {
-                return st;
-            }
+            s.timer_stop(T_FINALIZE);
 
-            timer_start(c, T_MESH_UPDATE);
-            // the second pass runs on the device only if the first one refined
-            if ((st = new_cells_from_tags(c, m, nm.cells)) || (st = grad_pass(c, nm.cells, F_GRAD0, nullptr))
-                || (!graphed && (st = grad_pass(c, nm.cells, F_GRAD1, c.d_flags + F_GRAD0))))
+            s.timer_start(T_MESH_UPDATE);
+            // the second graduation pass runs on the device only if the first one refined
+            s.add(OP_NEW_CELLS, minl, maxl);
+            grad_pass_phases(s, F_GRAD0, -1);
+            if (!graphed)
             {
-                return st;
+                grad_pass_phases(s, F_GRAD1, F_GRAD0);
             }
-            if (graphed)
+            else
             {
                 // make_graduation to its fixed point on the device: further passes while the last one refined
                 // (at most 64, as on the host path)
+                s.flush();
                 k_adapt_words<<<1, 1, 0, c.stream>>>(c.d_adapt, A_LOOP, c.d_flags + F_GRAD0, 0, 0);
                 k_adapt_words<<<1, 1, 0, c.stream>>>(c.d_adapt, A_ITER, nullptr, 0, 0);
                 launched(c, "adapt_words", 2);
-                st = capture_conditional(
+                const int st = capture_conditional(
                     c, cudaGraphCondTypeWhile,
                     [&](cudaGraphConditionalHandle h)
                     {
@@ -2623,25 +1222,28 @@ namespace sg
                     [&](cudaGraphConditionalHandle h)
                     {
                         cudaMemsetAsync(c.d_flags + F_GRADX, 0, sizeof(int), c.stream);
-                        int s2 = grad_pass(c, nm.cells, F_GRADX, nullptr);
-                        if (!s2)
+                        Sequence s2(c, m, nm);
+                        grad_pass_phases(s2, F_GRADX, -1);
+                        const int st2 = s2.done("graduation");
+                        if (!st2)
                         {
                             k_adapt_words<<<1, 1, 0, c.stream>>>(c.d_adapt, A_LOOP, c.d_flags + F_GRADX, 0, 0);
                             k_loop_next<<<1, 1, 0, c.stream>>>(h, c.d_adapt + A_LOOP, c.d_adapt + A_ITER, 64, c.g.err);
                             launched(c, "loop_next", 2);
                         }
-                        return s2;
+                        return st2;
                     });
                 if (st)
                 {
                     return st;
                 }
             }
-            if ((st = bitmaps_differ(c, nm.cells, m.cells, F_DIFFER)))
+            s.add(OP_COMPARE);
+            s.timer_stop(T_MESH_UPDATE);
+            if (int st = s.done("harten front"))
             {
                 return st;
             }
-            timer_stop(c, T_MESH_UPDATE);
             if (!graphed)
             {
                 cudaMemcpyAsync(c.h_flags, c.d_flags, F_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c.stream);
@@ -2654,26 +1256,27 @@ namespace sg
         // ghosts are updated first, mr/adapt.hpp:383)
         int seq_back(Ctx& c, DeviceMesh& m, DeviceMesh& nm, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os)
         {
-            int st;
-            for (DeviceField* f : os)
+            Sequence s(c, m, nm);
+            if (!os.empty())
             {
-                if ((st = seq_ghost(c, m, f->data, f->has_bc, f->bc_value)))
-                {
-                    return st;
-                }
+                s.timer_start(T_GHOST);
+                field_groups(s, slots_of(os), [&]() { ghost_phases(s); });
+                s.timer_stop(T_GHOST);
             }
-            if ((st = build_mesh(c, nm)))
+            s.timer_start(T_CONSTRUCTION);
+            build_mesh_phases(s);
+            s.timer_stop(T_CONSTRUCTION);
+            s.timer_start(T_FIELDS_UPDATE);
+            std::vector<DeviceField*> all(fs);
+            all.insert(all.end(), os.begin(), os.end());
+            field_groups(s, slots_of(all), [&]() { s.add(OP_UPDATE_FIELDS); });
+            s.timer_stop(T_FIELDS_UPDATE);
+            if (int st = s.done("update_fields"))
             {
                 return st;
             }
-            ScopedTimer tf(c, T_FIELDS_UPDATE);
-            for (const auto* list : {&fs, &os})
-            {
-                for (DeviceField* f : *list)
-                {
-                    update_fields_launch(c, m, nm, ValAcc{f->data}, ValAcc{f->spare});
-                }
-            }
+            cudaMemcpyAsync(nm.h_lo, nm.d_lo, COUNTS * sizeof(long long), cudaMemcpyDeviceToHost, c.stream);
+            nm.host_valid = false;
             return check(c, "update_fields");
         }
 
@@ -2757,15 +1360,12 @@ namespace sg
             c.err = "harten: ghost widths 1 and 2 are implemented";
             return SG_ERR_ARG;
         }
-        const int minl = c.cfg.min_level;
-        const int maxl = c.cfg.max_level;
-        const int dim  = c.g.dim;
         DeviceMesh& m  = c.m();
         DeviceMesh& nm = c.spare();
         // the pinned inputs staged here were consumed by the previous pass,
         // which ended with harten_end's synchronisation
-        *c.h_ite = ite;
-        pass_thresholds(c, ite, eps, regularity, c.h_eps);
+        c.h_setup->ite = ite;
+        pass_thresholds(c, ite, eps, regularity, c.h_setup->eps);
         // the captured front differs with relative details and with the
         // number of fields: keys of their own
         c.rel_detail = relative_detail;
@@ -2804,12 +1404,14 @@ namespace sg
         {
             // graduation still refining after two passes: finish the fixed
             // point with host-tested passes, then compare again
-            if ((st = graduate(c, nm.cells, nullptr)))
+            if ((st = graduate(c, m, nm, nullptr)))
             {
                 return st;
             }
             cudaMemsetAsync(c.d_flags + F_DIFFER, 0, sizeof(int), c.stream);
-            if ((st = bitmaps_differ(c, nm.cells, m.cells, F_DIFFER)))
+            Sequence s(c, m, nm);
+            s.add(OP_COMPARE);
+            if ((st = s.done("harten compare")))
             {
                 return st;
             }
@@ -2875,30 +1477,34 @@ namespace sg
     // transposed (reverse: the RevAcc accessor, launches in reverse order).
     int ghost_value(Ctx& c, DeviceMesh& m, double* u, bool has_bc, double bcv)
     {
-        return ghost_launches(c, m, ValAcc{u}, has_bc, bcv, c.fuse_top_field, false, [] {});
+        Sequence s(c, m, m);
+        const FieldSlot f{u, nullptr, bcv, has_bc ? 1 : 0};
+        s.fields(&f, 0, 1);
+        ghost_phases(s);
+        return s.done("update_ghost_mr");
     }
 
     // lam := G^T lam for the ghost update G of mesh m, in place.  The launch sequence is the one that separates
-    // every read from every write (corner projections in launches of their own, no one-block chains), captured
-    // once per mesh buffer and adjoint array and replayed backwards.
+    // every read from every write (corner projections in launches of their own), captured once per mesh buffer
+    // and adjoint array and replayed backwards.
     int ghost_reverse(Ctx& c, DeviceMesh& m, double* lam, int* overflow, bool has_bc)
     {
         const unsigned long long kind = 40ull | (has_bc ? 256ull : 0ull);
         return run_reversed(c, kind, ptr_key(m.ref), ptr_key(lam), ptr_key(overflow),
                             [&]()
                             {
-                                if (c.g.dim == 2)
-                                {
-                                    return ghost_launches(c, m, RevAcc<FormCap<2>::value>{lam, lam, overflow, 1}, has_bc, 0., -2, true, [] {});
-                                }
-                                return ghost_launches(c, m, RevAcc<FormCap<3>::value>{lam, lam, overflow, 1}, has_bc, 0., -2, true, [] {});
+                                return c.g.dim == 2 ? ghost_reverse_launches<2>(c, m, lam, overflow, has_bc)
+                                                    : ghost_reverse_launches<3>(c, m, lam, overflow, has_bc);
                             });
     }
 
     int update_fields_value(Ctx& c, DeviceMesh& m, DeviceMesh& nm, const double* uo, double* un)
     {
-        update_fields_launch(c, m, nm, ValAcc{const_cast<double*>(uo)}, ValAcc{un});
-        return check(c, "update_fields");
+        Sequence s(c, m, nm);
+        const FieldSlot f{const_cast<double*>(uo), un, 0., 0};
+        s.fields(&f, 0, 1);
+        s.add(OP_UPDATE_FIELDS);
+        return s.done("update_fields");
     }
 
     // lam_old += T^T lam_new for update_fields T from mesh m to mesh nm (lam_old is not cleared here)
@@ -2907,13 +1513,16 @@ namespace sg
         if (c.g.dim == 2)
         {
             const RevAcc<FormCap<2>::value> r{lam_new, lam_old, overflow, 0};
-            update_fields_launch(c, m, nm, r, r);
+            k_update_fields_reverse<2><<<blocks_words(c, 0, c.g.nlev - 1), c.block, 0, c.stream>>>(c.g, c.cfg.prediction_radius, nm.wl_ref, nm.d_lo, nm.ref,
+                                                                                              nm.cells, m.ref, m.cells, m.hc, r, r);
         }
         else
         {
             const RevAcc<FormCap<3>::value> r{lam_new, lam_old, overflow, 0};
-            update_fields_launch(c, m, nm, r, r);
+            k_update_fields_reverse<3><<<blocks_words(c, 0, c.g.nlev - 1), c.block, 0, c.stream>>>(c.g, c.cfg.prediction_radius, nm.wl_ref, nm.d_lo, nm.ref,
+                                                                                              nm.cells, m.ref, m.cells, m.hc, r, r);
         }
+        launched(c, "update_fields");
         return check(c, "update_fields (transpose)");
     }
 
@@ -3021,8 +1630,8 @@ namespace sg
                                                   [&]()
                                                   {
                                                       int s1 = capture_if(c, c.d_adapt + A_NEEDG,
-                                                                          [&]() { return ghost_launches(c, mf, ValAcc{ud}, bc, bcv, c.fuse_top_field, false, [] {}); });
-                                                      return s1 ? s1 : upwind_on(c, mf, ud, tail->unp1->data, tail->a, tail->dt, tail->scheme, true);
+                                                                          [&]() { return ghost_value(c, mf, ud, bc, bcv); });
+                                                      return s1 ? s1 : upwind_on(c, mf, ud, tail->unp1->data, tail->a, tail->dt, tail->scheme);
                                                   });
                 }
             }
@@ -3273,25 +1882,14 @@ namespace sg
         return device_error(c);
     }
 
-    namespace
-    {
-        __global__ void k_set_velocity(double* av, double a0, double a1, double a2)
-        {
-            av[0] = a0;
-            av[1] = a1;
-            av[2] = a2;
-        }
-    } // namespace
-
-    // the upwind step on mesh m from the values at ud into unp1d; baked: the
-    // velocity of the flux form is written by a kernel (inside a captured
-    // graph) instead of copied from the host array
-    int upwind_on(Ctx& c, const DeviceMesh& m, const double* ud, double* unp1d, const double* a, double dt, int scheme, bool baked)
+    // the upwind step on mesh m from the values at ud into unp1d
+    int upwind_on(Ctx& c, const DeviceMesh& m, const double* ud, double* unp1d, const double* a, double dt, int scheme)
     {
         const Geom& g = c.g;
         UpwindArgs p{};
         for (int d = 0; d < g.dim; ++d)
         {
+            p.a[d]  = a[d];
             p.ha[d] = .5 * a[d];
             p.hb[d] = .5 * std::fabs(a[d]);
         }
@@ -3300,23 +1898,13 @@ namespace sg
         const int nb = blocks_words(c, 0, g.nlev - 1);
         if (scheme == 2)
         {
-            double* av = c.d_eps + EPS_VELOCITY;
-            if (baked)
-            {
-                k_set_velocity<<<1, 1, 0, c.stream>>>(av, a[0], a[1], g.dim == 3 ? a[2] : 0.);
-                launched(c, "set_velocity");
-            }
-            else
-            {
-                cudaMemcpyAsync(av, a, g.dim * sizeof(double), cudaMemcpyHostToDevice, c.stream);
-            }
             if (g.dim == 2)
             {
-                k_convection<2><<<nb, c.block, 0, c.stream>>>(c.g, m.wl_cells, m.d_lo, m.cells, ud, unp1d, p, av);
+                k_convection<2><<<nb, c.block, 0, c.stream>>>(c.g, m.wl_cells, m.d_lo, m.cells, ud, unp1d, p);
             }
             else
             {
-                k_convection<3><<<nb, c.block, 0, c.stream>>>(c.g, m.wl_cells, m.d_lo, m.cells, ud, unp1d, p, av);
+                k_convection<3><<<nb, c.block, 0, c.stream>>>(c.g, m.wl_cells, m.d_lo, m.cells, ud, unp1d, p);
             }
         }
         else if (g.dim == 2)
@@ -3334,6 +1922,6 @@ namespace sg
     int upwind(Ctx& c, DeviceField& u, DeviceField& unp1, const double* a, double dt, int scheme)
     {
         ScopedTimer timer(c, T_UPWIND);
-        return upwind_on(c, c.m(), u.data, unp1.data, a, dt, scheme, false);
+        return upwind_on(c, c.m(), u.data, unp1.data, a, dt, scheme);
     }
 } // namespace sg

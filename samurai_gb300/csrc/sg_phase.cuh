@@ -1,0 +1,134 @@
+// The step as a sequence of phases.
+//
+// A phase is one data-parallel operation on the mesh or its fields (a level of
+// the ghost update, the details, a level of the tag finalisation, a pass of the
+// mesh construction, ...) whose items are independent; each phase reads what
+// the ones before it wrote.  The device code of a phase is written against a
+// Team of threads and launched as a kernel of its own (sg_phase.cu).
+#pragma once
+
+#include <vector>
+
+#include "sg_access.cuh"
+#include "sg_ctx.cuh"
+
+namespace sg
+{
+    constexpr int PHASE_FIELDS = 8;    // fields one phase works on together
+    constexpr int SCAN_WORDS   = 2048; // words per chunk of the scan
+
+    enum Op : int
+    {
+        OP_PASS_BEGIN,      // threshold bitmaps and flags cleared
+        OP_GHOST,           // top-down pass of update_ghost_mr, level l0
+        OP_PREDICT,         // bottom-up pass, level l0
+        OP_ABSMAX_INIT,     // relative details: max |u| over the leaves
+        OP_ABSMAX,
+        OP_DETAIL,          // details and their threshold bits, levels l0..l1
+        OP_CRITERIA,        // tags from the threshold bits
+        OP_MAXIMUM,         // tag finalisation, children at level l0
+        OP_NEW_CELLS,       // leaf cells of mesh n from the tags
+        OP_GRAD_COARSEN,    // graduation of mesh n's cells (the first to the last of these may hang on a flag)
+        OP_GRAD_EXPAND,
+        OP_GRAD_EXPAND_XY,
+        OP_GRAD_EXPAND_Z,
+        OP_GRAD_PERIODIC,
+        OP_GRAD_DOWN,       // level l0
+        OP_GRAD_REFINE,     // levels l0..l1
+        OP_GRAD_APPLY,      // levels l0..l1
+        OP_COMPARE,         // do the leaf cells of m and n differ
+        OP_CLEAR_UNION,     // construction of mesh n from its cells
+        OP_HC_CAG,
+        OP_HC2_CAG,         // levels l0..l1
+        OP_CAG_ON,          // levels l0..l1
+        OP_REF0,
+        OP_REF0_XY,
+        OP_REF0_Z,
+        OP_REF_PERIODIC_SRC,
+        OP_REF_PERIODIC,
+        OP_REF_CHILDREN,    // levels l0..l1
+        OP_REF_CHILDREN_LEVEL, // level l0
+        OP_PROJ,            // levels l0..l1
+        OP_SINGLE_LEVEL,
+        OP_SCAN_SUMS,
+        OP_SCAN_WRITE,
+        OP_UPDATE_FIELDS,   // from mesh m to mesh n
+        OP_PERIODIC_COPY,   // level l0, axis aux
+        OP_PERIODIC_TAG,    // level l0, axis aux >> 1, side aux & 1
+        OP_COUNT
+    };
+
+    // aux of a graduation phase: the slot of the flag it raises, and the slot of the flag it hangs on
+    inline int grad_aux(int slot, int guard = -1)
+    {
+        return slot | ((guard + 1) << 3);
+    }
+
+    struct Phase
+    {
+        short op, l0, l1, aux;
+    };
+
+    // device pointers of one mesh
+    struct MeshPtrs
+    {
+        uint32_t *cells, *cag, *proj, *uni, *ref, *hc, *hc2, *pred;
+        int *rank, *wl_ref, *wl_cells;
+        long long* lo;
+    };
+
+    struct FieldSlot
+    {
+        double* u;      // values on mesh m
+        double* un;     // update_fields: values on mesh n
+        double bcv;     // Dirichlet value
+        int has_bc;
+    };
+
+    // what the phases of one sequence work on: mesh m (the current one), mesh n
+    // (the one being built), scratch, up to PHASE_FIELDS fields
+    struct Env
+    {
+        Geom g;
+        MeshPtrs m, n;
+        uint32_t *t0, *t1, *t2, *t3, *rf;
+        uint32_t *tk, *tc, *tr;    // tags: keep, coarsen, refine
+        uint32_t *above, *ref_above, *par_above; // |detail| over the coarsen, refine and parent thresholds
+        double* det;
+        long long capacity;
+        const PassSetup* setup;
+        unsigned long long* absmax;
+        int* flags;
+        long long* block_sums;
+        int order;          // prediction stencil radius
+        int radius;         // max_stencil_radius
+        int grad_width;
+        int refine_boundary;
+        int relative;
+        int nf;
+        FieldSlot f[PHASE_FIELDS];
+    };
+
+    // Launches phases in order.
+    struct Sequence
+    {
+        Ctx& c;
+        Env env;
+        int status = SG_OK;
+
+        Sequence(Ctx& ctx, const DeviceMesh& m, const DeviceMesh& n);
+        void fields(const FieldSlot* fs, int first, int nf); // the fields of the following phases: fs[first .. first + nf)
+        void add(int op, int l0 = 0, int l1 = 0, int aux = 0);
+        void flush(); // before anything else is queued on the stream
+        void timer_start(int id);
+        void timer_stop(int id);
+        int done(const char* what);
+    };
+
+    void build_mesh_phases(Sequence& s);                       // mesh construction of mesh n from its cells
+    void grad_pass_phases(Sequence& s, int slot, int guard);   // one graduation pass on mesh n's cells
+    MeshPtrs mesh_ptrs(const DeviceMesh& m);
+    int launch_phase_alone(Ctx& c, const Env& e, const Phase& p);
+    long long phase_words(const Geom& g, const Phase& p);
+    const char* phase_name(int op);
+} // namespace sg
