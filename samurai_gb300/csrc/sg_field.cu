@@ -109,33 +109,23 @@ namespace sg
             const Geom& g = gp;
             if (static_cast<int>(blockIdx.x) < nb)
             {
-                const long long nc    = l >= g.min_level ? corner_count<DIM>(g, l) : 0;
-                const long long total = (parts & 1) ? boundary_count<DIM>(g, l) : nc;
-                for (long long t = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += static_cast<long long>(nb) * blockDim.x)
+                const int total = static_cast<int>((parts & 1) ? boundary_count<DIM>(g, l) : corner_slots<DIM>(g, l));
+                for (int t = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); t < total; t += nb * static_cast<int>(blockDim.x))
                 {
-                    if (t < nc)
-                    {
-                        corner_item<DIM>(g, l, t, m.cells, m.ref, u, parts);
-                    }
-                    else
-                    {
-                        const FaceArgs a{l, l < g.max_level, l >= g.min_level && has_bc, l >= g.min_level && l < g.max_level};
-                        face_item<DIM>(g, a, t - nc, m.cells, m.uni, m.ref, u, 0.);
-                    }
+                    boundary_item<DIM>(g, l, t, m, u, has_bc != 0, 0., parts);
                 }
                 return;
             }
-            project_items<DIM>(g, l, m.wl_ref, m.lo, m.proj, static_cast<int>(((blockIdx.x - nb) * blockDim.x + threadIdx.x) >> 5),
-                               static_cast<int>(((gridDim.x - nb) * blockDim.x) >> 5),
-                               [&](long long w, int b, const Cell& c) { project_transpose<DIM>(g, u, 32 * w + b, l, c.x, c.y, c.z); });
+            project_items(g, l, m, grid_team(nb), 1,
+                          [&](long long w, int b, const Cell& c, int) { project_transpose<DIM>(g, u, 32 * w + b, l, c.x, c.y, c.z); });
         }
 
         template <int DIM, int CAP>
         __global__ void k_predict_reverse(const __grid_constant__ Geom gp, int l, int order, MeshPtrs m, RevAcc<CAP> u)
         {
             const Geom& g = gp;
-            predict_items<DIM>(g, l, m.wl_ref, m.lo, m.pred, static_cast<int>(warp_id()), static_cast<int>(warp_count()),
-                               [&](long long w, int b, const Cell& c) { predict_transpose<DIM>(g, u, 32 * w + b, l, c.x, c.y, c.z, order); });
+            predict_items(g, l, m, grid_team(), 1,
+                          [&](long long w, int b, const Cell& c, int) { predict_transpose<DIM>(g, u, 32 * w + b, l, c.x, c.y, c.z, order); });
         }
 
         // update_fields (algorithm/update_fields.hpp:27-127): copy on
@@ -146,9 +136,14 @@ namespace sg
                                         const uint32_t* ncells, const uint32_t* oref, const uint32_t* ocells, const uint32_t* ohc, A uo, A un)
         {
             const Geom& g = gp;
-            warp_list_compact(wl, lo[LO_REF], lo[LO_REF + g.nlev], warp_id(), warp_count(), [&](long long w) { return nref[w]; },
-                      [&](long long w, int b)
+            block_items(wl, static_cast<int>(lo[LO_REF]), static_cast<int>(lo[LO_REF + g.nlev]), grid_team(), 1, [&](int w) { return nref[w]; },
+                      [&](bool valid, int w_, int b, int)
                       {
+                          if (!valid)
+                          {
+                              return;
+                          }
+                          const long long w = w_;
                           const long long e = 32 * w + b;
                           typename A::V v   = A::konst(0.);
                           if ((ncells[w] >> b) & 1u)
@@ -225,21 +220,20 @@ namespace sg
         {
             const Geom& g  = gp;
             const int lane = threadIdx.x & 31;
-            // the leaf cells compacted over the lanes (warp_items); a cell's left
+            // consecutive threads hold consecutive leaf cells (block_items); a cell's left
             // flux is its left neighbour's right flux when that neighbour is the
             // previous lane's cell (the same face, the same expression)
-            const long long nb = lo[LO_CELLS], ne = lo[LO_CELLS + g.nlev];
-            warp_items(wl, nb, ne, warp_id(), warp_count(), items_chunk(ne - nb, warp_count()), [&](long long w) { return cells[w]; },
-                           [&](bool valid, long long w, int b)
+            block_items(wl, static_cast<int>(lo[LO_CELLS]), static_cast<int>(lo[LO_CELLS + g.nlev]), grid_team(), 1, [&](int w) { return __ldg(cells + w); },
+                           [&](bool valid, int w, int b, int)
                            {
                                int l = 0;
                                long long e = 0, sy = 0, sz = 0;
                                double uc = 0., rf = 0.;
                                if (valid)
                                {
-                                   l                  = level_of(g, w);
+                                   l                  = level_down(g, w, 0, g.max_level);
                                    const LevelGeom& L = g.lv[l];
-                                   e                  = 32 * w + b;
+                                   e                  = 32LL * w + b;
                                    sy                 = 32LL * L.W;
                                    sz                 = sy * L.R;
                                    uc                 = u[e];
@@ -266,7 +260,7 @@ namespace sg
                                    rf              = p.ha[0] * (uc + ur) + p.hb[0] * (uc - ur);
                                }
                                const double rf_left = __shfl_up_sync(FULL_MASK, rf, 1);
-                               const long long wl_  = __shfl_up_sync(FULL_MASK, w, 1);
+                               const int wl_        = __shfl_up_sync(FULL_MASK, w, 1);
                                const int bl         = __shfl_up_sync(FULL_MASK, valid ? b : -2, 1);
                                if (!valid)
                                {
@@ -329,11 +323,15 @@ namespace sg
                                      double* __restrict__ unp1, UpwindArgs p)
         {
             const Geom& g     = gp;
-            const long long n = lo[LO_CELLS + g.nlev];
-            warp_list_compact(wl, lo[LO_CELLS], n, warp_id(), warp_count(), [&](long long w) { return cells[w]; },
-                              [&](long long w, int b)
+            block_items(wl, static_cast<int>(lo[LO_CELLS]), static_cast<int>(lo[LO_CELLS + g.nlev]), grid_team(), 1, [&](int w) { return __ldg(cells + w); },
+                              [&](bool valid, int w_, int b, int)
                               {
-                                  const int m        = level_of(g, w);
+                                  if (!valid)
+                                  {
+                                      return;
+                                  }
+                                  const long long w  = w_;
+                                  const int m        = level_down(g, w_, 0, g.max_level);
                                   const Cell cc      = cell_of(g, m, w, b);
                                   const int c[3]     = {cc.x, cc.y, cc.z};
                                   const long long eX = 32 * w + b;
@@ -1149,6 +1147,7 @@ namespace sg
             }
             const std::vector<FieldSlot> slots = slots_of(fs);
             Sequence s(c, m, nm);
+            s.fields(slots.data(), 0, std::min(PHASE_FIELDS, static_cast<int>(slots.size())));
             s.add(OP_PASS_BEGIN);
             s.timer_start(T_GHOST);
             field_groups(s, slots, [&]() { ghost_phases(s); });
@@ -1263,13 +1262,15 @@ namespace sg
                 field_groups(s, slots_of(os), [&]() { ghost_phases(s); });
                 s.timer_stop(T_GHOST);
             }
+            std::vector<DeviceField*> all(fs);
+            all.insert(all.end(), os.begin(), os.end());
+            const std::vector<FieldSlot> slots = slots_of(all);
+            s.fields(slots.data(), 0, std::min(PHASE_FIELDS, static_cast<int>(slots.size())));
             s.timer_start(T_CONSTRUCTION);
             build_mesh_phases(s);
             s.timer_stop(T_CONSTRUCTION);
             s.timer_start(T_FIELDS_UPDATE);
-            std::vector<DeviceField*> all(fs);
-            all.insert(all.end(), os.begin(), os.end());
-            field_groups(s, slots_of(all), [&]() { s.add(OP_UPDATE_FIELDS); });
+            field_groups(s, slots, [&]() { s.add(OP_UPDATE_FIELDS); });
             s.timer_stop(T_FIELDS_UPDATE);
             if (int st = s.done("update_fields"))
             {

@@ -53,41 +53,31 @@ namespace sg
         // finalised earlier, so they run side by side: corners and faces from
         // item b of nb threads, the projection onto level l-1 from warp0 of nwarps.
         template <int DIM>
-        __device__ __forceinline__ void ghost_boundary(const Env& E, int l, long long b, long long nb)
+        __device__ __forceinline__ void ghost_boundary(const Env& E, int l, int b, int nb)
         {
-            const Geom& g         = E.g;
-            const long long nc    = l >= g.min_level ? corner_count<DIM>(g, l) : 0;
-            const long long total = boundary_count<DIM>(g, l);
-            for (long long t = b; t < total; t += nb)
+            const int per   = static_cast<int>(boundary_count<DIM>(E.g, l));
+            const int total = per * E.nf;
+            for (int t = b; t < total; t += nb)
             {
-                for (int f = 0; f < E.nf; ++f)
+                int f = 0, k = t;
+                while (k >= per)
                 {
-                    const FieldSlot& F = E.f[f];
-                    const ValAcc u{F.u};
-                    if (t < nc)
-                    {
-                        corner_item<DIM>(g, l, t, E.m.cells, E.m.ref, u, 3);
-                    }
-                    else
-                    {
-                        const FaceArgs a{l, l < g.max_level, l >= g.min_level && F.has_bc, l >= g.min_level && l < g.max_level};
-                        face_item<DIM>(g, a, t - nc, E.m.cells, E.m.uni, E.m.ref, u, F.bcv);
-                    }
+                    k -= per;
+                    ++f;
                 }
+                boundary_item<DIM>(E.g, l, k, E.m, ValAcc{E.f[f].u}, E.f[f].has_bc != 0, E.f[f].bcv, 3);
             }
         }
 
         template <int DIM>
-        __device__ __forceinline__ void ghost_project(const Env& E, int l, int warp0, int nwarps)
+        __device__ __forceinline__ void ghost_project(const Env& E, int l, const Team& T)
         {
-            project_items<DIM>(E.g, l, E.m.wl_ref, E.m.lo, E.m.proj, warp0, nwarps,
-                               [&](long long w, int b, const Cell& c)
-                               {
-                                   for (int f = 0; f < E.nf; ++f)
-                                   {
-                                       E.f[f].u[32 * w + b] = project_one<DIM>(E.g, ValAcc{E.f[f].u}, l, c.x, c.y, c.z);
-                                   }
-                               });
+            project_items(E.g, l, E.m, T, E.nf,
+                          [&](long long w, int b, const Cell& c, int f)
+                          {
+                              double* u     = E.f[f].u;
+                              u[32 * w + b] = project_one<DIM>(E.g, ValAcc{u}, l, c.x, c.y, c.z);
+                          });
         }
 
         __device__ __forceinline__ int lowest_level(const Geom& g)
@@ -95,30 +85,27 @@ namespace sg
             return g.min_level >= 2 ? g.min_level - 2 : 0; // no reference cell below min_level - 2
         }
 
-        // in a chain: the boundary items from the last thread down, so that the
-        // first warps start on the projection at once
+        // in a chain: the boundary items go to the last blocks first, the projection to the first
         template <int DIM>
         __device__ __forceinline__ void op_ghost(const Env& E, int l, const Team& T)
         {
-            ghost_boundary<DIM>(E, l, T.nthr - 1 - T.tid, T.nthr);
+            const int back = T.nblocks - 1 - T.block; // whole warps stay together
+            ghost_boundary<DIM>(E, l, back * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x), T.nthr);
             if (l > lowest_level(E.g))
             {
-                __syncwarp();
-                ghost_project<DIM>(E, l, T.warp0(), T.nwarps());
+                ghost_project<DIM>(E, l, T);
             }
         }
 
         template <int DIM>
         __device__ __forceinline__ void op_predict(const Env& E, int l, const Team& T)
         {
-            predict_items<DIM>(E.g, l, E.m.wl_ref, E.m.lo, E.m.pred, T.warp0(), T.nwarps(),
-                               [&](long long w, int b, const Cell& c)
-                               {
-                                   for (int f = 0; f < E.nf; ++f)
-                                   {
-                                       E.f[f].u[32 * w + b] = predict_one<DIM>(E.g, ValAcc{E.f[f].u}, l, c.x, c.y, c.z, E.order);
-                                   }
-                               });
+            predict_items(E.g, l, E.m, T, E.nf,
+                          [&](long long w, int b, const Cell& c, int f)
+                          {
+                              double* u     = E.f[f].u;
+                              u[32 * w + b] = predict_one<DIM>(E.g, ValAcc{u}, l, c.x, c.y, c.z, E.order);
+                          });
         }
 
         // ---------------------------------------------------------- details
@@ -182,18 +169,23 @@ namespace sg
             const uint32_t* ref = E.m.ref;
             const uint32_t* hc  = E.m.hc;
             const uint32_t* hc2 = E.m.hc2;
-            warp_list_compact(
-                E.m.wl_ref, E.m.lo[LO_REF + l0], E.m.lo[LO_REF + le + 1], T.warp0(), T.nwarps(), [&](long long w) { return ref[w] & (hc[w] | hc2[w]); },
-                [&](long long w, int b)
+            block_items(
+                E.m.wl_ref, static_cast<int>(E.m.lo[LO_REF + l0]), static_cast<int>(E.m.lo[LO_REF + le + 1]), T, E.nf,
+                [&](int w) { return ref[w] & (hc[w] | hc2[w]); },
+                [&](bool valid, int w_, int b, int f)
                 {
-                    const int l   = level_down(g, static_cast<int>(w), l0, le);
+                    if (!valid)
+                    {
+                        return;
+                    }
+                    const long long w = w_;
+                    const int l   = level_down(g, w_, l0, le);
                     const Cell c  = cell_of(g, l, w, b);
                     const Box3 cb = box_at<DIM>(g, l + 1, 2 * c.x, 2 * c.y, 2 * c.z, 2);
                     const Box3 sb = E.order ? box_at<DIM>(g, l, c.x - 1, c.y - 1, c.z - 1, 3) : Box3{0, 0, 0};
                     const double t_above = eps[l + 1], t_ref = eps[MAXLEV + l + 1];
                     const double t_par   = l + 1 < g.max_level ? eps[2 * MAXLEV + l + 2] : 0.;
                     uint32_t fa = 0u, fr = 0u, fp = 0u; // one bit per child
-                    for (int f = 0; f < E.nf; ++f)
                     {
                         const double* u = E.f[f].u;
                         double* det     = E.det + f * E.capacity;
@@ -1192,40 +1184,36 @@ namespace sg
         __device__ __forceinline__ void op_update_fields(const Env& E, const Team& T)
         {
             const Geom& g = E.g;
-            warp_list_compact(E.n.wl_ref, E.n.lo[LO_REF], E.n.lo[LO_REF + g.nlev], T.warp0(), T.nwarps(), [&](long long w) { return E.n.ref[w]; },
-                              [&](long long w, int b)
-                              {
-                                  const long long e    = 32 * w + b;
-                                  const uint32_t cells = E.n.cells[w], hc = E.m.hc[w], ref = E.m.ref[w];
-                                  int how = 0; // 1 projection, 2 prediction, 3 copy, 0 zero
-                                  int l   = 0;
-                                  Cell c{0, 0, 0};
-                                  if ((cells >> b) & 1u)
-                                  {
-                                      l = level_down(g, static_cast<int>(w), 0, g.max_level);
-                                      c = cell_of(g, l, w, b);
-                                      how = ((hc >> b) & 1u) ? 1
-                                                             : (l >= 1 && test(E.m.cells, g, l - 1, c.x >> 1, c.y >> 1, c.z >> 1) ? 2 : (((ref >> b) & 1u) ? 3 : 0));
-                                  }
-                                  for (int f = 0; f < E.nf; ++f)
-                                  {
-                                      const ValAcc uo{E.f[f].u};
-                                      double v = 0.;
-                                      if (how == 1)
-                                      {
-                                          v = project_one<DIM>(g, uo, l + 1, c.x, c.y, c.z);
-                                      }
-                                      else if (how == 2)
-                                      {
-                                          v = predict_one<DIM>(g, uo, l, c.x, c.y, c.z, E.order);
-                                      }
-                                      else if (how == 3)
-                                      {
-                                          v = uo.get(e);
-                                      }
-                                      E.f[f].un[e] = v;
-                                  }
-                              });
+            block_items(E.n.wl_ref, static_cast<int>(E.n.lo[LO_REF]), static_cast<int>(E.n.lo[LO_REF + g.nlev]), T, E.nf, [&](int w) { return E.n.ref[w]; },
+                        [&](bool valid, int w, int b, int f)
+                        {
+                            if (!valid)
+                            {
+                                return;
+                            }
+                            const long long e    = 32LL * w + b;
+                            const uint32_t cells = E.n.cells[w], hc = E.m.hc[w], ref = E.m.ref[w];
+                            const ValAcc uo{E.f[f].u};
+                            double v = 0.;
+                            if ((cells >> b) & 1u)
+                            {
+                                const int l  = level_down(g, w, 0, g.max_level);
+                                const Cell c = cell_of(g, l, w, b);
+                                if ((hc >> b) & 1u)
+                                {
+                                    v = project_one<DIM>(g, uo, l + 1, c.x, c.y, c.z);
+                                }
+                                else if (l >= 1 && test(E.m.cells, g, l - 1, c.x >> 1, c.y >> 1, c.z >> 1))
+                                {
+                                    v = predict_one<DIM>(g, uo, l, c.x, c.y, c.z, E.order);
+                                }
+                                else if ((ref >> b) & 1u)
+                                {
+                                    v = uo.get(e);
+                                }
+                            }
+                            E.f[f].un[e] = v;
+                        });
         }
 
         // ---------------------------------------------------------- periodic axes
@@ -1371,12 +1359,11 @@ namespace sg
                 const int nb = p.l1;
                 if (static_cast<int>(blockIdx.x) < nb)
                 {
-                    ghost_boundary<DIM>(E, p.l0, static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x, static_cast<long long>(nb) * blockDim.x);
+                    ghost_boundary<DIM>(E, p.l0, static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x), nb * static_cast<int>(blockDim.x));
                 }
                 else
                 {
-                    ghost_project<DIM>(E, p.l0, static_cast<int>(((blockIdx.x - nb) * blockDim.x + threadIdx.x) >> 5),
-                                       static_cast<int>(((gridDim.x - nb) * blockDim.x) >> 5));
+                    ghost_project<DIM>(E, p.l0, grid_team(nb));
                 }
             }
             else
@@ -1470,12 +1457,12 @@ namespace sg
         Phase p       = ph;
         int block     = 256;
         long long grid = 1;
-        auto warps     = [&](long long words) // one warp per word, at most max_blocks blocks of 8 warps' worth of warps
+        // blocks that hand out the items of `words` words: a block per 16 words, at most max_blocks blocks of 256 threads
+        auto items = [&](long long words)
         {
-            block                = c.block;
-            const long long wpb  = block / 32;
-            const long long cap  = std::max(1LL, c.max_blocks * 8 / wpb);
-            return std::min(cap, std::max(1LL, (words + wpb - 1) / wpb));
+            block               = c.block;
+            const long long cap = std::max(1LL, c.max_blocks * 256 / block);
+            return std::min(cap, std::max(1LL, (words + 15) / 16));
         };
         switch (shape_of(p.op))
         {
@@ -1500,20 +1487,20 @@ namespace sg
             case Shape::ITEMS:
                 if (p.op == OP_GHOST)
                 {
-                    const long long nproj = p.l0 > (g.min_level >= 2 ? g.min_level - 2 : 0) ? warps(g.lv[p.l0 - 1].nwords) : 0;
+                    const long long nproj = p.l0 > (g.min_level >= 2 ? g.min_level - 2 : 0) ? items(g.lv[p.l0 - 1].nwords) : 0;
                     block                 = c.block;
-                    const long long items = g.dim == 2 ? boundary_count<2>(g, p.l0) : boundary_count<3>(g, p.l0);
-                    const long long nb    = std::min(16384LL, (items + block - 1) / block);
+                    const long long edge  = (g.dim == 2 ? boundary_count<2>(g, p.l0) : boundary_count<3>(g, p.l0)) * e.nf;
+                    const long long nb    = std::min(16384LL, (edge + block - 1) / block);
                     p.l1                  = static_cast<short>(nb);
                     grid                  = nb + nproj;
                 }
                 else if (p.op == OP_PREDICT)
                 {
-                    grid = warps(g.lv[p.l0].nwords);
+                    grid = items(g.lv[p.l0].nwords);
                 }
                 else
                 {
-                    grid = warps(p.l0 <= p.l1 && p.l1 > 0 ? range_words(g, p.l0, p.l1) : g.total_words);
+                    grid = items(p.l0 <= p.l1 && p.l1 > 0 ? range_words(g, p.l0, p.l1) : g.total_words);
                 }
                 break;
             case Shape::SCAN: grid = (g.total_words + SCAN_WORDS - 1) / SCAN_WORDS; break;
@@ -1571,6 +1558,10 @@ namespace sg
 
     void Sequence::fields(const FieldSlot* fs, int first, int nf)
     {
+        if (env.nf == nf && std::memcmp(env.f, fs + first, static_cast<size_t>(nf) * sizeof(FieldSlot)) == 0)
+        {
+            return; // the fields the sequence already works on
+        }
         flush();
         env.nf = nf;
         for (int k = 0; k < nf; ++k)
@@ -1593,15 +1584,22 @@ namespace sg
     {
     }
 
+    // the named timers bracket launches: a chain ends where one starts or stops
     void Sequence::timer_start(int id)
     {
-        flush();
+        if (c.timers.enabled)
+        {
+            flush();
+        }
         sg::timer_start(c, id);
     }
 
     void Sequence::timer_stop(int id)
     {
-        flush();
+        if (c.timers.enabled)
+        {
+            flush();
+        }
         sg::timer_stop(c, id);
     }
 

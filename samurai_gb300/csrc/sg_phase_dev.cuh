@@ -2,6 +2,8 @@
 // share with the transposed launches.
 #pragma once
 
+#include <type_traits>
+
 #include "sg_phase.cuh"
 
 namespace sg
@@ -31,116 +33,7 @@ namespace sg
         }
     }
 
-    // Compacted traversal for the FP64-heavy kernels.  On the traversal
-    // above a warp works on one word and the lanes of its empty bits idle
-    // while the others issue FP64 instructions, which the narrow FP64 pipe
-    // executes for the whole warp (42 % of the lanes of the leaf-cell
-    // words of the 2D max_level-12 workload hold a cell).  Here a warp
-    // takes ch consecutive words of the list, ranks their set bits with a
-    // warp prefix sum and processes them 32 at a time, one per lane.
-    // item(valid, w, b) is called by every lane of the warp (so that it
-    // may shuffle); only lanes with valid set hold an item, bit b of word w.
     constexpr unsigned FULL_MASK = 0xffffffffu;
-
-    // words per warp: the largest power of two (<= 32) that still leaves
-    // every warp of the launch a chunk; 1 on lists shorter than two words
-    // per warp, where the launch is latency-bound and the compaction does
-    // not pay
-    __device__ __forceinline__ int items_chunk(long long n, long long nwarps)
-    {
-        const long long per = n / (nwarps > 0 ? nwarps : 1);
-        int ch              = 1;
-        while (ch < 32 && 2 * ch <= per)
-        {
-            ch <<= 1;
-        }
-        return ch;
-    }
-
-    template <class WordF, class ItemF>
-    __device__ __forceinline__ void warp_items(const int* list, long long begin, long long end, long long warp0, long long nwarps, int ch,
-                                               WordF word_of, ItemF item)
-    {
-        const int lane = threadIdx.x & 31;
-        for (long long c0 = begin + warp0 * ch; c0 < end; c0 += nwarps * ch)
-        {
-            long long w = 0;
-            uint32_t m  = 0u;
-            if (lane < ch && c0 + lane < end)
-            {
-                w = list ? list[c0 + lane] : c0 + lane;
-                m = word_of(w);
-            }
-            int incl = __popc(m); // inclusive prefix of the item counts over the lanes
-            for (int o = 1; o < 32; o <<= 1)
-            {
-                const int t = __shfl_up_sync(FULL_MASK, incl, o);
-                if (lane >= o)
-                {
-                    incl += t;
-                }
-            }
-            const int total = __shfl_sync(FULL_MASK, incl, 31);
-            for (int base = 0; base < total; base += 32)
-            {
-                const int j = base + lane;
-                // the word of item j: the first lane whose inclusive prefix exceeds j
-                int lo_k = 0, hi_k = 31;
-                for (int s = 0; s < 5; ++s)
-                {
-                    const int mid = (lo_k + hi_k) >> 1;
-                    if (__shfl_sync(FULL_MASK, incl, mid) > j)
-                    {
-                        hi_k = mid;
-                    }
-                    else
-                    {
-                        lo_k = mid + 1;
-                    }
-                }
-                const long long wk = __shfl_sync(FULL_MASK, w, lo_k);
-                const uint32_t mk  = __shfl_sync(FULL_MASK, m, lo_k);
-                const int before   = __shfl_sync(FULL_MASK, incl, lo_k) - __popc(mk);
-                const bool valid   = j < total;
-                // position of set bit number r (from 0) of mk
-                int r = valid ? j - before : 0, pos = 0;
-                uint32_t x = mk;
-                for (int sh = 16; sh > 0; sh >>= 1)
-                {
-                    const int cnt = __popc(x & ((1u << sh) - 1u));
-                    if (r >= cnt)
-                    {
-                        r -= cnt;
-                        x >>= sh;
-                        pos += sh;
-                    }
-                }
-                item(valid, wk, pos);
-            }
-        }
-    }
-
-    // warp_list with the compacted traversal where the list is long enough:
-    // cell(w, b) for every set bit
-    template <class WordF, class CellF>
-    __device__ __forceinline__ void warp_list_compact(const int* list, long long begin, long long end, long long warp0, long long nwarps,
-                                                      WordF word_of, CellF cell)
-    {
-        const int ch = items_chunk(end - begin, nwarps);
-        if (ch == 1)
-        {
-            warp_list(list, begin, end, warp0, nwarps, word_of, cell);
-            return;
-        }
-        warp_items(list, begin, end, warp0, nwarps, ch, word_of,
-                   [&](bool valid, long long w, int b)
-                   {
-                       if (valid)
-                       {
-                           cell(w, b);
-                       }
-                   });
-    }
 
     __device__ __forceinline__ long long warp_id()
     {
@@ -315,44 +208,13 @@ namespace sg
         u.put(e2, (u.get(em) - u.get(e0) * 3.0) + u.get(e1) * 3.0);
     }
 
-    // face position helper: direction index k in 0..2*dim-1 is
-    // (+e0,-e0,+e1,-e1,...) (stencil.hpp:301-317)
-    __device__ __forceinline__ void face_cell(const Geom& g, int l, int k, long long t, int* in, int* dir)
-    {
-        const int axis = k >> 1;
-        const int sgn  = (k & 1) ? -1 : 1;
-        const int n    = g.lv[l].n;
-        const int f0 = static_cast<int>(t % n), f1 = static_cast<int>(t / n);
-        // the free coordinates fill the non-normal axes in order
-        dir[0] = dir[1] = dir[2] = 0;
-        in[2]                    = 0;
-        if (axis == 0)
-        {
-            in[0] = sgn > 0 ? n - 1 : 0;
-            in[1] = f0;
-            in[2] = (g.dim == 3) ? f1 : 0;
-        }
-        else if (axis == 1)
-        {
-            in[0] = f0;
-            in[1] = sgn > 0 ? n - 1 : 0;
-            in[2] = (g.dim == 3) ? f1 : 0;
-        }
-        else
-        {
-            in[0] = f0;
-            in[1] = f1;
-            in[2] = sgn > 0 ? n - 1 : 0;
-        }
-        dir[axis] = sgn;
-    }
-
     // ------------------------------------------------------------ threads
     // the threads a phase runs on: the whole grid of its own launch, or the
     // cluster of a chain
     struct Team
     {
-        int tid, nthr;
+        int tid, nthr;      // thread
+        int block, nblocks; // block
 
         __device__ __forceinline__ int warp0() const
         {
@@ -365,9 +227,134 @@ namespace sg
         }
     };
 
-    __device__ __forceinline__ Team grid_team()
+    // the blocks from `first` on
+    __device__ __forceinline__ Team grid_team(int first = 0)
     {
-        return {static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x), static_cast<int>(gridDim.x * blockDim.x)};
+        const int b = static_cast<int>(blockIdx.x) - first, n = static_cast<int>(gridDim.x) - first;
+        return {b * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x), n * static_cast<int>(blockDim.x), b, n};
+    }
+
+    // ------------------------------------------------------------ items
+    // The cells of a set, spread evenly over the threads of each block: a block
+    // takes a chunk of words (at most one per thread, loaded together), ranks
+    // their set bits with a block prefix sum and hands the items out in order, one
+    // per thread and round; with several fields the rounds run over (field, item)
+    // pairs.  The bands of cells the path works on fill a few words of a row and
+    // leave the next ones empty; a warp per word (or per few words) waits for its
+    // fullest word.  item(valid, w, b, field) is called by every thread of a
+    // block (it may shuffle), consecutive threads on consecutive items.
+    constexpr int ITEM_THREADS = 1024; // largest block
+
+    struct ItemShared
+    {
+        int pre[ITEM_THREADS];
+        int w[ITEM_THREADS];
+        uint32_t m[ITEM_THREADS];
+        int part[32];
+    };
+
+    __device__ __forceinline__ ItemShared& item_shared()
+    {
+        __shared__ ItemShared s;
+        return s;
+    }
+
+    // position of set bit number r (from 0) of m
+    __device__ __forceinline__ int nth_bit(uint32_t m, int r)
+    {
+        int pos = 0;
+#pragma unroll
+        for (int sh = 16; sh > 0; sh >>= 1)
+        {
+            const int cnt = __popc(m & ((1u << sh) - 1u));
+            if (r >= cnt)
+            {
+                r -= cnt;
+                m >>= sh;
+                pos += sh;
+            }
+        }
+        return pos;
+    }
+
+    // list: word indices, entries [begin, end); null: the words [begin, end) themselves
+    template <class WordF, class ItemF>
+    __device__ __forceinline__ void block_items(const int* list, int begin, int end, const Team& T, int nf, WordF word_of, ItemF item)
+    {
+        ItemShared& S  = item_shared();
+        const int B    = static_cast<int>(blockDim.x), t = static_cast<int>(threadIdx.x);
+        const int lane = t & 31, warp = t >> 5, nwarp = B >> 5;
+        const int n    = end - begin;
+        // words per block and round: an even share, between 16 and one per thread
+        const int chunk = min(B, max(16, (n + T.nblocks - 1) / T.nblocks));
+        for (int c0 = T.block * chunk; c0 < n; c0 += T.nblocks * chunk)
+        {
+            int w      = 0;
+            uint32_t m = 0u;
+            if (t < chunk && c0 + t < n)
+            {
+                w = list ? list[begin + c0 + t] : begin + c0 + t;
+                m = word_of(w);
+            }
+            int incl = __popc(m);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const int x = __shfl_up_sync(FULL_MASK, incl, o);
+                incl += lane >= o ? x : 0;
+            }
+            __syncthreads(); // the previous round's readers are done
+            if (lane == 31)
+            {
+                S.part[warp] = incl;
+            }
+            __syncthreads();
+            int before = 0, total = 0;
+            if (lane < nwarp)
+            {
+                total = S.part[lane];
+            }
+            before = lane < warp ? total : 0;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                before += __shfl_xor_sync(FULL_MASK, before, o);
+                total += __shfl_xor_sync(FULL_MASK, total, o);
+            }
+            if (total == 0)
+            {
+                continue; // the same on every thread
+            }
+            S.pre[t] = before + incl - __popc(m);
+            S.w[t]   = w;
+            S.m[t]   = m;
+            __syncthreads();
+            const int all = total * nf;
+            for (int base = 0; base < all; base += B)
+            {
+                int j = base + t, f = 0;
+                const bool valid = j < all;
+                if (!valid)
+                {
+                    j = 0;
+                }
+                while (j >= total)
+                {
+                    j -= total;
+                    ++f;
+                }
+                // the word of item j: the last one whose prefix does not exceed j
+                int lo = 0;
+                for (int step = 1 << (31 - __clz(B - 1)); step > 0; step >>= 1)
+                {
+                    if (lo + step < B && S.pre[lo + step] <= j)
+                    {
+                        lo += step;
+                    }
+                }
+                item(valid, S.w[lo], nth_bit(S.m[lo], j - S.pre[lo]), f);
+            }
+        }
     }
 
     // ------------------------------------------------------------ words
@@ -541,35 +528,41 @@ namespace sg
     }
 
     // ------------------------------------------------------- ghost update
-    // The 2^DIM (m = 2) or 4^DIM (m = 4) cells under cell (x, y, z) of level l
-    // at level l + log2 m: the rows' reference words are loaded together, then
-    // the values, then f is called in the reference's order (z, y, x ascending)
-    // on the members of ref.  Returns their number.
-    template <int DIM, int M, class F>
-    __device__ __forceinline__ int for_children(const Geom& g, int lc, int x, int y, int z, const uint32_t* ref, F f)
+    // The 2^DIM (M = 2) or 4^DIM (M = 4) cells under cell (x, y, z) of level l
+    // at level l + log2 M: the members of ref, row by row (M consecutive cells,
+    // aligned to M: one word)
+    template <int DIM, int M>
+    struct Children
     {
-        constexpr int ROWS = DIM == 3 ? M * M : M;
+        static constexpr int ROWS = DIM == 3 ? M * M : M;
         uint32_t bits[ROWS];
         long long el[ROWS];
-#pragma unroll
-        for (int s = 0; s < ROWS; ++s)
+
+        __device__ __forceinline__ void load(const Geom& g, int lc, int x, int y, int z, const uint32_t* ref)
         {
-            const Pos p = pos_of(g, lc, M * x, M * y + s % M, DIM == 3 ? M * z + s / M : 0);
-            bits[s]     = 0u;
-            el[s]       = 0;
-            if (p.w >= 0) // M consecutive cells, aligned to M: one word
+#pragma unroll
+            for (int s = 0; s < ROWS; ++s)
             {
-                bits[s] = (ref[p.w] >> p.b) & ((1u << M) - 1u);
-                el[s]   = elem(p);
+                const Pos p = pos_of(g, lc, M * x, M * y + s % M, DIM == 3 ? M * z + s / M : 0);
+                bits[s]     = p.w >= 0 ? (ref[p.w] >> p.b) & ((1u << M) - 1u) : 0u;
+                el[s]       = elem(p);
             }
         }
-        int n = 0;
-#pragma unroll
-        for (int s = 0; s < ROWS; ++s)
+
+        __device__ __forceinline__ int count() const
         {
-            n += __popc(bits[s]);
+            int n = 0;
+#pragma unroll
+            for (int s = 0; s < ROWS; ++s)
+            {
+                n += __popc(bits[s]);
+            }
+            return n;
         }
-        if (n)
+
+        // f on the members in the reference's order (z, y, x ascending)
+        template <class F>
+        __device__ __forceinline__ void each(F f) const
         {
 #pragma unroll
             for (int s = 0; s < ROWS; ++s)
@@ -577,11 +570,56 @@ namespace sg
 #pragma unroll
                 for (int k = 0; k < M; ++k)
                 {
-                    f((bits[s] >> k) & 1u, el[s] + k);
+                    if ((bits[s] >> k) & 1u)
+                    {
+                        f(el[s] + k);
+                    }
                 }
             }
         }
-        return n;
+    };
+
+    // the sum of the members' values, in order from 0: loaded together, then added one by one
+    template <int DIM, int M, class A>
+    __device__ __forceinline__ typename A::V sum_children(const Children<DIM, M>& ch, const A& u)
+    {
+        typename A::V sum = A::konst(0.);
+        if constexpr (std::is_same<A, ValAcc>::value && (DIM == 2 || M == 2))
+        {
+            double v[Children<DIM, M>::ROWS * M];
+#pragma unroll
+            for (int s = 0; s < Children<DIM, M>::ROWS * M; ++s)
+            {
+                v[s] = ((ch.bits[s / M] >> (s % M)) & 1u) ? u.get(ch.el[s / M] + s % M) : 0.;
+            }
+#pragma unroll
+            for (int s = 0; s < Children<DIM, M>::ROWS * M; ++s)
+            {
+                if ((ch.bits[s / M] >> (s % M)) & 1u)
+                {
+                    sum = sum + v[s];
+                }
+            }
+        }
+        else
+        {
+            ch.each([&](long long e) { sum = sum + u.get(e); });
+        }
+        return sum;
+    }
+
+    // v / n for a member count n: a power of two only moves the exponent
+    template <class A>
+    __device__ __forceinline__ typename A::V mean_of(const typename A::V& v, int n)
+    {
+        if constexpr (std::is_same<A, ValAcc>::value)
+        {
+            if ((n & (n - 1)) == 0)
+            {
+                return n == 1 ? v : scale_down(v, 31 - __clz(n));
+            }
+        }
+        return v / static_cast<double>(n);
     }
 
     struct FaceArgs
@@ -600,28 +638,37 @@ namespace sg
     __device__ __forceinline__ void face_item(const Geom& g, const FaceArgs& a, long long t, const uint32_t* cells, const uint32_t* uni,
                                               const uint32_t* ref, const A& u, double value)
     {
-        const int l        = a.l;
-        const int n        = g.lv[l].n;
-        const long long nf = (DIM == 2) ? n : static_cast<long long>(n) * n;
-        const int k        = static_cast<int>(t / nf);
-        int in[3], dir[3];
-        face_cell(g, l, k, t - k * nf, in, dir);
-        if (crosses_periodic(g, dir))
+        const int l = a.l;
+        // n = 2^l: the direction and the position on the face are bit fields of t
+        const int n = g.lv[l].n, k = static_cast<int>(t >> (l * (DIM - 1)));
+        const int axis = k >> 1, sgn = (k & 1) ? -1 : 1; // (+e0, -e0, +e1, -e1, ...) (stencil.hpp:301-317)
+        const int f0 = static_cast<int>(t) & (n - 1), f1 = DIM == 3 ? static_cast<int>(t >> l) & (n - 1) : 0;
+        if ((g.periodic >> axis) & 1)
         {
             return; // a periodic axis has no boundary
         }
-        const Pos pi = pos_of(g, l, in[0], in[1], in[2]);
+        const int at = sgn > 0 ? n - 1 : 0;
+        // the free coordinates fill the other axes in order
+        const int in[3]  = {axis == 0 ? at : f0, axis == 1 ? at : (axis == 0 ? f0 : f1), DIM == 3 ? (axis == 2 ? at : f1) : 0};
+        const int dir[3] = {axis == 0 ? sgn : 0, axis == 1 ? sgn : 0, axis == 2 ? sgn : 0};
         const int gx = in[0] + dir[0], gy = in[1] + dir[1], gz = in[2] + dir[2];
-        const Pos pg        = pos_of(g, l, gx, gy, gz);
-        const uint32_t wc   = cells[pi.w], wu = uni[pi.w];
-        const bool in_ref   = pg.w >= 0 && ((ref[pg.w] >> pg.b) & 1u);
-        const long long eg  = elem(pg);
+        // everything the roles ask first is loaded together
+        const Pos pi = pos_of(g, l, in[0], in[1], in[2]);
+        const Pos pg = pos_of(g, l, gx, gy, gz);
+        const uint32_t wc  = cells[pi.w], wu = uni[pi.w], wg = ref[pg.w];
+        const long long eg = elem(pg);
+        const typename A::V ui = u.get(elem(pi));
+        Children<DIM, 2> c2;
+        if (l + 1 < g.nlev)
+        {
+            c2.load(g, l + 1, gx, gy, gz, ref);
+        }
         if ((a.do_dirichlet || a.do_predict) && ((wc >> pi.b) & 1u))
         {
             typename A::V v;
             if (a.do_dirichlet)
             {
-                v = A::konst(2 * value) - u.get(elem(pi));
+                v = A::konst(2 * value) - ui;
                 u.put(eg, v);
                 // update_further_ghosts_by_polynomial_extrapolation (bc/apply_field_bc.hpp:531-593), ghost
                 // width 2: the second layer beyond a boundary leaf, where it is a reference cell
@@ -636,36 +683,32 @@ namespace sg
             }
             if (a.do_predict)
             {
-                for_children<DIM, 2>(g, l + 1, gx, gy, gz, ref,
-                                     [&](bool member, long long e)
-                                     {
-                                         if (member)
-                                         {
-                                             u.put(e, v);
-                                         }
-                                     });
+                c2.each([&](long long e) { u.put(e, v); });
             }
         }
         else if (a.do_project && ((wu >> pi.b) & 1u))
         {
-            if (!in_ref)
+            if (!((wg >> pg.b) & 1u))
             {
                 return;
             }
-            typename A::V sum = A::konst(0.);
-            auto add          = [&](bool member, long long e)
+            typename A::V v = A::konst(0.);
+            int nch         = c2.count();
+            if (nch)
             {
-                if (member)
-                {
-                    sum = sum + u.get(e);
-                }
-            };
-            int nch = l + 1 < g.nlev ? for_children<DIM, 2>(g, l + 1, gx, gy, gz, ref, add) : 0;
-            if (nch == 0 && l + 2 < g.nlev)
-            {
-                nch = for_children<DIM, 4>(g, l + 2, gx, gy, gz, ref, add);
+                v = mean_of<A>(sum_children<DIM, 2>(c2, u), nch);
             }
-            u.put(eg, nch > 0 ? sum / static_cast<double>(nch) : A::konst(0.));
+            else if (l + 2 < g.nlev)
+            {
+                Children<DIM, 4> c4;
+                c4.load(g, l + 2, gx, gy, gz, ref);
+                nch = c4.count();
+                if (nch)
+                {
+                    v = mean_of<A>(sum_children<DIM, 4>(c4, u), nch);
+                }
+            }
+            u.put(eg, v);
             // the second ghost layer beyond a boundary cell that is not a leaf but has finer leaves
             // (apply_extrapolation_bc_ghosts, bc/apply_field_bc.hpp:196-214), ghost width 2
             if (g.ghost_width >= 2 && a.do_dirichlet && test(ref, g, l, gx + dir[0], gy + dir[1], gz + dir[2]))
@@ -704,8 +747,8 @@ namespace sg
         }
         else
         {
-            const int e = static_cast<int>((t - 8) / n);
-            pos         = static_cast<int>((t - 8) - static_cast<long long>(e) * n);
+            const int e = static_cast<int>((t - 8) >> l); // n = 2^l positions per edge
+            pos         = static_cast<int>(t - 8) & (n - 1);
             free_axis   = e >> 2;
             d[free_axis == 0 ? 1 : 0] = (e & 1) ? 1 : -1;
             d[free_axis == 2 ? 1 : 2] = (e & 2) ? 1 : -1;
@@ -719,13 +762,33 @@ namespace sg
         {
             c[k] = d[k] > 0 ? n - 1 : (d[k] < 0 ? 0 : pos);
         }
-        if (parts & 1)
+        // the fine position of a projection below is the ghost eg of this thread; all it reads is loaded together
+        const Pos pc = pos_of(g, l, c[0], c[1], c[2]);
+        const Pos pe = pos_of(g, l, c[0] + d[0], c[1] + d[1], DIM == 3 ? c[2] + d[2] : 0);
+        const long long eg = elem(pe);
+        Pos below[2];
+        bool project[2];
+        const bool in_ref = test(ref, pe);
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
         {
-            const Pos pc = pos_of(g, l, c[0], c[1], c[2]);
-            if (test(cells, pc))
+            const int dl = k + 1, pl = l - dl;
+            below[k]   = Pos{-1, 0};
+            project[k] = (parts & 2) && pl >= 0 && (free_axis < 0 || (pos & ((1 << dl) - 1)) == 0);
+            if (project[k])
             {
-                const long long eg = elem_at(g, l, c[0] + d[0], c[1] + d[1], DIM == 3 ? c[2] + d[2] : 0);
-                u.put(eg, u.get(elem(pc)));
+                const int np = g.lv[pl].n;
+                below[k]     = pos_of(g, pl, d[0] > 0 ? np : (d[0] < 0 ? -1 : pos >> dl), d[1] > 0 ? np : (d[1] < 0 ? -1 : pos >> dl),
+                                  DIM == 3 ? (d[2] > 0 ? np : (d[2] < 0 ? -1 : pos >> dl)) : 0);
+                project[k]   = test(ref, below[k]);
+            }
+        }
+        const bool leaf       = (parts & 1) && test(cells, pc);
+        const typename A::V v = leaf ? u.get(elem(pc)) : u.get(eg);
+        if (leaf)
+        {
+            {
+                u.put(eg, v);
                 if (g.ghost_width >= 2)
                 {
                     if (test(ref, g, l, c[0] + 2 * d[0], c[1] + 2 * d[1], DIM == 3 ? c[2] + 2 * d[2] : 0))
@@ -768,71 +831,84 @@ namespace sg
                 }
             }
         }
-        if (!(parts & 2))
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
         {
-            return;
-        }
-        for (int dl = 1; dl <= 2 && dl <= l; ++dl)
-        {
-            const int pl = l - dl;
-            if (free_axis >= 0 && (pos & ((1 << dl) - 1)) != 0)
+            if (project[k] && in_ref)
             {
-                continue;
-            }
-            int gc[3] = {0, 0, 0}, ch[3] = {0, 0, 0};
-            for (int k = 0; k < DIM; ++k)
-            {
-                gc[k] = d[k] > 0 ? g.lv[pl].n : (d[k] < 0 ? -1 : pos >> dl);
-                ch[k] = (gc[k] << dl) + (d[k] == -1 ? ((1 << dl) - 1) : 0);
-            }
-            const Pos pg = pos_of(g, pl, gc[0], gc[1], gc[2]);
-            const Pos pf = pos_of(g, l, ch[0], ch[1], ch[2]);
-            if (test(ref, pg) && test(ref, pf))
-            {
-                u.put(elem(pg), u.get(elem(pf)));
+                u.put(elem(below[k]), v);
             }
         }
     }
 
-    // the words of level l a phase's warps walk: the listed ones, or every word
-    // of a level that gives each warp at most one (two dependent loads fewer)
-    __device__ __forceinline__ bool dense_level(const LevelGeom& L, int nwarps)
+    // The items of the set bm on level l.  Every word of the level is looked at
+    // when the team has a thread for it (one load to the bits); larger levels go
+    // through the list of reference words.
+    template <class ItemF>
+    __device__ __forceinline__ void level_items(const Geom& g, int l, const MeshPtrs& m, const uint32_t* bm, const Team& T, int nf, ItemF item)
     {
-        return L.nwords <= nwarps;
+        const LevelGeom& L = g.lv[l];
+        const int first    = static_cast<int>(L.woff);
+        const bool dense   = L.nwords <= T.nthr;
+        block_items(dense ? nullptr : m.wl_ref, dense ? first : static_cast<int>(m.lo[LO_REF + l]),
+                    dense ? first + static_cast<int>(L.nwords) : static_cast<int>(m.lo[LO_REF + l + 1]), T, nf, [&](int w) { return bm[w]; },
+                    [&](bool valid, int w, int b, int f)
+                    {
+                        if (valid)
+                        {
+                            item(static_cast<long long>(w), b, cell_of(g, l, w, b), f);
+                        }
+                    });
     }
 
     // projection of the reference cells of level l onto proj_cells[l-1]
     // (numeric/projection.hpp:15-65); the children of a projection cell are
-    // reference cells by construction.  item(word, bit, cell)
-    template <int DIM, class ItemF>
-    __device__ __forceinline__ void project_items(const Geom& g, int l, const int* wl_ref, const long long* lo, const uint32_t* proj, int warp0, int nwarps,
-                                                  ItemF item)
+    // reference cells by construction.  item(word, bit, cell, field)
+    template <class ItemF>
+    __device__ __forceinline__ void project_items(const Geom& g, int l, const MeshPtrs& m, const Team& T, int nf, ItemF item)
     {
-        const int lc       = l - 1;
-        const LevelGeom& C = g.lv[lc];
-        const bool dense   = dense_level(C, nwarps);
-        warp_list_compact(dense ? nullptr : wl_ref, dense ? C.woff : lo[LO_REF + lc], dense ? C.woff + C.nwords : lo[LO_REF + lc + 1], warp0, nwarps,
-                          [&](long long w) { return proj[w]; }, [&](long long w, int b) { item(w, b, cell_of(g, lc, w, b)); });
+        level_items(g, l - 1, m, m.proj, T, nf, item);
     }
 
     // prediction of the ghosts of level l from level l-1
     // (algorithm/update_ghost_mr.hpp:224-233)
-    template <int DIM, class ItemF>
-    __device__ __forceinline__ void predict_items(const Geom& g, int l, const int* wl_ref, const long long* lo, const uint32_t* pred, int warp0, int nwarps,
-                                                  ItemF item)
+    template <class ItemF>
+    __device__ __forceinline__ void predict_items(const Geom& g, int l, const MeshPtrs& m, const Team& T, int nf, ItemF item)
     {
-        const LevelGeom& L = g.lv[l];
-        const bool dense   = dense_level(L, nwarps);
-        warp_list_compact(dense ? nullptr : wl_ref, dense ? L.woff : lo[LO_REF + l], dense ? L.woff + L.nwords : lo[LO_REF + l + 1], warp0, nwarps,
-                          [&](long long w) { return pred[w]; }, [&](long long w, int b) { item(w, b, cell_of(g, l, w, b)); });
+        level_items(g, l, m, m.pred, T, nf, item);
     }
 
-    // corner and face positions of level l
+    // Boundary positions of level l: corners first, padded to whole warps (corner
+    // and face items take different branches), then the faces.
+    template <int DIM>
+    __host__ __device__ __forceinline__ long long corner_slots(const Geom& g, int l)
+    {
+        return l >= g.min_level ? (corner_count<DIM>(g, l) + 31) / 32 * 32 : 0;
+    }
+
     template <int DIM>
     __host__ __device__ __forceinline__ long long boundary_count(const Geom& g, int l)
     {
-        const int n           = g.lv[l].n;
-        const long long faces = (l < g.max_level || l >= g.min_level) ? 2LL * DIM * (DIM == 2 ? n : static_cast<long long>(n) * n) : 0;
-        return faces + (l >= g.min_level ? corner_count<DIM>(g, l) : 0);
+        const int n = g.lv[l].n;
+        return corner_slots<DIM>(g, l) + 2LL * DIM * (DIM == 2 ? n : static_cast<long long>(n) * n);
+    }
+
+    // boundary position t of level l on accessor u
+    template <int DIM, class A>
+    __device__ __forceinline__ void boundary_item(const Geom& g, int l, long long t, const MeshPtrs& m, const A& u, bool has_bc, double value, int corner_parts)
+    {
+        const long long nc = corner_slots<DIM>(g, l);
+        if (t < nc)
+        {
+            if (t < corner_count<DIM>(g, l))
+            {
+                corner_item<DIM>(g, l, t, m.cells, m.ref, u, corner_parts);
+            }
+        }
+        else
+        {
+            const FaceArgs a{l, l < g.max_level, l >= g.min_level && has_bc, l >= g.min_level && l < g.max_level};
+            face_item<DIM>(g, a, t - nc, m.cells, m.uni, m.ref, u, value);
+        }
     }
 } // namespace sg
