@@ -31,7 +31,6 @@ namespace sg
     int step_finish(Ctx& c, DeviceField& u, DeviceField& unp1, int* n_harten);
     int ensure_spare(Ctx& c, DeviceField& f);
     void set_fusion(Ctx& c, long long mesh_words, long long field_words, long long max_words);
-    void set_fusion_tops(Ctx& c, int mesh_top, int field_top, int max_top);
     void clear_graphs(Ctx& c);
 }
 
@@ -40,9 +39,9 @@ struct sg_batch_s
     std::vector<sg_field_t> u, unp1;
     std::vector<size_t> order; // instances by decreasing size: the largest are launched first
     int n_threads = 1;
-    std::vector<int> saved_tops;   // the instances' own one-block chain limits, restored on destroy
+    std::vector<long long> saved_fuse; // the instances' own chain limits and cluster sizes, restored on destroy
     std::vector<int> saved_blocks; // the instances' own threads per block, restored on destroy
-    long long fuse_words = sg::BATCH_FUSE_WORDS; // one-block chain limit of every instance (words per level)
+    long long fuse_words = sg::BATCH_FUSE_WORDS; // chain limit of every instance (words per level)
     int block            = 0;                    // threads per block of every instance's FP64 list kernels (0: their own)
 
     // worker pool: thread t runs job(t) for every new generation
@@ -388,8 +387,9 @@ extern "C"
         for (int k = 0; k < n; ++k)
         {
             sg::Ctx& c = u[k]->mesh->ctx;
-            b->saved_tops.insert(b->saved_tops.end(), {c.fuse_top, c.fuse_top_field, c.fuse_top_max});
+            b->saved_fuse.insert(b->saved_fuse.end(), {c.fuse_words_mesh, c.fuse_words_field, c.fuse_words_max, c.chain_blocks});
             b->saved_blocks.push_back(c.block);
+            c.chain_blocks = std::min(c.chain_blocks, sg::BATCH_CHAIN_BLOCKS);
             sg::set_fusion(c, sg::BATCH_FUSE_WORDS, sg::BATCH_FUSE_WORDS, sg::BATCH_FUSE_WORDS);
         }
         b->n_threads = std::min(n_threads, n);
@@ -414,7 +414,8 @@ extern "C"
             {
                 sg::Ctx& c = b->u[k]->mesh->ctx;
                 c.block    = b->saved_blocks[k];
-                sg::set_fusion_tops(c, b->saved_tops[3 * k], b->saved_tops[3 * k + 1], b->saved_tops[3 * k + 2]);
+                c.chain_blocks = static_cast<int>(b->saved_fuse[4 * k + 3]);
+                sg::set_fusion(c, b->saved_fuse[4 * k], b->saved_fuse[4 * k + 1], b->saved_fuse[4 * k + 2]);
             }
         }
         delete b;
@@ -544,7 +545,7 @@ extern "C"
     SG_API_CATCH(sg_batch_synchronize)
 
     // The batch's launch-shape autotuner: times `steps` batched steps from the instances' current state under
-    // candidate shapes (coordinate descent over the one-block chain limit shared by the instances, then the
+    // candidate shapes (coordinate descent over the chain limit shared by the instances, then the
     // threads per block of their FP64 list kernels), every candidate from the same saved state after one
     // untimed run that captures its graphs, every step after an L2 flush; keeps the fastest and leaves every
     // instance as it found it.

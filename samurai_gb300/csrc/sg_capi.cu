@@ -9,7 +9,7 @@
 #include <vector>
 
 #include "../../include/samurai_gpu.h"
-#include "sg_ctx.cuh"
+#include "sg_phase.cuh"
 
 #include "sg_handles.cuh"
 
@@ -298,23 +298,15 @@ namespace sg
         fail(0, msg, detail);
     }
 
-    // one-block chain limits of a mesh; the captured launch sequences are
-    // dropped, since they were recorded with the previous limits
-    void set_fusion_tops(Ctx& c, int mesh_top, int field_top, int max_top)
-    {
-        cudaStreamSynchronize(c.stream);
-        c.fuse_top       = mesh_top;
-        c.fuse_top_field = field_top;
-        c.fuse_top_max   = max_top;
-        sg::clear_graphs(c);
-    }
-
+    // chain limits of a mesh; the captured launch sequences are dropped, since
+    // they were recorded with the previous limits
     void set_fusion(Ctx& c, long long mesh_words, long long field_words, long long max_words)
     {
+        cudaStreamSynchronize(c.stream);
         c.fuse_words_mesh  = mesh_words;
         c.fuse_words_field = field_words;
         c.fuse_words_max   = max_words;
-        set_fusion_tops(c, fuse_top_of(c.g, mesh_words), fuse_top_of(c.g, field_words), fuse_top_of(c.g, max_words));
+        sg::clear_graphs(c);
     }
 
     // the spare buffer adaptation swaps into, allocated on first use
@@ -464,9 +456,7 @@ extern "C"
             return fail(SG_ERR_CUDA, "sg_mesh_create: no CUDA device");
         }
         sg::apply_tuned_launch(c); // the autotuner's choice for this device and level range, unless overridden above
-        c.fuse_top                 = sg::fuse_top_of(c.g, c.fuse_words_mesh);
-        c.fuse_top_field           = sg::fuse_top_of(c.g, c.fuse_words_field);
-        c.fuse_top_max             = sg::fuse_top_of(c.g, c.fuse_words_max);
+        c.chain_blocks             = static_cast<int>(std::min<long long>(sg::chain_blocks(dim), tuned("SG_CHAIN_BLOCKS", 16)));
         if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess)
         {
             cudaGetLastError();

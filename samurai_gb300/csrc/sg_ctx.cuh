@@ -185,14 +185,12 @@ namespace sg
         long long capacity  = 0;       // dense elements per field (32 * total_words)
         bool use_graphs     = true;    // replay captured launch sequences
         unsigned long long mesh_version = 1; // bumped at every change of the current mesh
-        int fuse_top        = -1;      // levels 0..fuse_top are small enough for one-block mesh chains
-        int fuse_top_field  = -1;      // the same for the FP64 field chains
-        int fuse_top_max    = -1;      // the same for the tag-finalisation chain
         long long max_blocks = 152LL * 8; // grid limit of the one-warp-per-word launches, in blocks of 8 warps (x4 for one thread per word)
         int block            = 256;       // threads per block of the FP64 list kernels
-        long long fuse_words_mesh  = 0; // one-block chain limits (words per level) behind fuse_top, fuse_top_field, fuse_top_max
-        long long fuse_words_field = 0;
-        long long fuse_words_max   = 0;
+        int chain_blocks           = 0; // blocks of the cluster that runs a chain of phases (0: no chains)
+        long long fuse_words_mesh  = 0; // largest phases that join a chain, in words they walk: mesh and tag phases over all levels,
+        long long fuse_words_field = 0; // a level of the ghost update,
+        long long fuse_words_max   = 0; // a level of the tag finalisation
         struct GraphEntry
         {
             unsigned long long key[4];
@@ -291,38 +289,12 @@ namespace sg
         }
     };
 
-    // A level-serial chain (union, reference children, graduation, tag
-    // finalisation, ghost passes) runs its levels of at most FUSE_WORDS words
-    // in a single block that steps through them with __syncthreads(), instead
-    // of one launch per level.
-    // The integer word chains of the mesh construction stay in one block up
-    // to 1K words per level (on the 2D max_level-12 step: 1.14 ms/step at 1K,
-    // 1.16 at 4K, 1.25 at 16K, 1.20 without fusion).  The FP64 field chains
-    // and the tag finalisation are not fused: their cells wait on memory, and
-    // one block serialises that latency (measured slower than one launch per
-    // level even at 1K-2K words), so their limit is 0.
-    constexpr long long FUSE_WORDS       = 1024;
-    constexpr long long FUSE_WORDS_FIELD = 0;
-    constexpr long long FUSE_WORDS_MAX   = 0;
-    // In batched mode many meshes share the GPU and the launch rate, not one
-    // mesh's latency, sets the pace: every chain runs its levels of at most
-    // 10K words in one block (measured on 256 meshes of max_level 7..11:
-    // 23.7 ms per batched step against 28.9 ms with the single-mesh limits
-    // and 25.0 ms with every level in one block).
+    // Limits of the phases that join a chain (sg_phase.cuh), in words
+    constexpr long long FUSE_WORDS       = 16384;
+    constexpr long long FUSE_WORDS_FIELD = 5000;
+    constexpr long long FUSE_WORDS_MAX   = 12288;
     constexpr long long BATCH_FUSE_WORDS = 10000;
-
-    inline int fuse_top_of(const Geom& g, long long limit)
-    {
-        int t = -1;
-        for (int l = 0; l < g.nlev; ++l)
-        {
-            if (g.lv[l].nwords <= limit)
-            {
-                t = l;
-            }
-        }
-        return t;
-    }
+    constexpr int BATCH_CHAIN_BLOCKS     = 8; // smaller clusters in batched mode, where many meshes share the chip
 
     // blocks of 256 threads (8 warps) for a warp-per-item loop over at most
     // max_items list entries: one wave of resident warps at most

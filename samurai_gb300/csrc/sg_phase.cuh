@@ -3,8 +3,13 @@
 // A phase is one data-parallel operation on the mesh or its fields (a level of
 // the ghost update, the details, a level of the tag finalisation, a pass of the
 // mesh construction, ...) whose items are independent; each phase reads what
-// the ones before it wrote.  The device code of a phase is written against a
-// Team of threads and launched as a kernel of its own (sg_phase.cu).
+// the ones before it wrote.  The device code of a phase is written once,
+// against a Team of threads, and runs in one of two ways (sg_phase.cu):
+//  - as a kernel of its own over the whole chip (large levels), or
+//  - as one link of a chain: consecutive small phases in a single launch of one
+//    thread-block cluster that separates them by hardware cluster barriers.
+// Data written by one phase and read by the next may cross SMs inside a chain:
+// phases load with plain (coherent) loads, never through the read-only path.
 #pragma once
 
 #include <vector>
@@ -109,12 +114,23 @@ namespace sg
         FieldSlot f[PHASE_FIELDS];
     };
 
-    // Launches phases in order.
+    constexpr int CHAIN_MAX     = 96;  // phases of one chain
+    constexpr int CHAIN_THREADS = 512; // threads per block of a chain
+
+    struct PhaseList
+    {
+        int n;
+        Phase p[CHAIN_MAX];
+    };
+
+    // Launches phases in order: small consecutive ones as one chain, the others
+    // one by one.
     struct Sequence
     {
         Ctx& c;
         Env env;
         int status = SG_OK;
+        std::vector<Phase> chain; // pending
 
         Sequence(Ctx& ctx, const DeviceMesh& m, const DeviceMesh& n);
         void fields(const FieldSlot* fs, int first, int nf); // the fields of the following phases: fs[first .. first + nf)
@@ -129,6 +145,7 @@ namespace sg
     void grad_pass_phases(Sequence& s, int slot, int guard);   // one graduation pass on mesh n's cells
     MeshPtrs mesh_ptrs(const DeviceMesh& m);
     int launch_phase_alone(Ctx& c, const Env& e, const Phase& p);
+    int chain_blocks(int dim);
     long long phase_words(const Geom& g, const Phase& p);
     const char* phase_name(int op);
 } // namespace sg

@@ -289,25 +289,24 @@ extern "C"
         // coordinate descent over the launch parameters, each from the best shape so far
         const std::vector<long long> blocks = {128, 256, 512};
         const std::vector<long long> grids  = {152LL * 4, 152LL * 8, 152LL * 16};
-        const std::vector<long long> fuses  = {0, 32, 128, 512};
+        const std::vector<long long> fuses  = {0, 2500, 5000, 12288};
         const std::vector<long long> flags  = {0, 1};
-        for (int param = 0; param < 6 && !st; ++param)
+        for (int param = 1; param < 6 && !st; ++param)
         {
-            const std::vector<long long>& cands = param <= 1 ? flags : (param == 2 ? blocks : (param == 3 ? grids : fuses));
+            const std::vector<long long>& cands = param == 1 ? flags : (param == 2 ? blocks : (param == 3 ? grids : fuses));
             const sg::LaunchShape from          = best;
             for (long long v : cands)
             {
                 sg::LaunchShape s = from;
                 switch (param)
                 {
-                case 0: s.graphed = static_cast<int>(v); break;
-                case 1: s.level_pairs = static_cast<int>(v); break;
+                case 1: s.graphed = static_cast<int>(v); break;
                 case 2: s.block = static_cast<int>(v); break;
                 case 3: s.max_blocks = v; break;
                 case 4: s.fuse_field = v; break;
                 default: s.fuse_max = v; break;
                 }
-                if (s.graphed == from.graphed && s.level_pairs == from.level_pairs && s.block == from.block
+                if (s.graphed == from.graphed && s.block == from.block
                     && s.max_blocks == from.max_blocks && s.fuse_field == from.fuse_field && s.fuse_max == from.fuse_max)
                 {
                     continue;
