@@ -161,6 +161,7 @@ namespace
     void adapt_share(sg_batch_s& b, int t, const double* eps, const double* regularity, int* n_harten)
     {
         std::vector<size_t> live;
+        std::vector<char> kept(b.u.size(), 0); // the instance's last pass kept its mesh
         int max_passes = 0;
         b.for_mine(t,
                    [&](size_t k)
@@ -210,6 +211,7 @@ namespace
                 {
                     n_harten[k] = ite + 1;
                 }
+                kept[k] = conv ? 1 : 0;
                 if (!conv)
                 {
                     live.push_back(k);
@@ -222,7 +224,7 @@ namespace
                        sg::Ctx& c = b.u[k]->mesh->ctx;
                        if (b.status == SG_OK)
                        {
-                           const int st = sg::device_error(c);
+                           const int st = sg::pass_error(c, kept[k] != 0);
                            if (st)
                            {
                                b.record(st, c.err.c_str());

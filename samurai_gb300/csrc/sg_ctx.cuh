@@ -39,7 +39,7 @@ namespace sg
         // mirrored asynchronously into pinned host memory; kernels read the
         // device copy, so no launch waits for the host.
         long long* d_lo = nullptr;
-        long long* h_lo = nullptr;
+        long long* h_lo = nullptr; // the first four, pinned: written by the scan
         bool host_valid = false; // h_lo reflects d_lo (after a synchronisation)
         long long nb_ref   = 0;  // host copies, valid when host_valid
         long long nb_cells = 0;
@@ -74,6 +74,7 @@ namespace sg
         F_GRAD1 = 1,  // graduation pass 2 found cells to refine (more passes needed)
         F_DIFFER = 2, // new leaf cells differ from the current ones
         F_GRADX = 3,  // scratch for extra graduation passes
+        F_ERR   = 4,  // the mesh's error word, in the host's copy
         F_COUNT = 8
     };
 
@@ -144,6 +145,7 @@ namespace sg
         PassSetup* h_setup = nullptr; // pinned staging
         unsigned long long* d_absmax = nullptr; // bits of max |u| over the leaf cells, per adapted field (relative details)
         int detail_comps             = 1;       // dense detail slabs allocated (one per adapted field)
+        bool back_ahead = false;                // the pass in flight has its second half queued already
         bool rel_detail = false;                // the Harten pass in flight divides the details by max |u|
         bool refine_boundary = false;           // args::refine_boundary: keep the boundary cells of max_level
         cudaStream_t stream = nullptr;
@@ -231,6 +233,7 @@ namespace sg
     // kernels and drivers (sg_mesh.cu / sg_field.cu)
     int build_mesh(Ctx& c, DeviceMesh& m);           // from m.cells; asynchronous
     int host_counts(Ctx& c, DeviceMesh& m);          // synchronises and refreshes nb_ref / nb_cells
+    int counts_arrived(Ctx& c, DeviceMesh& m);       // the same when the stream has been waited for since the scan
     int update_ghost_mr(Ctx& c, DeviceField& f);     // update_ghost_mr(u)
     int adapt(Ctx& c, DeviceField& f, double eps, double regularity, int* n_harten, bool relative_detail = false);
     int upwind(Ctx& c, DeviceField& u, DeviceField& unp1, const double* a, double dt, int scheme);
@@ -251,8 +254,10 @@ namespace sg
     int update_fields_value(Ctx& c, DeviceMesh& m, DeviceMesh& nm, const double* uo, double* un);
     int update_fields_reverse(Ctx& c, DeviceMesh& m, DeviceMesh& nm, double* lam_new, double* lam_old, int* overflow); // lam_old += T^T lam_new
     int harten_end(Ctx& c, DeviceField& f, bool* converged);
+    int pass_error(Ctx& c, bool converged); // the mesh's error word after an adaptation's last pass
     // the same for the fields fs driving the criteria and the fields os carried along
-    int harten_begin_fields(Ctx& c, const std::vector<DeviceField*>& fs, int ite, double eps, double regularity, bool relative_detail);
+    int harten_begin_fields(Ctx& c, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os, int ite, double eps, double regularity,
+                            bool relative_detail);
     int harten_end_fields(Ctx& c, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os, bool* converged);
     int adapt_fields(Ctx& c, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os, double eps, double regularity,
                      bool relative_detail, int* n_harten);

@@ -1141,12 +1141,9 @@ namespace sg
                 k_pass_setup<<<1, 128, 0, c.stream>>>(*graphed, c.d_setup);
                 launched(c, "pass_setup");
             }
-            else
-            {
-                cudaMemcpyAsync(c.d_setup, c.h_setup, sizeof(PassSetup), cudaMemcpyHostToDevice, c.stream);
-            }
             const std::vector<FieldSlot> slots = slots_of(fs);
             Sequence s(c, m, nm);
+            s.env.setup_host = graphed ? nullptr : c.h_setup;
             s.fields(slots.data(), 0, std::min(PHASE_FIELDS, static_cast<int>(slots.size())));
             s.add(OP_PASS_BEGIN);
             s.timer_start(T_GHOST);
@@ -1238,24 +1235,24 @@ namespace sg
                 }
             }
             s.add(OP_COMPARE);
-            s.timer_stop(T_MESH_UPDATE);
-            if (int st = s.done("harten front"))
-            {
-                return st;
-            }
             if (!graphed)
             {
-                cudaMemcpyAsync(c.h_flags, c.d_flags, F_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c.stream);
+                s.add(OP_REPORT);
             }
-            return check(c, "harten front");
+            s.timer_stop(T_MESH_UPDATE);
+            return s.done("harten front");
         }
 
         // new mesh from the new cells and update_fields (mr/adapt.hpp:380-386)
         // for the adapted fields fs and the fields os carried along (their
         // ghosts are updated first, mr/adapt.hpp:383)
-        int seq_back(Ctx& c, DeviceMesh& m, DeviceMesh& nm, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os)
+        // ahead: launched before the host knows whether the pass changed the mesh;
+        // the phases hang on the pass's flag
+        int seq_back(Ctx& c, DeviceMesh& m, DeviceMesh& nm, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os,
+                     bool ahead = false)
         {
             Sequence s(c, m, nm);
+            s.guard(ahead ? c.d_flags + F_DIFFER : nullptr);
             if (!os.empty())
             {
                 s.timer_start(T_GHOST);
@@ -1272,13 +1269,7 @@ namespace sg
             s.timer_start(T_FIELDS_UPDATE);
             field_groups(s, slots, [&]() { s.add(OP_UPDATE_FIELDS); });
             s.timer_stop(T_FIELDS_UPDATE);
-            if (int st = s.done("update_fields"))
-            {
-                return st;
-            }
-            cudaMemcpyAsync(nm.h_lo, nm.d_lo, COUNTS * sizeof(long long), cudaMemcpyDeviceToHost, c.stream);
-            nm.host_valid = false;
-            return check(c, "update_fields");
+            return s.done("update_fields");
         }
 
         // graph-cache key of a list of fields: their buffers and boundary values
@@ -1329,7 +1320,7 @@ namespace sg
     // host may launch other meshes' work (batched mode).
     int harten_begin(Ctx& c, DeviceField& f, int ite, double eps, double regularity, bool relative_detail)
     {
-        return harten_begin_fields(c, {&f}, ite, eps, regularity, relative_detail);
+        return harten_begin_fields(c, {&f}, {}, ite, eps, regularity, relative_detail);
     }
 
     namespace
@@ -1354,7 +1345,29 @@ namespace sg
         }
     } // namespace
 
-    int harten_begin_fields(Ctx& c, const std::vector<DeviceField*>& fs, int ite, double eps, double regularity, bool relative_detail)
+    namespace
+    {
+        // the second half of a pass, from its graph
+        int launch_back(Ctx& c, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os, bool ahead)
+        {
+            DeviceMesh& m  = c.m();
+            DeviceMesh& nm = c.spare();
+            const unsigned long long kind = ahead ? 1ull << 40 : 0ull;
+            if (fs.size() == 1 && os.empty())
+            {
+                DeviceField& f = *fs[0];
+                return run_cached(c, 3 | kind, static_cast<unsigned long long>(c.cur), ptr_key(f.data), ptr_key(f.spare),
+                                  [&]() { return seq_back(c, m, nm, fs, os, ahead); });
+            }
+            std::vector<DeviceField*> all(fs);
+            all.insert(all.end(), os.begin(), os.end());
+            return run_cached(c, (7 + 16 * fs.size()) | kind, static_cast<unsigned long long>(c.cur), fields_key(all, false), fields_key(all, true),
+                              [&]() { return seq_back(c, m, nm, fs, os, ahead); });
+        }
+    } // namespace
+
+    int harten_begin_fields(Ctx& c, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os, int ite, double eps, double regularity,
+                            bool relative_detail)
     {
         if (c.cfg.ghost_width > 2)
         {
@@ -1370,16 +1383,29 @@ namespace sg
         // the captured front differs with relative details and with the
         // number of fields: keys of their own
         c.rel_detail = relative_detail;
-        // the keep_boundary launch is part of the captured front only with --refine-boundary
+        // boundary cells are kept in the captured front only with --refine-boundary
         const unsigned long long rb = c.refine_boundary ? 256ull : 0ull;
+        int st;
         if (fs.size() == 1)
         {
             DeviceField& f = *fs[0];
-            return run_cached(c, (relative_detail ? 4 : 2) | rb, static_cast<unsigned long long>(c.cur), ptr_key(f.data),
-                              f.has_bc ? bits_of(f.bc_value) : 1ull, [&]() { return seq_front(c, m, nm, fs); });
+            st             = run_cached(c, (relative_detail ? 4 : 2) | rb, static_cast<unsigned long long>(c.cur), ptr_key(f.data),
+                                        f.has_bc ? bits_of(f.bc_value) : 1ull, [&]() { return seq_front(c, m, nm, fs); });
         }
-        return run_cached(c, (relative_detail ? 6 : 5) | rb, static_cast<unsigned long long>(c.cur), fields_key(fs, false), fs.size(),
-                          [&]() { return seq_front(c, m, nm, fs); });
+        else
+        {
+            st = run_cached(c, (relative_detail ? 6 : 5) | rb, static_cast<unsigned long long>(c.cur), fields_key(fs, false), fs.size(),
+                            [&]() { return seq_front(c, m, nm, fs); });
+        }
+        // The first pass of an adaptation usually changes the mesh: its second half is queued before the host
+        // hears of it (it writes only the spare mesh and the spare buffers, and hangs on the pass's flag), so
+        // the GPU does not wait for the round trip.
+        c.back_ahead = !st && ite == 0;
+        if (c.back_ahead)
+        {
+            st = launch_back(c, fs, os, true);
+        }
+        return st;
     }
 
     int harten_end(Ctx& c, DeviceField& f, bool* converged)
@@ -1389,12 +1415,17 @@ namespace sg
 
     int harten_end_fields(Ctx& c, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os, bool* converged)
     {
-        DeviceMesh& m  = c.m();
-        DeviceMesh& nm = c.spare();
+        DeviceMesh& m    = c.m();
+        DeviceMesh& nm   = c.spare();
+        bool back_queued = c.back_ahead;
         int st;
         if (cudaStreamSynchronize(c.stream) != cudaSuccess)
         {
             return check(c, "harten front sync");
+        }
+        if (!m.host_valid && (st = counts_arrived(c, m)))
+        {
+            return st;
         }
         for (DeviceField* f : fs)
         {
@@ -1405,6 +1436,7 @@ namespace sg
         {
             // graduation still refining after two passes: finish the fixed
             // point with host-tested passes, then compare again
+            back_queued = false;
             if ((st = graduate(c, m, nm, nullptr)))
             {
                 return st;
@@ -1428,20 +1460,7 @@ namespace sg
             return SG_OK;
         }
         *converged = false;
-        if (fs.size() == 1 && os.empty())
-        {
-            DeviceField& f = *fs[0];
-            st             = run_cached(c, 3, static_cast<unsigned long long>(c.cur), ptr_key(f.data), ptr_key(f.spare),
-                                        [&]() { return seq_back(c, m, nm, fs, os); });
-        }
-        else
-        {
-            std::vector<DeviceField*> all(fs);
-            all.insert(all.end(), os.begin(), os.end());
-            st = run_cached(c, 7 + 16 * fs.size(), static_cast<unsigned long long>(c.cur), fields_key(all, false), fields_key(all, true),
-                            [&]() { return seq_back(c, m, nm, fs, os); });
-        }
-        if (st)
+        if (!back_queued && (st = launch_back(c, fs, os, false)))
         {
             return st;
         }
@@ -1457,6 +1476,13 @@ namespace sg
         c.cur = 1 - c.cur;
         ++c.mesh_version;
         return SG_OK;
+    }
+
+    // The error word of an adaptation: a last pass that kept the mesh reported it with its flags, and nothing
+    // ran after it; otherwise it is read from the device.
+    int pass_error(Ctx& c, bool converged)
+    {
+        return converged && c.h_flags[F_ERR] == 0 ? SG_OK : device_error(c);
     }
 
     // No synchronisation before the pass: the pinned thresholds it rewrites
@@ -1823,11 +1849,12 @@ namespace sg
         }
         const int minl = c.cfg.min_level, maxl = c.cfg.max_level;
         int it         = 0;
+        bool conv      = false;
         for (int i = 0; minl != maxl && i < maxl - minl; ++i)
         {
             ++it;
-            bool conv = false;
-            int st    = harten_begin_fields(c, fs, i, eps, regularity, relative_detail);
+            conv      = false;
+            int st    = harten_begin_fields(c, fs, os, i, eps, regularity, relative_detail);
             if (!st)
             {
                 st = harten_end_fields(c, fs, os, &conv);
@@ -1845,7 +1872,7 @@ namespace sg
         {
             *n_harten = it;
         }
-        return device_error(c);
+        return pass_error(c, conv);
     }
 
     // Adapt::operator() (mr/adapt.hpp:147-195)
@@ -1859,12 +1886,13 @@ namespace sg
         }
         const int minl = c.cfg.min_level, maxl = c.cfg.max_level;
         int it         = 0;
+        bool conv      = false;
         if (minl != maxl)
         {
             for (int i = 0; i < maxl - minl; ++i)
             {
                 ++it;
-                bool conv = false;
+                conv      = false;
                 int st    = harten(c, f, i, eps, regularity, &conv, relative_detail);
                 if (st)
                 {
@@ -1880,7 +1908,7 @@ namespace sg
         {
             *n_harten = it;
         }
-        return device_error(c);
+        return pass_error(c, conv);
     }
 
     // the upwind step on mesh m from the values at ud into unp1d

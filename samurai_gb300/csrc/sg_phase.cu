@@ -37,6 +37,17 @@ namespace sg
             {
                 E.flags[T.tid] = 0;
             }
+            if (E.setup_host)
+            {
+                for (int k = T.tid; k < 3 * MAXLEV; k += T.nthr)
+                {
+                    E.setup->eps[k] = E.setup_host->eps[k];
+                }
+                if (T.tid == 0)
+                {
+                    E.setup->ite = E.setup_host->ite;
+                }
+            }
             team_ref_words(E, E.m, T,
                            [&](int w)
                            {
@@ -1171,6 +1182,10 @@ namespace sg
                         M.lo[3]                 = static_cast<long long>(nz >> 32);
                         M.lo[LO_REF + g.nlev]   = M.lo[1];
                         M.lo[LO_CELLS + g.nlev] = M.lo[3];
+                        for (int k = 0; k < 4; ++k)
+                        {
+                            M.host_lo[k] = M.lo[k];
+                        }
                     }
                 }
             }
@@ -1296,6 +1311,14 @@ namespace sg
             }
         }
 
+        __device__ __forceinline__ void op_report(const Env& E, const Team& T)
+        {
+            if (T.tid < F_COUNT)
+            {
+                E.report[T.tid] = T.tid == F_ERR ? *E.g.err : E.flags[T.tid];
+            }
+        }
+
         // ---------------------------------------------------------- dispatch
         template <int DIM, int OP>
         __device__ __forceinline__ void run_op(const Env& E, const Phase& p, const Team& T)
@@ -1332,6 +1355,7 @@ namespace sg
             if constexpr (OP == OP_SCAN_WRITE) op_scan_write<DIM>(E);
             if constexpr (OP == OP_UPDATE_FIELDS) op_update_fields<DIM>(E, T);
             if constexpr (OP == OP_PERIODIC_COPY) op_periodic_copy(E, p.l0, p.aux, T);
+            if constexpr (OP == OP_REPORT) op_report(E, T);
             if constexpr (OP == OP_PERIODIC_TAG) op_periodic_tag(E, p.l0, p.aux >> 1, p.aux & 1, T);
         }
 
@@ -1349,7 +1373,7 @@ namespace sg
         template <int DIM, int OP>
         __global__ void k_phase(const __grid_constant__ Env E, const __grid_constant__ Phase p)
         {
-            if (OP >= OP_GRAD_COARSEN && OP <= OP_GRAD_APPLY && guarded_off(E, p))
+            if ((OP >= OP_GRAD_COARSEN && OP <= OP_GRAD_APPLY && guarded_off(E, p)) || (E.guard && *E.guard == 0))
             {
                 return;
             }
@@ -1418,6 +1442,10 @@ namespace sg
                 __syncthreads();
             }
             const Env& E = *reinterpret_cast<const Env*>(store);
+            if (E.guard && *E.guard == 0)
+            {
+                return; // the whole cluster: the flag was settled before the launch
+            }
             const Team T = grid_team();
             for (int i = 0; i < L.n; ++i)
             {
@@ -1446,7 +1474,7 @@ namespace sg
             "new_cells",      "grad_coarsen", "grad_expand",   "grad_expand_xy", "grad_expand_z", "grad_periodic", "grad_down", "grad_refine",
             "grad_apply",     "compare",      "clear_union",   "hc_cag",       "hc2_cag",      "cag_on",       "ref0",       "ref0_xy",
             "ref0_z",         "ref_periodic_src", "ref_periodic", "ref_children", "ref_children", "proj",      "single_level", "scan_sums",
-            "scan_write",     "update_fields", "periodic_copy", "periodic_tag"};
+            "scan_write",     "update_fields", "periodic_copy", "periodic_tag", "report"};
 
         enum class Shape
         {
@@ -1472,7 +1500,8 @@ namespace sg
                 case OP_SCAN_WRITE: return Shape::SCAN;
                 case OP_ABSMAX_INIT:
                 case OP_PERIODIC_COPY:
-                case OP_PERIODIC_TAG: return Shape::OTHER;
+                case OP_PERIODIC_TAG:
+                case OP_REPORT: return Shape::OTHER;
                 default: return Shape::WORDS;
             }
         }
@@ -1500,7 +1529,8 @@ namespace sg
             case OP_GRAD_DOWN:
             case OP_REF_CHILDREN_LEVEL: return range_words(g, p.l0, p.l0);
             case OP_MAXIMUM: return range_words(g, p.l0 - 1, p.l0 - 1);
-            case OP_ABSMAX_INIT: return 1;
+            case OP_ABSMAX_INIT:
+            case OP_REPORT: return 1;
             default: return g.total_words;
         }
     }
@@ -1559,7 +1589,7 @@ namespace sg
                 break;
             case Shape::SCAN: grid = (g.total_words + SCAN_WORDS - 1) / SCAN_WORDS; break;
             case Shape::OTHER:
-                grid = p.op == OP_ABSMAX_INIT ? 1 : (2 * periodic_side_items(g, p.l0) + block - 1) / block;
+                grid = p.op == OP_ABSMAX_INIT || p.op == OP_REPORT ? 1 : (2 * periodic_side_items(g, p.l0) + block - 1) / block;
                 break;
         }
         if (grid < 1)
@@ -1632,7 +1662,7 @@ namespace sg
     // ------------------------------------------------------------ sequences
     MeshPtrs mesh_ptrs(const DeviceMesh& m)
     {
-        return {m.cells, m.cag, m.proj, m.uni, m.ref, m.hc, m.hc2, m.pred, m.rank, m.wl_ref, m.wl_cells, m.d_lo};
+        return {m.cells, m.cag, m.proj, m.uni, m.ref, m.hc, m.hc2, m.pred, m.rank, m.wl_ref, m.wl_cells, m.d_lo, m.h_lo};
     }
 
     Sequence::Sequence(Ctx& ctx, const DeviceMesh& m, const DeviceMesh& n)
@@ -1656,6 +1686,7 @@ namespace sg
         env.det             = c.detail;
         env.capacity        = c.capacity;
         env.setup           = c.d_setup;
+        env.report          = c.h_flags;
         env.absmax          = c.d_absmax;
         env.flags           = c.d_flags;
         env.block_sums      = c.block_sums;
@@ -1680,6 +1711,15 @@ namespace sg
         }
         env.det    = c.detail ? c.detail + static_cast<long long>(first) * c.capacity : nullptr;
         env.absmax = c.d_absmax + first;
+    }
+
+    void Sequence::guard(const int* flag)
+    {
+        if (flag != env.guard)
+        {
+            flush();
+            env.guard = flag;
+        }
     }
 
     // A phase joins the pending chain when it walks few enough words for one

@@ -60,6 +60,7 @@ namespace sg
         OP_UPDATE_FIELDS,   // from mesh m to mesh n
         OP_PERIODIC_COPY,   // level l0, axis aux
         OP_PERIODIC_TAG,    // level l0, axis aux >> 1, side aux & 1
+        OP_REPORT,          // flags and error word to the host
         OP_COUNT
     };
 
@@ -80,6 +81,7 @@ namespace sg
         uint32_t *cells, *cag, *proj, *uni, *ref, *hc, *hc2, *pred;
         int *rank, *wl_ref, *wl_cells;
         long long* lo;
+        long long* host_lo; // pinned: the scan leaves the counters [0..3] here too
     };
 
     struct FieldSlot
@@ -101,7 +103,10 @@ namespace sg
         uint32_t *above, *ref_above, *par_above; // |detail| over the coarsen, refine and parent thresholds
         double* det;
         long long capacity;
-        const PassSetup* setup;
+        PassSetup* setup;
+        const PassSetup* setup_host; // pinned: copied into setup when a pass begins (null: setup is in place)
+        int* report;                 // pinned: the flags of a pass, with the mesh's error word at F_ERR
+        const int* guard;            // when not null, the phases run only if this flag is set
         unsigned long long* absmax;
         int* flags;
         long long* block_sums;
@@ -135,7 +140,8 @@ namespace sg
         Sequence(Ctx& ctx, const DeviceMesh& m, const DeviceMesh& n);
         void fields(const FieldSlot* fs, int first, int nf); // the fields of the following phases: fs[first .. first + nf)
         void add(int op, int l0 = 0, int l1 = 0, int aux = 0);
-        void flush(); // before anything else is queued on the stream
+        void guard(const int* flag); // the following phases hang on a device flag
+        void flush();                // before anything else is queued on the stream
         void timer_start(int id);
         void timer_stop(int id);
         int done(const char* what);
