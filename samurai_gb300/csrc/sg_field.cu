@@ -198,9 +198,11 @@ namespace sg
 
         struct UpwindArgs
         {
-            double a[3];
             double ha[3]; // .5 * a_d, as the reference's flux forms it
             double hb[3]; // .5 * |a_d|
+            double fl[3]; // the flux form's coefficients of the left and the right value: (a, 0) or (0, a)
+            double fr[3];
+            bool zero_l[3], zero_r[3]; // which of them are zero
             double dt;
             int scheme;
         };
@@ -318,182 +320,270 @@ namespace sg
         // Coefficients: face length^(dim-1) / cell volume times the upwind flux
         // coefficients (a, 0) for a >= 0, (0, a) otherwise; every factor is a
         // power of two.
-        template <int DIM>
-        __global__ void k_convection(const __grid_constant__ Geom gp, const int* __restrict__ wl, const long long* __restrict__ lo, const uint32_t* __restrict__ cells, const double* __restrict__ u,
-                                     double* __restrict__ unp1, UpwindArgs p)
+        // Bound by the FP64 pipe, so only the terms that can change the sum are
+        // formed: one of the two flux coefficients is zero, and a term 0 * v adds
+        // +-0 to a sum that starts at +0 and is never -0, which leaves its bits as
+        // they are unless v is infinite or NaN (tested on the exponent).  Products
+        // with 2^l move the exponent, same-level neighbours sit at fixed strides.
+
+        // acc + c * v; zero: c is zero
+        __device__ __forceinline__ double add_term(double acc, double c, bool zero, double v)
         {
-            const Geom& g     = gp;
-            block_items(wl, static_cast<int>(lo[LO_CELLS]), static_cast<int>(lo[LO_CELLS + g.nlev]), grid_team(), 1, [&](int w) { return __ldg(cells + w); },
-                              [&](bool valid, int w_, int b, int)
-                              {
-                                  if (!valid)
-                                  {
-                                      return;
-                                  }
-                                  const long long w  = w_;
-                                  const int m        = level_down(g, w_, 0, g.max_level);
-                                  const Cell cc      = cell_of(g, m, w, b);
-                                  const int c[3]     = {cc.x, cc.y, cc.z};
-                                  const long long eX = 32 * w + b;
-                                  const double uX    = u[eX];
-                                  const int nm       = 1 << m;
-                                  auto leaf = [&](int l, const int* q)
-                                  {
-                                      const Pos at = l >= 0 && l <= g.max_level ? pos_of(g, l, q[0], q[1], DIM == 3 ? q[2] : 0) : Pos{-1, 0};
-                                      return at.w >= 0 && ((__ldg(cells + at.w) >> at.b) & 1u);
-                                  };
-                                  auto val  = [&](int l, const int* q) { return u[elem_at(g, l, q[0], q[1], DIM == 3 ? q[2] : 0)]; };
-                                  double acc = 0.;
-                                  for (int d = 0; d < DIM; ++d)
-                                  {
-                                      const double a  = p.a[d];
-                                      const double fl = a >= 0 ? a : 0.;
-                                      const double fr = a >= 0 ? 0. : a;
-                                      int xp[3] = {c[0], c[1], c[2]}, xm[3] = {c[0], c[1], c[2]};
-                                      ++xp[d];
-                                      --xm[d];
-                                      const double s2   = pow2(m);
-                                      const double lc0 = s2 * fl, lc1 = s2 * fr;
-                                      const double rc0 = -lc0, rc1 = -lc1;
-                                      const bool rs = leaf(m, xp), ls = leaf(m, xm);
-                                      // same level
-                                      if (d == 0)
-                                      {
-                                          if (rs) acc = acc + lc0 * uX;
-                                          if (ls) acc = acc + rc0 * val(m, xm);
-                                          if (rs) acc = acc + lc1 * val(m, xp);
-                                          if (ls) acc = acc + rc1 * uX;
-                                      }
-                                      else
-                                      {
-                                          if (ls)
-                                          {
-                                              acc = acc + rc0 * val(m, xm);
-                                              acc = acc + rc1 * uX;
-                                          }
-                                          if (rs)
-                                          {
-                                              acc = acc + lc0 * uX;
-                                              acc = acc + lc1 * val(m, xp);
-                                          }
-                                      }
-                                      const bool out_r = xp[d] >= nm, out_l = xm[d] < 0;
-                                      // level jumps with X the fine cell
-                                      int pp[3] = {xp[0] >> 1, xp[1] >> 1, xp[2] >> 1}, pm[3] = {xm[0] >> 1, xm[1] >> 1, xm[2] >> 1};
-                                      const bool lcoarse = !ls && !out_l && m >= 1 && leaf(m - 1, pm);
-                                      const bool rcoarse = !rs && !out_r && m >= 1 && leaf(m - 1, pp);
-                                      if (lcoarse)
-                                      {
-                                          acc = acc + rc0 * val(m, xm);
-                                          acc = acc + rc1 * uX;
-                                      }
-                                      if (rcoarse)
-                                      {
-                                          acc = acc + lc0 * uX;
-                                          acc = acc + lc1 * val(m, xp);
-                                      }
-                                      // level jumps with X the coarse cell: its face children at m+1
-                                      const double sf = pow2(m - DIM + 1);
-                                      int ch[3]       = {2 * c[0], 2 * c[1], 2 * c[2]};
-                                      ch[d]           = 2 * c[d] + 2;
-                                      const bool rfine = !rs && !rcoarse && !out_r && leaf(m + 1, ch);
-                                      ch[d]            = 2 * c[d] - 1;
-                                      const bool lfine = !ls && !lcoarse && !out_l && leaf(m + 1, ch);
-                                      // fine rows of the face in row order (z outer, y inner); a face
-                                      // normal to y or z has the pair of fine cells within each row
-                                      const int nrow = (d == 0) ? (DIM == 3 ? 4 : 2) : (DIM == 3 ? 2 : 1);
-                                      if (rfine)
-                                      {
-                                          const double j0 = sf * fl, j1 = sf * fr;
-                                          for (int r = 0; r < nrow; ++r)
-                                          {
-                                              int q[3] = {2 * c[0], 2 * c[1], 2 * c[2]};
-                                              q[d]     = 2 * c[d] + 1;
-                                              if (d == 0)
-                                              {
-                                                  q[1] += r & 1;
-                                                  if (DIM == 3)
-                                                  {
-                                                      q[2] += r >> 1;
-                                                  }
-                                                  int qe[3] = {q[0] + 1, q[1], q[2]};
-                                                  acc       = acc + j0 * val(m + 1, q);
-                                                  acc       = acc + j1 * val(m + 1, qe);
-                                              }
-                                              else
-                                              {
-                                                  if (DIM == 3)
-                                                  {
-                                                      q[d == 1 ? 2 : 1] += r;
-                                                  }
-                                                  int qb[3] = {q[0] + 1, q[1], q[2]};
-                                                  int qe[3] = {q[0], q[1], q[2]}, qbe[3] = {qb[0], qb[1], qb[2]};
-                                                  ++qe[d];
-                                                  ++qbe[d];
-                                                  acc = acc + (j0 * val(m + 1, q) + j0 * val(m + 1, qb));
-                                                  acc = acc + (j1 * val(m + 1, qe) + j1 * val(m + 1, qbe));
-                                              }
-                                          }
-                                      }
-                                      if (lfine)
-                                      {
-                                          const double j0 = -sf * fl, j1 = -sf * fr;
-                                          for (int r = 0; r < nrow; ++r)
-                                          {
-                                              int q[3] = {2 * c[0], 2 * c[1], 2 * c[2]}; // Q, inside X on its left face
-                                              if (d == 0)
-                                              {
-                                                  q[1] += r & 1;
-                                                  if (DIM == 3)
-                                                  {
-                                                      q[2] += r >> 1;
-                                                  }
-                                                  int qm[3] = {q[0] - 1, q[1], q[2]};
-                                                  acc       = acc + j0 * val(m + 1, qm);
-                                                  acc       = acc + j1 * val(m + 1, q);
-                                              }
-                                              else
-                                              {
-                                                  if (DIM == 3)
-                                                  {
-                                                      q[d == 1 ? 2 : 1] += r;
-                                                  }
-                                                  int qb[3] = {q[0] + 1, q[1], q[2]};
-                                                  int qm[3] = {q[0], q[1], q[2]}, qbm[3] = {qb[0], qb[1], qb[2]};
-                                                  --qm[d];
-                                                  --qbm[d];
-                                                  acc = acc + (j0 * val(m + 1, qm) + j0 * val(m + 1, qbm));
-                                                  acc = acc + (j1 * val(m + 1, q) + j1 * val(m + 1, qb));
-                                              }
-                                          }
-                                      }
-                                      // boundary interfaces
-                                      if (out_r)
-                                      {
-                                          acc = acc + lc0 * uX;
-                                          acc = acc + lc1 * val(m, xp);
-                                      }
-                                      if (out_l)
-                                      {
-                                          acc = acc + (-lc0) * val(m, xm);
-                                          acc = acc + (-lc1) * uX;
-                                      }
-                                  }
-                                  unp1[eX] = uX - p.dt * acc;
-            });
+            if (zero && ((__double2hiint(v) >> 20) & 0x7FF) != 0x7FF)
+            {
+                return acc;
+            }
+            return acc + c * v;
+        }
+
+        // acc + (c * v + c * w)
+        __device__ __forceinline__ double add_pair(double acc, double c, bool zero, double v, double w)
+        {
+            if (zero && ((__double2hiint(v) >> 20) & 0x7FF) != 0x7FF && ((__double2hiint(w) >> 20) & 0x7FF) != 0x7FF)
+            {
+                return acc;
+            }
+            return acc + (c * v + c * w);
+        }
+
+        template <int DIM>
+        __global__ void k_convection(const __grid_constant__ Geom gp, const int* __restrict__ wl, const long long* __restrict__ lo,
+                                     const uint32_t* __restrict__ cells, const double* __restrict__ u, double* __restrict__ unp1, UpwindArgs p)
+        {
+            const Geom& g = gp;
+            block_items(
+                wl, static_cast<int>(lo[LO_CELLS]), static_cast<int>(lo[LO_CELLS + g.nlev]), grid_team(), 1, [&](int w) { return __ldg(cells + w); },
+                [&](bool valid, int w_, int b, int)
+                {
+                    if (!valid)
+                    {
+                        return;
+                    }
+                    const long long w  = w_;
+                    const int m        = level_down(g, w_, 0, g.max_level);
+                    const Cell cc      = cell_of(g, m, w, b);
+                    const int c[3]     = {cc.x, cc.y, cc.z};
+                    const long long eX = 32 * w + b;
+                    const long long strides[3] = {1, 32LL * g.lv[m].W, 32LL * g.lv[m].W * g.lv[m].R};
+                    const double uX    = u[eX];
+                    const int nm       = 1 << m;
+                    auto leaf          = [&](int l, const int* q)
+                    {
+                        const Pos at = l >= 0 && l <= g.max_level ? pos_of(g, l, q[0], q[1], DIM == 3 ? q[2] : 0) : Pos{-1, 0};
+                        return at.w >= 0 && ((__ldg(cells + at.w) >> at.b) & 1u);
+                    };
+                    auto val = [&](int l, const int* q) { return u[elem_at(g, l, q[0], q[1], DIM == 3 ? q[2] : 0)]; };
+                    // a same-level leaf at element e
+                    auto leaf_elem = [&](long long e) { return (__ldg(cells + (e >> 5)) >> (e & 31)) & 1u; };
+                    double um[DIM], up[DIM];
+                    bool ls_[DIM], rs_[DIM];
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d)
+                    {
+                        um[d]  = u[eX - strides[d]];
+                        up[d]  = u[eX + strides[d]];
+                        ls_[d] = leaf_elem(eX - strides[d]);
+                        rs_[d] = leaf_elem(eX + strides[d]);
+                    }
+                    double acc = 0.;
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d)
+                    {
+                        // (a, 0) or (0, a): the coefficient of the left and of the right value
+                        const double fl = p.fl[d], fr = p.fr[d];
+                        const bool zl = p.zero_l[d], zr = p.zero_r[d];
+                        const double lc0 = scale2(fl, m), lc1 = scale2(fr, m);
+                        const double rc0 = -lc0, rc1 = -lc1;
+                        const bool rs = rs_[d], ls = ls_[d];
+                        // same level
+                        if (d == 0)
+                        {
+                            if (rs) acc = add_term(acc, lc0, zl, uX);
+                            if (ls) acc = add_term(acc, rc0, zl, um[d]);
+                            if (rs) acc = add_term(acc, lc1, zr, up[d]);
+                            if (ls) acc = add_term(acc, rc1, zr, uX);
+                        }
+                        else
+                        {
+                            if (ls)
+                            {
+                                acc = add_term(acc, rc0, zl, um[d]);
+                                acc = add_term(acc, rc1, zr, uX);
+                            }
+                            if (rs)
+                            {
+                                acc = add_term(acc, lc0, zl, uX);
+                                acc = add_term(acc, lc1, zr, up[d]);
+                            }
+                        }
+                        if (rs && ls)
+                        {
+                            continue; // no other face along d
+                        }
+                        int xp[3] = {c[0], c[1], c[2]}, xm[3] = {c[0], c[1], c[2]};
+                        ++xp[d];
+                        --xm[d];
+                        const bool out_r = xp[d] >= nm, out_l = xm[d] < 0;
+                        // level jumps with X the fine cell
+                        int pp[3] = {xp[0] >> 1, xp[1] >> 1, xp[2] >> 1}, pm[3] = {xm[0] >> 1, xm[1] >> 1, xm[2] >> 1};
+                        const bool lcoarse = !ls && !out_l && m >= 1 && leaf(m - 1, pm);
+                        const bool rcoarse = !rs && !out_r && m >= 1 && leaf(m - 1, pp);
+                        if (lcoarse)
+                        {
+                            acc = add_term(acc, rc0, zl, um[d]);
+                            acc = add_term(acc, rc1, zr, uX);
+                        }
+                        if (rcoarse)
+                        {
+                            acc = add_term(acc, lc0, zl, uX);
+                            acc = add_term(acc, lc1, zr, up[d]);
+                        }
+                        // level jumps with X the coarse cell: its face children at m+1
+                        int ch[3]        = {2 * c[0], 2 * c[1], 2 * c[2]};
+                        ch[d]            = 2 * c[d] + 2;
+                        const bool rfine = !rs && !rcoarse && !out_r && leaf(m + 1, ch);
+                        ch[d]            = 2 * c[d] - 1;
+                        const bool lfine = !ls && !lcoarse && !out_l && leaf(m + 1, ch);
+                        // fine rows of the face in row order (z outer, y inner); a face
+                        // normal to y or z has the pair of fine cells within each row
+                        const int nrow = (d == 0) ? (DIM == 3 ? 4 : 2) : (DIM == 3 ? 2 : 1);
+                        const double sf = pow2(m - DIM + 1);
+                        if (rfine)
+                        {
+                            const double j0 = sf * fl, j1 = sf * fr;
+                            for (int r = 0; r < nrow; ++r)
+                            {
+                                int q[3] = {2 * c[0], 2 * c[1], 2 * c[2]};
+                                q[d]     = 2 * c[d] + 1;
+                                if (d == 0)
+                                {
+                                    q[1] += r & 1;
+                                    if (DIM == 3)
+                                    {
+                                        q[2] += r >> 1;
+                                    }
+                                    int qe[3] = {q[0] + 1, q[1], q[2]};
+                                    acc       = add_term(acc, j0, zl, val(m + 1, q));
+                                    acc       = add_term(acc, j1, zr, val(m + 1, qe));
+                                }
+                                else
+                                {
+                                    if (DIM == 3)
+                                    {
+                                        q[d == 1 ? 2 : 1] += r;
+                                    }
+                                    int qb[3] = {q[0] + 1, q[1], q[2]};
+                                    int qe[3] = {q[0], q[1], q[2]}, qbe[3] = {qb[0], qb[1], qb[2]};
+                                    ++qe[d];
+                                    ++qbe[d];
+                                    acc = add_pair(acc, j0, zl, val(m + 1, q), val(m + 1, qb));
+                                    acc = add_pair(acc, j1, zr, val(m + 1, qe), val(m + 1, qbe));
+                                }
+                            }
+                        }
+                        if (lfine)
+                        {
+                            const double j0 = -sf * fl, j1 = -sf * fr;
+                            for (int r = 0; r < nrow; ++r)
+                            {
+                                int q[3] = {2 * c[0], 2 * c[1], 2 * c[2]}; // Q, inside X on its left face
+                                if (d == 0)
+                                {
+                                    q[1] += r & 1;
+                                    if (DIM == 3)
+                                    {
+                                        q[2] += r >> 1;
+                                    }
+                                    int qm[3] = {q[0] - 1, q[1], q[2]};
+                                    acc       = add_term(acc, j0, zl, val(m + 1, qm));
+                                    acc       = add_term(acc, j1, zr, val(m + 1, q));
+                                }
+                                else
+                                {
+                                    if (DIM == 3)
+                                    {
+                                        q[d == 1 ? 2 : 1] += r;
+                                    }
+                                    int qb[3] = {q[0] + 1, q[1], q[2]};
+                                    int qm[3] = {q[0], q[1], q[2]}, qbm[3] = {qb[0], qb[1], qb[2]};
+                                    --qm[d];
+                                    --qbm[d];
+                                    acc = add_pair(acc, j0, zl, val(m + 1, qm), val(m + 1, qbm));
+                                    acc = add_pair(acc, j1, zr, val(m + 1, q), val(m + 1, qb));
+                                }
+                            }
+                        }
+                        // boundary interfaces
+                        if (out_r)
+                        {
+                            acc = add_term(acc, lc0, zl, uX);
+                            acc = add_term(acc, lc1, zr, up[d]);
+                        }
+                        if (out_l)
+                        {
+                            acc = add_term(acc, -lc0, zl, um[d]);
+                            acc = add_term(acc, -lc1, zr, uX);
+                        }
+                    }
+                    unp1[eX] = uX - p.dt * acc;
+                });
         }
 
         // --------------------------------------------------- layout moves
-        __global__ void k_gather(const int* wl, const long long* lo, int nlev, const uint32_t* ref, const int* rank, const double* dense, double* compact)
+        // Each warp takes MOVE_WORDS listed words at a time: their bits and ranks are loaded by one lane each, then
+        // the words' values move together, all loads in flight at once (a warp per word waits for list entry,
+        // bits, rank and value in turn, word after word).
+        constexpr int MOVE_WORDS = 8;
+
+        template <class LoadF, class StoreF>
+        __device__ __forceinline__ void move_words(const int* __restrict__ wl, const long long* __restrict__ lo, int nlev, const uint32_t* __restrict__ ref,
+                                                   const int* __restrict__ rank, LoadF load, StoreF store)
         {
-            warp_list(wl, lo[LO_REF], lo[LO_REF + nlev], warp_id(), warp_count(), [&](long long w) { return ref[w]; },
-                      [&](long long w, int b) { compact[ref_index(ref, rank, Pos{w, b})] = dense[32 * w + b]; });
+            const int lane  = threadIdx.x & 31;
+            const int begin = static_cast<int>(lo[LO_REF]), end = static_cast<int>(lo[LO_REF + nlev]);
+            for (int c0 = begin + static_cast<int>(warp_id()) * MOVE_WORDS; c0 < end; c0 += static_cast<int>(warp_count()) * MOVE_WORDS)
+            {
+                int w      = 0, r = 0;
+                uint32_t m = 0u;
+                if (lane < MOVE_WORDS && c0 + lane < end)
+                {
+                    w = wl[c0 + lane];
+                    m = ref[w];
+                    r = rank[w];
+                }
+                double v[MOVE_WORDS];
+#pragma unroll
+                for (int k = 0; k < MOVE_WORDS; ++k)
+                {
+                    const long long e   = 32LL * __shfl_sync(FULL_MASK, w, k) + lane;
+                    const uint32_t bits = __shfl_sync(FULL_MASK, m, k);
+                    const int at        = __shfl_sync(FULL_MASK, r, k) + __popc(bits & ((1u << lane) - 1u));
+                    v[k]                = ((bits >> lane) & 1u) ? load(e, at) : 0.;
+                }
+#pragma unroll
+                for (int k = 0; k < MOVE_WORDS; ++k)
+                {
+                    const long long e   = 32LL * __shfl_sync(FULL_MASK, w, k) + lane;
+                    const uint32_t bits = __shfl_sync(FULL_MASK, m, k);
+                    const int at        = __shfl_sync(FULL_MASK, r, k) + __popc(bits & ((1u << lane) - 1u));
+                    if ((bits >> lane) & 1u)
+                    {
+                        store(e, at, v[k]);
+                    }
+                }
+            }
         }
 
-        __global__ void k_scatter(const int* wl, const long long* lo, int nlev, const uint32_t* ref, const int* rank, const double* compact, double* dense)
+        __global__ void k_gather(const int* wl, const long long* lo, int nlev, const uint32_t* ref, const int* rank, const double* __restrict__ dense,
+                                 double* __restrict__ compact)
         {
-            warp_list(wl, lo[LO_REF], lo[LO_REF + nlev], warp_id(), warp_count(), [&](long long w) { return ref[w]; },
-                      [&](long long w, int b) { dense[32 * w + b] = compact[ref_index(ref, rank, Pos{w, b})]; });
+            move_words(wl, lo, nlev, ref, rank, [&](long long e, int) { return dense[e]; }, [&](long long, int at, double v) { compact[at] = v; });
+        }
+
+        __global__ void k_scatter(const int* wl, const long long* lo, int nlev, const uint32_t* ref, const int* rank, const double* __restrict__ compact,
+                                  double* __restrict__ dense)
+        {
+            move_words(wl, lo, nlev, ref, rank, [&](long long, int at) { return compact[at]; }, [&](long long e, int, double v) { dense[e] = v; });
         }
 
         // details in the reference numbering: a cell whose parent the pass did not examine has none (0)
@@ -1918,7 +2008,10 @@ namespace sg
         UpwindArgs p{};
         for (int d = 0; d < g.dim; ++d)
         {
-            p.a[d]  = a[d];
+            p.fl[d] = a[d] >= 0 ? a[d] : 0.;
+            p.fr[d] = a[d] >= 0 ? 0. : a[d];
+            p.zero_l[d] = p.fl[d] == 0.;
+            p.zero_r[d] = p.fr[d] == 0.;
             p.ha[d] = .5 * a[d];
             p.hb[d] = .5 * std::fabs(a[d]);
         }
