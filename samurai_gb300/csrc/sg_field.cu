@@ -346,8 +346,9 @@ namespace sg
             return acc + (c * v + c * w);
         }
 
+        // 64 registers: the level-jump branches want 90, which leaves two blocks of 256 on an SM
         template <int DIM>
-        __global__ void k_convection(const __grid_constant__ Geom gp, const int* __restrict__ wl, const long long* __restrict__ lo,
+        __global__ void __launch_bounds__(ITEM_BLOCK, 2) k_convection(const __grid_constant__ Geom gp, const int* __restrict__ wl, const long long* __restrict__ lo,
                                      const uint32_t* __restrict__ cells, const double* __restrict__ u, double* __restrict__ unp1, UpwindArgs p)
         {
             const Geom& g = gp;
@@ -2017,16 +2018,17 @@ namespace sg
         }
         p.dt     = dt;
         p.scheme = scheme;
-        const int nb = blocks_words(c, 0, g.nlev - 1);
+        const int nb    = blocks_words(c, 0, g.nlev - 1);
+        const int block = std::min(c.block, ITEM_BLOCK);
         if (scheme == 2)
         {
             if (g.dim == 2)
             {
-                k_convection<2><<<nb, c.block, 0, c.stream>>>(c.g, m.wl_cells, m.d_lo, m.cells, ud, unp1d, p);
+                k_convection<2><<<nb, block, 0, c.stream>>>(c.g, m.wl_cells, m.d_lo, m.cells, ud, unp1d, p);
             }
             else
             {
-                k_convection<3><<<nb, c.block, 0, c.stream>>>(c.g, m.wl_cells, m.d_lo, m.cells, ud, unp1d, p);
+                k_convection<3><<<nb, block, 0, c.stream>>>(c.g, m.wl_cells, m.d_lo, m.cells, ud, unp1d, p);
             }
         }
         else if (g.dim == 2)

@@ -1117,6 +1117,22 @@ namespace sg
                     const int w       = s + lane;
                     const bool in     = w < n;
                     const uint32_t r  = in ? M.ref[w] : 0u, c = in ? M.cells[w] : 0u;
+                    const uint32_t br = __ballot_sync(FULL_MASK, r != 0u), bc = __ballot_sync(FULL_MASK, c != 0u);
+                    const int l       = in ? level_down(g, w, 0, g.max_level) : 0;
+                    if ((br | bc) == 0u)
+                    {
+                        // 32 empty words (most of a 3D mesh): no cell is looked up in them, so no rank
+                        if (in)
+                        {
+                            M.pred[w] = 0u;
+                            if (w == static_cast<int>(g.lv[l].woff))
+                            {
+                                M.lo[LO_REF + l]   = static_cast<unsigned>(before.nz);
+                                M.lo[LO_CELLS + l] = static_cast<unsigned>(before.nz >> 32);
+                            }
+                        }
+                        continue;
+                    }
                     const Pair t      = word_counts(r, c);
                     unsigned pr       = static_cast<unsigned>(t.pop); // inclusive prefix of the reference cells
                     for (int o = 1; o < 32; o <<= 1)
@@ -1124,7 +1140,6 @@ namespace sg
                         const unsigned x = __shfl_up_sync(FULL_MASK, pr, o);
                         pr += lane >= o ? x : 0u;
                     }
-                    const uint32_t br = __ballot_sync(FULL_MASK, r != 0u), bc = __ballot_sync(FULL_MASK, c != 0u);
                     const uint32_t lower = (1u << lane) - 1u;
                     const unsigned ir = static_cast<unsigned>(before.nz) + __popc(br & lower);
                     const unsigned ic = static_cast<unsigned>(before.nz >> 32) + __popc(bc & lower);
@@ -1139,8 +1154,8 @@ namespace sg
                         {
                             M.wl_cells[ic] = w;
                         }
-                        uint32_t pd = r & ~(c | M.proj[w]);
-                        const int l = level_down(g, w, 0, g.max_level);
+                        uint32_t pd = r & ~c;
+                        pd          = pd ? pd & ~M.proj[w] : 0u;
                         if (pd)
                         {
                             const Word p = word_at<DIM>(g, l, w);
@@ -1544,7 +1559,7 @@ namespace sg
         // blocks that hand out the items of `words` words: a block per 16 words, at most max_blocks blocks of 256 threads
         auto items = [&](long long words)
         {
-            block               = c.block;
+            block               = std::min(c.block, ITEM_BLOCK);
             const long long cap = std::max(1LL, c.max_blocks * 256 / block);
             return std::min(cap, std::max(1LL, (words + 15) / 16));
         };
@@ -1572,7 +1587,7 @@ namespace sg
                 if (p.op == OP_GHOST)
                 {
                     const long long nproj = p.l0 > (g.min_level >= 2 ? g.min_level - 2 : 0) ? items(g.lv[p.l0 - 1].nwords) : 0;
-                    block                 = c.block;
+                    block                 = std::min(c.block, ITEM_BLOCK);
                     const long long edge  = (g.dim == 2 ? boundary_count<2>(g, p.l0) : boundary_count<3>(g, p.l0)) * e.nf;
                     const long long nb    = std::min(16384LL, (edge + block - 1) / block);
                     p.l1                  = static_cast<short>(nb);

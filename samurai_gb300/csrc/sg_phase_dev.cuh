@@ -244,6 +244,7 @@ namespace sg
     // fullest word.  item(valid, w, b, field) is called by every thread of a
     // block (it may shuffle), consecutive threads on consecutive items.
     constexpr int ITEM_THREADS = 1024; // largest block
+    constexpr int ITEM_BLOCK   = 512;  // largest block of the phases and kernels that need more than 64 registers
 
     struct ItemShared
     {
@@ -652,10 +653,16 @@ namespace sg
         const int in[3]  = {axis == 0 ? at : f0, axis == 1 ? at : (axis == 0 ? f0 : f1), DIM == 3 ? (axis == 2 ? at : f1) : 0};
         const int dir[3] = {axis == 0 ? sgn : 0, axis == 1 ? sgn : 0, axis == 2 ? sgn : 0};
         const int gx = in[0] + dir[0], gy = in[1] + dir[1], gz = in[2] + dir[2];
+        // most positions of a fine level have neither a leaf nor a finer leaf behind them; for the others
         // everything the roles ask first is loaded together
-        const Pos pi = pos_of(g, l, in[0], in[1], in[2]);
-        const Pos pg = pos_of(g, l, gx, gy, gz);
-        const uint32_t wc  = cells[pi.w], wu = uni[pi.w], wg = ref[pg.w];
+        const Pos pi      = pos_of(g, l, in[0], in[1], in[2]);
+        const uint32_t wc = cells[pi.w], wu = uni[pi.w];
+        if (!(((wc | wu) >> pi.b) & 1u))
+        {
+            return;
+        }
+        const Pos pg       = pos_of(g, l, gx, gy, gz);
+        const uint32_t wg  = ref[pg.w];
         const long long eg = elem(pg);
         const typename A::V ui = u.get(elem(pi));
         Children<DIM, 2> c2;
