@@ -75,6 +75,7 @@ namespace sg
         F_DIFFER = 2, // new leaf cells differ from the current ones
         F_GRADX = 3,  // scratch for extra graduation passes
         F_ERR   = 4,  // the mesh's error word, in the host's copy
+        F_DONE  = 5,  // blocks of the comparison that are through
         F_COUNT = 8
     };
 

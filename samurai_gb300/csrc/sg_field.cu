@@ -1271,10 +1271,17 @@ namespace sg
             {
                 for (int d = 0; d < g.dim; ++d)
                 {
-                    for (int side = 0; side < 2 && ((g.periodic >> d) & 1); ++side)
+                    if (!((g.periodic >> d) & 1))
                     {
-                        s.add(OP_PERIODIC_TAG, l, l, 2 * d + side);
+                        continue;
                     }
+                    if (g.lv[l].n >= 2 * g.ghost_width)
+                    {
+                        s.add(OP_PERIODIC_TAG, l, l, 4 * d + 3);
+                        continue;
+                    }
+                    s.add(OP_PERIODIC_TAG, l, l, 4 * d + 1);
+                    s.add(OP_PERIODIC_TAG, l, l, 4 * d + 2);
                 }
                 if (l >= std::max(1, minl))
                 {
@@ -1325,11 +1332,8 @@ namespace sg
                     return st;
                 }
             }
+            s.report(graphed ? nullptr : c.h_flags);
             s.add(OP_COMPARE);
-            if (!graphed)
-            {
-                s.add(OP_REPORT);
-            }
             s.timer_stop(T_MESH_UPDATE);
             return s.done("harten front");
         }
@@ -1338,9 +1342,10 @@ namespace sg
         // for the adapted fields fs and the fields os carried along (their
         // ghosts are updated first, mr/adapt.hpp:383)
         // ahead: launched before the host knows whether the pass changed the mesh;
-        // the phases hang on the pass's flag
+        // the phases hang on the pass's flag.  clear: not the first time after the
+        // pass's front, which left the union of the new mesh empty.
         int seq_back(Ctx& c, DeviceMesh& m, DeviceMesh& nm, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os,
-                     bool ahead = false)
+                     bool ahead = false, bool clear = false)
         {
             Sequence s(c, m, nm);
             s.guard(ahead ? c.d_flags + F_DIFFER : nullptr);
@@ -1355,7 +1360,7 @@ namespace sg
             const std::vector<FieldSlot> slots = slots_of(all);
             s.fields(slots.data(), 0, std::min(PHASE_FIELDS, static_cast<int>(slots.size())));
             s.timer_start(T_CONSTRUCTION);
-            build_mesh_phases(s);
+            build_mesh_phases(s, clear);
             s.timer_stop(T_CONSTRUCTION);
             s.timer_start(T_FIELDS_UPDATE);
             field_groups(s, slots, [&]() { s.add(OP_UPDATE_FIELDS); });
@@ -1439,21 +1444,21 @@ namespace sg
     namespace
     {
         // the second half of a pass, from its graph
-        int launch_back(Ctx& c, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os, bool ahead)
+        int launch_back(Ctx& c, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os, bool ahead, bool clear)
         {
             DeviceMesh& m  = c.m();
             DeviceMesh& nm = c.spare();
-            const unsigned long long kind = ahead ? 1ull << 40 : 0ull;
+            const unsigned long long kind = (ahead ? 1ull << 40 : 0ull) | (clear ? 1ull << 41 : 0ull);
             if (fs.size() == 1 && os.empty())
             {
                 DeviceField& f = *fs[0];
                 return run_cached(c, 3 | kind, static_cast<unsigned long long>(c.cur), ptr_key(f.data), ptr_key(f.spare),
-                                  [&]() { return seq_back(c, m, nm, fs, os, ahead); });
+                                  [&]() { return seq_back(c, m, nm, fs, os, ahead, clear); });
             }
             std::vector<DeviceField*> all(fs);
             all.insert(all.end(), os.begin(), os.end());
             return run_cached(c, (7 + 16 * fs.size()) | kind, static_cast<unsigned long long>(c.cur), fields_key(all, false), fields_key(all, true),
-                              [&]() { return seq_back(c, m, nm, fs, os, ahead); });
+                              [&]() { return seq_back(c, m, nm, fs, os, ahead, clear); });
         }
     } // namespace
 
@@ -1494,7 +1499,7 @@ namespace sg
         c.back_ahead = !st && ite == 0;
         if (c.back_ahead)
         {
-            st = launch_back(c, fs, os, true);
+            st = launch_back(c, fs, os, true, false);
         }
         return st;
     }
@@ -1551,7 +1556,7 @@ namespace sg
             return SG_OK;
         }
         *converged = false;
-        if (!back_queued && (st = launch_back(c, fs, os, false)))
+        if (!back_queued && (st = launch_back(c, fs, os, false, c.back_ahead)))
         {
             return st;
         }

@@ -172,7 +172,7 @@ namespace sg
     // non-empty only on a known range of levels; it is computed on that range,
     // and its other levels keep the zeros they were created with (no phase ever
     // writes them).  Operations that read the same inputs share a phase.
-    void build_mesh_phases(Sequence& s)
+    void build_mesh_phases(Sequence& s, bool clear)
     {
         const Geom& g    = s.c.g;
         const int minl   = g.min_level, maxl = g.max_level;
@@ -180,7 +180,10 @@ namespace sg
         const int lmin   = minl >= 2 ? minl - 2 : 0; // lowest level of the reference
         const int h2lo = std::max(minl - 2, 0), h2hi = maxl - 2;
         const int t1lo = std::max(minl - 1, 0), t1hi = maxl - 1;
-        s.add(OP_CLEAR_UNION);
+        if (clear)
+        {
+            s.add(OP_CLEAR_UNION);
+        }
         s.add(OP_HC_CAG, std::min(std::max(minl - 1, 0), minl), maxl);
         if (g.dim == 2)
         {
@@ -240,7 +243,10 @@ namespace sg
                 }
             }
         }
-        s.add(OP_SCAN_SUMS);
+        if (!multi || g.periodic)
+        {
+            s.add(OP_SCAN_SUMS); // otherwise added up by the children's pass
+        }
         s.add(OP_SCAN_WRITE);
     }
 
@@ -248,7 +254,7 @@ namespace sg
     {
         ScopedTimer timer(c, T_CONSTRUCTION);
         Sequence s(c, m, m);
-        build_mesh_phases(s);
+        build_mesh_phases(s, true);
         if (int st = s.done("build_mesh"))
         {
             return st;

@@ -443,6 +443,11 @@ namespace sg
                 const uint32_t c = l > g.min_level ? cells[w] : 0u;
                 return c ? c & E.tc[w] & ~E.tk[w] & ~(l < g.max_level ? E.tr[w] : 0u) : 0u;
             };
+            // the union of the next mesh starts empty
+            for (int w = T.tid; w < static_cast<int>(g.total_words); w += T.nthr)
+            {
+                E.n.uni[w] = 0u;
+            }
             team_words<DIM>(g, T, g.min_level, g.max_level,
                             [&](const Word& p)
                             {
@@ -728,6 +733,49 @@ namespace sg
             {
                 raise(E.flags + F_DIFFER);
             }
+            if (!E.report)
+            {
+                return;
+            }
+            // the last block leaves the flags and the mesh's error word with the host
+            __shared__ bool last;
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0)
+            {
+                last = atomicAdd(E.flags + F_DONE, 1) == T.nblocks - 1;
+            }
+            __syncthreads();
+            if (last && threadIdx.x < F_COUNT)
+            {
+                __threadfence();
+                const int k = static_cast<int>(threadIdx.x);
+                E.report[k] = *static_cast<volatile int*>(k == F_ERR ? E.g.err : E.flags + k);
+            }
+        }
+
+        constexpr int SCAN_CHUNK = SCAN_WORDS;
+
+        struct Pair
+        {
+            unsigned long long pop; // cells: reference in the low, leaves in the high 32 bits
+            unsigned long long nz;  // non-empty words, likewise
+        };
+
+        __device__ __forceinline__ Pair warp_sum(Pair v)
+        {
+            for (int o = 16; o > 0; o >>= 1)
+            {
+                v.pop += __shfl_xor_sync(FULL_MASK, v.pop, o);
+                v.nz += __shfl_xor_sync(FULL_MASK, v.nz, o);
+            }
+            return v;
+        }
+
+        __device__ __forceinline__ Pair word_counts(uint32_t r, uint32_t c)
+        {
+            return {static_cast<unsigned long long>(__popc(r)) | (static_cast<unsigned long long>(__popc(c)) << 32),
+                    static_cast<unsigned long long>(r != 0u) | (static_cast<unsigned long long>(c != 0u) << 32)};
         }
 
         // ---------------------------------------------------------- mesh construction
@@ -749,6 +797,10 @@ namespace sg
             const int minl = g.min_level, maxl = g.max_level;
             const int hlo  = max(minl - 1, 0), hhi = maxl - 1;
             uint32_t* cxy  = DIM == 2 ? E.n.cag : E.t0;
+            for (int k = T.tid; k < 2 * ((static_cast<int>(g.total_words) + SCAN_CHUNK - 1) / SCAN_CHUNK); k += T.nthr)
+            {
+                E.block_sums[k] = 0; // the totals op_ref_children adds up
+            }
             team_words<DIM>(g, T, min(hlo, minl), maxl,
                             [&](const Word& p)
                             {
@@ -956,6 +1008,28 @@ namespace sg
                                 {
                                     E.n.proj[p.w] = v ? v & E.n.uni[p.w] : 0u;
                                 }
+                                // the scan's totals of the word's chunk, a leaf word being a reference word
+                                const unsigned lanes = __activemask();
+                                if (__any_sync(lanes, v != 0u))
+                                {
+                                    const int ch    = p.w / SCAN_CHUNK;
+                                    const Pair t    = word_counts(v, v ? E.n.cells[p.w] : 0u);
+                                    const int first = __ffs(lanes) - 1;
+                                    if (lanes == FULL_MASK && __all_sync(lanes, ch == __shfl_sync(lanes, ch, first)))
+                                    {
+                                        const Pair sum = warp_sum(t);
+                                        if ((threadIdx.x & 31) == 0)
+                                        {
+                                            atomicAdd(reinterpret_cast<unsigned long long*>(E.block_sums) + 2 * ch, sum.pop);
+                                            atomicAdd(reinterpret_cast<unsigned long long*>(E.block_sums) + 2 * ch + 1, sum.nz);
+                                        }
+                                    }
+                                    else if (v)
+                                    {
+                                        atomicAdd(reinterpret_cast<unsigned long long*>(E.block_sums) + 2 * ch, t.pop);
+                                        atomicAdd(reinterpret_cast<unsigned long long*>(E.block_sums) + 2 * ch + 1, t.nz);
+                                    }
+                                }
                             });
         }
 
@@ -1005,30 +1079,6 @@ namespace sg
         // and the counters, in two phases over chunks of SCAN_CHUNK words: the chunks' totals, then each chunk
         // adds up the totals before it and writes its words, 32 consecutive words per warp and step (every load
         // and store coalesced).
-        constexpr int SCAN_CHUNK = SCAN_WORDS;
-
-        struct Pair
-        {
-            unsigned long long pop; // cells: reference in the low, leaves in the high 32 bits
-            unsigned long long nz;  // non-empty words, likewise
-        };
-
-        __device__ __forceinline__ Pair warp_sum(Pair v)
-        {
-            for (int o = 16; o > 0; o >>= 1)
-            {
-                v.pop += __shfl_xor_sync(FULL_MASK, v.pop, o);
-                v.nz += __shfl_xor_sync(FULL_MASK, v.nz, o);
-            }
-            return v;
-        }
-
-        __device__ __forceinline__ Pair word_counts(uint32_t r, uint32_t c)
-        {
-            return {static_cast<unsigned long long>(__popc(r)) | (static_cast<unsigned long long>(__popc(c)) << 32),
-                    static_cast<unsigned long long>(r != 0u) | (static_cast<unsigned long long>(c != 0u) << 32)};
-        }
-
         // the block's sum of v, on every thread
         __device__ __forceinline__ Pair block_sum(Pair v)
         {
@@ -1252,25 +1302,20 @@ namespace sg
         // side 1 those of [-gw, 0) with [n - gw, n); the other axes span
         // [-gw, n + gw).  Only pairs of two reference cells count.  Work item t
         // of the side: gw * (n + 2 gw)^(dim-1) of them.
-        __device__ __forceinline__ bool periodic_pair(const Geom& g, int l, int d, int side, long long t, const uint32_t* ref, Pos* pg, Pos* pi)
+        __device__ __forceinline__ bool periodic_pair(const Geom& g, int l, int d, int side, unsigned t, const uint32_t* ref, Pos* pg, Pos* pi)
         {
-            const int n = g.lv[l].n, gw = g.ghost_width, span = n + 2 * gw;
-            int c[3]    = {0, 0, 0};
-            c[d]        = (side == 0 ? n : -gw) + static_cast<int>(t % gw);
-            long long r = t / gw;
-            for (int k = 0; k < g.dim; ++k)
-            {
-                if (k != d)
-                {
-                    c[k] = -gw + static_cast<int>(r % span);
-                    r /= span;
-                }
-            }
-            int q[3] = {c[0], c[1], c[2]};
-            q[d] += side == 0 ? -n : n;
-            *pg = pos_of(g, l, c[0], c[1], c[2]);
-            *pi = pos_of(g, l, q[0], q[1], q[2]);
-            return test(ref, *pg) && test(ref, *pi);
+            const int n = g.lv[l].n, gw = g.ghost_width; // 1 or 2
+            const int on     = (side == 0 ? n : -gw) + static_cast<int>(gw == 2 ? t & 1u : 0u);
+            const unsigned r = gw == 2 ? t >> 1 : t;
+            const unsigned span = static_cast<unsigned>(n + 2 * gw);
+            const unsigned hi   = g.dim == 3 ? r / span : 0u;
+            const int a = static_cast<int>(r - hi * span) - gw, b = static_cast<int>(hi) - gw; // the other axes, in order
+            const int x = d == 0 ? on : a, y = d == 1 ? on : (d == 0 ? a : b), z = g.dim == 3 ? (d == 2 ? on : b) : 0;
+            const int back = side == 0 ? -n : n;
+            *pg = pos_of(g, l, x, y, z);
+            *pi = pos_of(g, l, x + (d == 0 ? back : 0), y + (d == 1 ? back : 0), z + (d == 2 ? back : 0));
+            const bool rg = test(ref, *pg), ri = test(ref, *pi);
+            return rg && ri;
         }
 
         __host__ __device__ inline long long periodic_side_items(const Geom& g, int l)
@@ -1284,8 +1329,8 @@ namespace sg
         // outer ghosts, so no item reads what another writes)
         __device__ __forceinline__ void op_periodic_copy(const Env& E, int l, int d, const Team& T)
         {
-            const long long per = periodic_side_items(E.g, l);
-            for (long long t = T.tid; t < 2 * per; t += T.nthr)
+            const unsigned per = static_cast<unsigned>(periodic_side_items(E.g, l));
+            for (unsigned t = T.tid; t < 2 * per; t += T.nthr)
             {
                 const int side = t >= per ? 1 : 0;
                 Pos pg, pi;
@@ -1300,14 +1345,16 @@ namespace sg
         }
 
         // update_tag_periodic(level, tag) (algorithm/update_periodic.hpp:178-300)
-        // on one axis and side: both cells of a pair take the union of their tags
-        __device__ __forceinline__ void op_periodic_tag(const Env& E, int l, int d, int side, const Team& T)
+        // on one axis: both cells of a pair take the union of their tags, side after side.  The two sides touch
+        // different cells where the box is at least two ghost widths wide and then run together (sides 3).
+        __device__ __forceinline__ void op_periodic_tag(const Env& E, int l, int d, int sides, const Team& T)
         {
-            const long long per = periodic_side_items(E.g, l);
-            for (long long t = T.tid; t < per; t += T.nthr)
+            const unsigned per = static_cast<unsigned>(periodic_side_items(E.g, l));
+            for (unsigned t = T.tid; t < (sides == 3 ? 2 * per : per); t += T.nthr)
             {
+                const int side = sides == 3 ? (t >= per ? 1 : 0) : sides - 1;
                 Pos pg, pi;
-                if (!periodic_pair(E.g, l, d, side, t, E.m.ref, &pg, &pi))
+                if (!periodic_pair(E.g, l, d, side, t >= per ? t - per : t, E.m.ref, &pg, &pi))
                 {
                     continue;
                 }
@@ -1323,14 +1370,6 @@ namespace sg
                         atomicOr(bm + pg.w, 1u << pg.b);
                     }
                 }
-            }
-        }
-
-        __device__ __forceinline__ void op_report(const Env& E, const Team& T)
-        {
-            if (T.tid < F_COUNT)
-            {
-                E.report[T.tid] = T.tid == F_ERR ? *E.g.err : E.flags[T.tid];
             }
         }
 
@@ -1370,8 +1409,7 @@ namespace sg
             if constexpr (OP == OP_SCAN_WRITE) op_scan_write<DIM>(E);
             if constexpr (OP == OP_UPDATE_FIELDS) op_update_fields<DIM>(E, T);
             if constexpr (OP == OP_PERIODIC_COPY) op_periodic_copy(E, p.l0, p.aux, T);
-            if constexpr (OP == OP_REPORT) op_report(E, T);
-            if constexpr (OP == OP_PERIODIC_TAG) op_periodic_tag(E, p.l0, p.aux >> 1, p.aux & 1, T);
+            if constexpr (OP == OP_PERIODIC_TAG) op_periodic_tag(E, p.l0, p.aux >> 2, p.aux & 3, T);
         }
 
         // graduation phases may hang on a flag of an earlier one (bits 3.. of aux: its slot + 1)
@@ -1418,19 +1456,53 @@ namespace sg
         }
 
         // ---------------------------------------------------------- chain
-        template <int DIM, int OP>
-        __device__ __forceinline__ void run_from(const Env& E, const Phase& p, const Team& T)
+        template <int DIM>
+        __device__ __forceinline__ void run_any(const Env& E, const Phase& p, const Team& T)
         {
-            if constexpr (OP < OP_COUNT)
+            switch (p.op)
             {
-                if (p.op == OP)
-                {
-                    run_op<DIM, OP>(E, p, T);
-                }
-                else
-                {
-                    run_from<DIM, OP + 1>(E, p, T);
-                }
+#define SG_OP(op)                    \
+    case op:                         \
+        run_op<DIM, op>(E, p, T);    \
+        break;
+                SG_OP(OP_PASS_BEGIN)
+                SG_OP(OP_GHOST)
+                SG_OP(OP_PREDICT)
+                SG_OP(OP_ABSMAX_INIT)
+                SG_OP(OP_ABSMAX)
+                SG_OP(OP_DETAIL)
+                SG_OP(OP_CRITERIA)
+                SG_OP(OP_MAXIMUM)
+                SG_OP(OP_NEW_CELLS)
+                SG_OP(OP_GRAD_COARSEN)
+                SG_OP(OP_GRAD_EXPAND)
+                SG_OP(OP_GRAD_EXPAND_XY)
+                SG_OP(OP_GRAD_EXPAND_Z)
+                SG_OP(OP_GRAD_PERIODIC)
+                SG_OP(OP_GRAD_DOWN)
+                SG_OP(OP_GRAD_REFINE)
+                SG_OP(OP_GRAD_APPLY)
+                SG_OP(OP_COMPARE)
+                SG_OP(OP_CLEAR_UNION)
+                SG_OP(OP_HC_CAG)
+                SG_OP(OP_HC2_CAG)
+                SG_OP(OP_CAG_ON)
+                SG_OP(OP_REF0)
+                SG_OP(OP_REF0_XY)
+                SG_OP(OP_REF0_Z)
+                SG_OP(OP_REF_PERIODIC_SRC)
+                SG_OP(OP_REF_PERIODIC)
+                SG_OP(OP_REF_CHILDREN)
+                SG_OP(OP_REF_CHILDREN_LEVEL)
+                SG_OP(OP_PROJ)
+                SG_OP(OP_SINGLE_LEVEL)
+                SG_OP(OP_SCAN_SUMS)
+                SG_OP(OP_SCAN_WRITE)
+                SG_OP(OP_UPDATE_FIELDS)
+                SG_OP(OP_PERIODIC_COPY)
+                SG_OP(OP_PERIODIC_TAG)
+#undef SG_OP
+                default: break;
             }
         }
 
@@ -1469,7 +1541,7 @@ namespace sg
                 {
                     continue; // the same on every thread: the flag was settled before the last barrier
                 }
-                run_from<DIM, 0>(E, p, T);
+                run_any<DIM>(E, p, T);
                 __syncwarp();
                 asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
             }
@@ -1489,7 +1561,7 @@ namespace sg
             "new_cells",      "grad_coarsen", "grad_expand",   "grad_expand_xy", "grad_expand_z", "grad_periodic", "grad_down", "grad_refine",
             "grad_apply",     "compare",      "clear_union",   "hc_cag",       "hc2_cag",      "cag_on",       "ref0",       "ref0_xy",
             "ref0_z",         "ref_periodic_src", "ref_periodic", "ref_children", "ref_children", "proj",      "single_level", "scan_sums",
-            "scan_write",     "update_fields", "periodic_copy", "periodic_tag", "report"};
+            "scan_write",     "update_fields", "periodic_copy", "periodic_tag"};
 
         enum class Shape
         {
@@ -1515,8 +1587,7 @@ namespace sg
                 case OP_SCAN_WRITE: return Shape::SCAN;
                 case OP_ABSMAX_INIT:
                 case OP_PERIODIC_COPY:
-                case OP_PERIODIC_TAG:
-                case OP_REPORT: return Shape::OTHER;
+                case OP_PERIODIC_TAG: return Shape::OTHER;
                 default: return Shape::WORDS;
             }
         }
@@ -1544,8 +1615,7 @@ namespace sg
             case OP_GRAD_DOWN:
             case OP_REF_CHILDREN_LEVEL: return range_words(g, p.l0, p.l0);
             case OP_MAXIMUM: return range_words(g, p.l0 - 1, p.l0 - 1);
-            case OP_ABSMAX_INIT:
-            case OP_REPORT: return 1;
+            case OP_ABSMAX_INIT: return 1;
             default: return g.total_words;
         }
     }
@@ -1604,7 +1674,7 @@ namespace sg
                 break;
             case Shape::SCAN: grid = (g.total_words + SCAN_WORDS - 1) / SCAN_WORDS; break;
             case Shape::OTHER:
-                grid = p.op == OP_ABSMAX_INIT || p.op == OP_REPORT ? 1 : (2 * periodic_side_items(g, p.l0) + block - 1) / block;
+                grid = p.op == OP_ABSMAX_INIT ? 1 : (2 * periodic_side_items(g, p.l0) + block - 1) / block;
                 break;
         }
         if (grid < 1)
@@ -1701,7 +1771,6 @@ namespace sg
         env.det             = c.detail;
         env.capacity        = c.capacity;
         env.setup           = c.d_setup;
-        env.report          = c.h_flags;
         env.absmax          = c.d_absmax;
         env.flags           = c.d_flags;
         env.block_sums      = c.block_sums;
@@ -1726,6 +1795,12 @@ namespace sg
         }
         env.det    = c.detail ? c.detail + static_cast<long long>(first) * c.capacity : nullptr;
         env.absmax = c.d_absmax + first;
+    }
+
+    // the pending phases have no use for it
+    void Sequence::report(int* host)
+    {
+        env.report = host;
     }
 
     void Sequence::guard(const int* flag)

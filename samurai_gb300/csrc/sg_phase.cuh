@@ -59,8 +59,7 @@ namespace sg
         OP_SCAN_WRITE,
         OP_UPDATE_FIELDS,   // from mesh m to mesh n
         OP_PERIODIC_COPY,   // level l0, axis aux
-        OP_PERIODIC_TAG,    // level l0, axis aux >> 1, side aux & 1
-        OP_REPORT,          // flags and error word to the host
+        OP_PERIODIC_TAG,    // level l0, axis aux >> 2, sides aux & 3 (1: upper, 2: lower, 3: both)
         OP_COUNT
     };
 
@@ -105,7 +104,7 @@ namespace sg
         long long capacity;
         PassSetup* setup;
         const PassSetup* setup_host; // pinned: copied into setup when a pass begins (null: setup is in place)
-        int* report;                 // pinned: the flags of a pass, with the mesh's error word at F_ERR
+        int* report;                 // pinned: where OP_COMPARE leaves the flags, with the mesh's error word at F_ERR (or null)
         const int* guard;            // when not null, the phases run only if this flag is set
         unsigned long long* absmax;
         int* flags;
@@ -140,6 +139,7 @@ namespace sg
         Sequence(Ctx& ctx, const DeviceMesh& m, const DeviceMesh& n);
         void fields(const FieldSlot* fs, int first, int nf); // the fields of the following phases: fs[first .. first + nf)
         void add(int op, int l0 = 0, int l1 = 0, int aux = 0);
+        void report(int* host);      // where OP_COMPARE reports
         void guard(const int* flag); // the following phases hang on a device flag
         void flush();                // before anything else is queued on the stream
         void timer_start(int id);
@@ -147,7 +147,7 @@ namespace sg
         int done(const char* what);
     };
 
-    void build_mesh_phases(Sequence& s);                       // mesh construction of mesh n from its cells
+    void build_mesh_phases(Sequence& s, bool clear);           // mesh construction of mesh n from its cells; clear: its union may hold marks
     void grad_pass_phases(Sequence& s, int slot, int guard);   // one graduation pass on mesh n's cells
     MeshPtrs mesh_ptrs(const DeviceMesh& m);
     int launch_phase_alone(Ctx& c, const Env& e, const Phase& p);
