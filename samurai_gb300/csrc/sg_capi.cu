@@ -456,7 +456,8 @@ extern "C"
             return fail(SG_ERR_CUDA, "sg_mesh_create: no CUDA device");
         }
         sg::apply_tuned_launch(c); // the autotuner's choice for this device and level range, unless overridden above
-        c.chain_blocks             = static_cast<int>(std::min<long long>(sg::chain_blocks(dim), tuned("SG_CHAIN_BLOCKS", 16)));
+        c.overlap_levels           = tuned("SG_OVERLAP_LEVELS", 1) != 0;
+        c.chain_blocks             = static_cast<int>(std::min<long long>(sg::chain_blocks(c.g), tuned("SG_CHAIN_BLOCKS", 16)));
         if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess)
         {
             cudaGetLastError();

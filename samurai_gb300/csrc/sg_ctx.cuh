@@ -190,6 +190,7 @@ namespace sg
         unsigned long long mesh_version = 1; // bumped at every change of the current mesh
         long long max_blocks = 152LL * 8; // grid limit of the one-warp-per-word launches, in blocks of 8 warps (x4 for one thread per word)
         int block            = 256;       // threads per block of the FP64 list kernels
+        bool overlap_levels        = true; // levels of the ghost update as programmatic dependents of each other
         int chain_blocks           = 0; // blocks of the cluster that runs a chain of phases (0: no chains)
         long long fuse_words_mesh  = 0; // largest phases that join a chain, in words they walk: mesh and tag phases over all levels,
         long long fuse_words_field = 0; // a level of the ghost update,

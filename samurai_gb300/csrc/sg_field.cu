@@ -112,11 +112,11 @@ namespace sg
                 const int total = static_cast<int>((parts & 1) ? boundary_count<DIM>(g, l) : corner_slots<DIM>(g, l));
                 for (int t = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); t < total; t += nb * static_cast<int>(blockDim.x))
                 {
-                    boundary_item<DIM>(g, l, t, m, u, has_bc != 0, 0., parts);
+                    boundary_item<DIM, false>(g, l, t, m, u, has_bc != 0, 0., parts);
                 }
                 return;
             }
-            project_items(g, l, m, grid_team(nb), 1,
+            project_items<false>(g, l, m, grid_team(nb), 1,
                           [&](long long w, int b, const Cell& c, int) { project_transpose<DIM>(g, u, 32 * w + b, l, c.x, c.y, c.z); });
         }
 
@@ -124,7 +124,7 @@ namespace sg
         __global__ void k_predict_reverse(const __grid_constant__ Geom gp, int l, int order, MeshPtrs m, RevAcc<CAP> u)
         {
             const Geom& g = gp;
-            predict_items(g, l, m, grid_team(), 1,
+            predict_items<false>(g, l, m, grid_team(), 1,
                           [&](long long w, int b, const Cell& c, int) { predict_transpose<DIM>(g, u, 32 * w + b, l, c.x, c.y, c.z, order); });
         }
 

@@ -63,7 +63,7 @@ namespace sg
         // reference's operations touch disjoint cells and read only cells
         // finalised earlier, so they run side by side: corners and faces from
         // item b of nb threads, the projection onto level l-1 from warp0 of nwarps.
-        template <int DIM>
+        template <int DIM, bool PDL>
         __device__ __forceinline__ void ghost_boundary(const Env& E, int l, int b, int nb)
         {
             const int per   = static_cast<int>(boundary_count<DIM>(E.g, l));
@@ -76,14 +76,14 @@ namespace sg
                     k -= per;
                     ++f;
                 }
-                boundary_item<DIM>(E.g, l, k, E.m, ValAcc{E.f[f].u}, E.f[f].has_bc != 0, E.f[f].bcv, 3);
+                boundary_item<DIM, PDL>(E.g, l, k, E.m, ValAcc{E.f[f].u}, E.f[f].has_bc != 0, E.f[f].bcv, 3);
             }
         }
 
-        template <int DIM>
+        template <int DIM, bool PDL>
         __device__ __forceinline__ void ghost_project(const Env& E, int l, const Team& T)
         {
-            project_items(E.g, l, E.m, T, E.nf,
+            project_items<PDL>(E.g, l, E.m, T, E.nf,
                           [&](long long w, int b, const Cell& c, int f)
                           {
                               double* u     = E.f[f].u;
@@ -101,17 +101,17 @@ namespace sg
         __device__ __forceinline__ void op_ghost(const Env& E, int l, const Team& T)
         {
             const int back = T.nblocks - 1 - T.block; // whole warps stay together
-            ghost_boundary<DIM>(E, l, back * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x), T.nthr);
+            ghost_boundary<DIM, false>(E, l, back * static_cast<int>(blockDim.x) + static_cast<int>(threadIdx.x), T.nthr);
             if (l > lowest_level(E.g))
             {
-                ghost_project<DIM>(E, l, T);
+                ghost_project<DIM, false>(E, l, T);
             }
         }
 
-        template <int DIM>
+        template <int DIM, bool PDL>
         __device__ __forceinline__ void op_predict(const Env& E, int l, const Team& T)
         {
-            predict_items(E.g, l, E.m, T, E.nf,
+            predict_items<PDL>(E.g, l, E.m, T, E.nf,
                           [&](long long w, int b, const Cell& c, int f)
                           {
                               double* u     = E.f[f].u;
@@ -1058,12 +1058,6 @@ namespace sg
                             });
         }
 
-        template <int DIM>
-        __device__ __forceinline__ void op_proj(const Env& E, int l0, int l1, const Team& T)
-        {
-            team_words<DIM>(E.g, T, l0, l1, [&](const Word& p) { E.n.proj[p.w] = E.n.ref[p.w] & E.n.uni[p.w]; });
-        }
-
         // a mesh of one level: no coarser reference, no projection
         __device__ __forceinline__ void op_single_level(const Env& E, const Team& T)
         {
@@ -1374,13 +1368,13 @@ namespace sg
         }
 
         // ---------------------------------------------------------- dispatch
-        template <int DIM, int OP>
+        template <int DIM, int OP, bool PDL>
         __device__ __forceinline__ void run_op(const Env& E, const Phase& p, const Team& T)
         {
             const int slot = p.aux & 7;
             if constexpr (OP == OP_PASS_BEGIN) op_pass_begin(E, T);
             if constexpr (OP == OP_GHOST) op_ghost<DIM>(E, p.l0, T);
-            if constexpr (OP == OP_PREDICT) op_predict<DIM>(E, p.l0, T);
+            if constexpr (OP == OP_PREDICT) op_predict<DIM, PDL>(E, p.l0, T);
             if constexpr (OP == OP_ABSMAX_INIT) op_absmax_init(E, T);
             if constexpr (OP == OP_ABSMAX) op_absmax(E, T);
             if constexpr (OP == OP_DETAIL) op_detail<DIM>(E, p.l0, p.l1, T);
@@ -1403,7 +1397,6 @@ namespace sg
             if constexpr (OP == OP_REF_PERIODIC) op_ref_periodic<DIM>(E, T);
             if constexpr (OP == OP_REF_CHILDREN) op_ref_children<DIM>(E, p.l0, p.l1, T);
             if constexpr (OP == OP_REF_CHILDREN_LEVEL) op_ref_children_level<DIM>(E, p.l0, T);
-            if constexpr (OP == OP_PROJ) op_proj<DIM>(E, p.l0, p.l1, T);
             if constexpr (OP == OP_SINGLE_LEVEL) op_single_level(E, T);
             if constexpr (OP == OP_SCAN_SUMS) op_scan_sums(E);
             if constexpr (OP == OP_SCAN_WRITE) op_scan_write<DIM>(E);
@@ -1430,40 +1423,90 @@ namespace sg
             {
                 return;
             }
+            if constexpr (OP == OP_GHOST || OP == OP_PREDICT)
+            {
+                // the next level's launch may come in as soon as every block of this one has a place
+                asm volatile("griddepcontrol.launch_dependents;");
+            }
             if constexpr (OP == OP_GHOST)
             {
                 // the first l1 blocks take the boundary, the others the projection
                 const int nb = p.l1;
                 if (static_cast<int>(blockIdx.x) < nb)
                 {
-                    ghost_boundary<DIM>(E, p.l0, static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x), nb * static_cast<int>(blockDim.x));
+                    ghost_boundary<DIM, true>(E, p.l0, static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x), nb * static_cast<int>(blockDim.x));
                 }
                 else
                 {
-                    ghost_project<DIM>(E, p.l0, grid_team(nb));
+                    ghost_project<DIM, true>(E, p.l0, grid_team(nb));
                 }
             }
             else
             {
-                run_op<DIM, OP>(E, p, grid_team());
+                run_op<DIM, OP, true>(E, p, grid_team());
+            }
+            if constexpr (OP == OP_GHOST || OP == OP_PREDICT)
+            {
+                dependency_wait<true>(); // a block without items must not end before the launch it follows
             }
         }
 
+        // Levels of the ghost update follow each other as programmatic dependents: a level's launch loads its bitmap
+        // words and hands out its items (nothing of that changes during the ghost update) while the level before
+        // still runs, and waits for it just before the first value.
         template <int DIM, int OP>
         void launch_one(Ctx& c, const Env& e, const Phase& p, int grid, int block)
         {
+            if constexpr (OP == OP_GHOST || OP == OP_PREDICT)
+            {
+                if (c.overlap_levels && c.cap_depth == 0 && !c.trace.enabled)
+                {
+                    cudaLaunchConfig_t cfg{};
+                    cfg.gridDim  = dim3(static_cast<unsigned>(grid));
+                    cfg.blockDim = dim3(static_cast<unsigned>(block));
+                    cfg.stream   = c.stream;
+                    cudaLaunchAttribute at{};
+                    at.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+                    at.val.programmaticStreamSerializationAllowed = 1;
+                    cfg.attrs                                     = &at;
+                    cfg.numAttrs                                  = 1;
+                    cudaLaunchKernelEx(&cfg, k_phase<DIM, OP>, e, p);
+                    return;
+                }
+            }
             k_phase<DIM, OP><<<grid, block, 0, c.stream>>>(e, p);
         }
 
         // ---------------------------------------------------------- chain
-        template <int DIM>
+        // PERIODIC: the phases of meshes with periodic axes too (a chain fetches its instructions as it goes: the
+        // other meshes' kernel leaves them out)
+        template <int DIM, bool PERIODIC>
         __device__ __forceinline__ void run_any(const Env& E, const Phase& p, const Team& T)
         {
+            if constexpr (PERIODIC)
+            {
+                switch (p.op)
+                {
+#define SG_OP(op)                        \
+    case op:                             \
+        run_op<DIM, op, false>(E, p, T); \
+        return;
+                    SG_OP(OP_GRAD_PERIODIC)
+                    SG_OP(OP_GRAD_DOWN)
+                    SG_OP(OP_REF_PERIODIC_SRC)
+                    SG_OP(OP_REF_PERIODIC)
+                    SG_OP(OP_REF_CHILDREN_LEVEL)
+                    SG_OP(OP_PERIODIC_COPY)
+                    SG_OP(OP_PERIODIC_TAG)
+#undef SG_OP
+                    default: break;
+                }
+            }
             switch (p.op)
             {
 #define SG_OP(op)                    \
     case op:                         \
-        run_op<DIM, op>(E, p, T);    \
+        run_op<DIM, op, false>(E, p, T); \
         break;
                 SG_OP(OP_PASS_BEGIN)
                 SG_OP(OP_GHOST)
@@ -1478,8 +1521,6 @@ namespace sg
                 SG_OP(OP_GRAD_EXPAND)
                 SG_OP(OP_GRAD_EXPAND_XY)
                 SG_OP(OP_GRAD_EXPAND_Z)
-                SG_OP(OP_GRAD_PERIODIC)
-                SG_OP(OP_GRAD_DOWN)
                 SG_OP(OP_GRAD_REFINE)
                 SG_OP(OP_GRAD_APPLY)
                 SG_OP(OP_COMPARE)
@@ -1490,17 +1531,11 @@ namespace sg
                 SG_OP(OP_REF0)
                 SG_OP(OP_REF0_XY)
                 SG_OP(OP_REF0_Z)
-                SG_OP(OP_REF_PERIODIC_SRC)
-                SG_OP(OP_REF_PERIODIC)
                 SG_OP(OP_REF_CHILDREN)
-                SG_OP(OP_REF_CHILDREN_LEVEL)
-                SG_OP(OP_PROJ)
                 SG_OP(OP_SINGLE_LEVEL)
                 SG_OP(OP_SCAN_SUMS)
                 SG_OP(OP_SCAN_WRITE)
                 SG_OP(OP_UPDATE_FIELDS)
-                SG_OP(OP_PERIODIC_COPY)
-                SG_OP(OP_PERIODIC_TAG)
 #undef SG_OP
                 default: break;
             }
@@ -1513,8 +1548,15 @@ namespace sg
         // mesh of 8 levels (device time, warm), of which 0.9 us is the boundary
         // between two nodes and most of the rest launch, cold instructions and
         // ramp-up; a cluster barrier takes 0.25 us (16 blocks of 512 threads),
-        // a barrier over the whole grid 1.3 us.
-        template <int DIM>
+        // a barrier over the whole grid 1.3 us.  A cluster barrier that has to
+        // wait for the blocks' stores takes 0.8 us, though, and every load after it
+        // comes from L2 (0.2 us).  With periodic axes the exchanges between the
+        // levels double the phases, most of them nearly empty: there the phases of
+        // the smallest levels run in the first block alone, block barriers between
+        // them, and only the end of such a run is a cluster barrier (2D levels 3 to
+        // 9: 566 -> 522 us a step; without periodic axes the lone block loses what
+        // the barriers save).
+        template <int DIM, bool PERIODIC>
         __global__ void __launch_bounds__(CHAIN_THREADS, 1) k_chain(const __grid_constant__ Env Ep, const __grid_constant__ PhaseList L)
         {
             // the environment is read at every step of every phase: from shared memory, not from parameter
@@ -1533,15 +1575,32 @@ namespace sg
             {
                 return; // the whole cluster: the flag was settled before the launch
             }
-            const Team T = grid_team();
+            const Team all  = grid_team();
+            const Team solo = {static_cast<int>(threadIdx.x), static_cast<int>(blockDim.x), 0, 1};
             for (int i = 0; i < L.n; ++i)
             {
-                const Phase p = L.p[i];
+                Phase p          = L.p[i];
+                const bool alone = PERIODIC && (p.op & PHASE_SOLO) != 0;
+                if (PERIODIC)
+                {
+                    p.op &= static_cast<short>(~PHASE_SOLO);
+                }
                 if (guarded_off(E, p))
                 {
                     continue; // the same on every thread: the flag was settled before the last barrier
                 }
-                run_any<DIM>(E, p, T);
+                if (!alone || blockIdx.x == 0)
+                {
+                    run_any<DIM, PERIODIC>(E, p, alone ? solo : all);
+                }
+                if (alone)
+                {
+                    __syncthreads();
+                    if (i + 1 < L.n && (L.p[i + 1].op & PHASE_SOLO) != 0)
+                    {
+                        continue; // the other blocks wait at the end of the run
+                    }
+                }
                 __syncwarp();
                 asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
             }
@@ -1560,7 +1619,7 @@ namespace sg
             "pass_begin",     "ghost_level",  "predict",       "absmax_init",  "absmax",       "detail",       "criteria",   "maximum",
             "new_cells",      "grad_coarsen", "grad_expand",   "grad_expand_xy", "grad_expand_z", "grad_periodic", "grad_down", "grad_refine",
             "grad_apply",     "compare",      "clear_union",   "hc_cag",       "hc2_cag",      "cag_on",       "ref0",       "ref0_xy",
-            "ref0_z",         "ref_periodic_src", "ref_periodic", "ref_children", "ref_children", "proj",      "single_level", "scan_sums",
+            "ref0_z",         "ref_periodic_src", "ref_periodic", "ref_children", "ref_children", "single_level", "scan_sums",
             "scan_write",     "update_fields", "periodic_copy", "periodic_tag"};
 
         enum class Shape
@@ -1688,11 +1747,19 @@ namespace sg
         return check(c, phase_name(p.op));
     }
 
+    namespace
+    {
+        auto chain_kernel(const Geom& g)
+        {
+            return g.dim == 2 ? (g.periodic ? k_chain<2, true> : k_chain<2, false>) : (g.periodic ? k_chain<3, true> : k_chain<3, false>);
+        }
+    } // namespace
+
     // The largest cluster a chain may use on this device: 16 blocks where the
     // device grants that (above the portable 8), 0 where it grants none.
-    int chain_blocks(int dim)
+    int chain_blocks(const Geom& g)
     {
-        const void* k = dim == 2 ? reinterpret_cast<const void*>(k_chain<2>) : reinterpret_cast<const void*>(k_chain<3>);
+        const void* k = reinterpret_cast<const void*>(chain_kernel(g));
         const bool big = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
         for (int n = big ? 16 : 8; n >= 2; n /= 2)
         {
@@ -1732,7 +1799,7 @@ namespace sg
             at.val.clusterDim.y = at.val.clusterDim.z = 1;
             cfg.attrs    = &at;
             cfg.numAttrs = 1;
-            const cudaError_t err = c.g.dim == 2 ? cudaLaunchKernelEx(&cfg, k_chain<2>, e, list) : cudaLaunchKernelEx(&cfg, k_chain<3>, e, list);
+            const cudaError_t err = cudaLaunchKernelEx(&cfg, chain_kernel(c.g), e, list);
             if (err != cudaSuccess)
             {
                 cudaGetLastError();
@@ -1842,6 +1909,22 @@ namespace sg
         if (c.chain_blocks > 0 && !c.trace.enabled && words <= limit)
         {
             chain.push_back(p);
+            switch (op)
+            {
+                case OP_GHOST:
+                case OP_PREDICT:
+                case OP_MAXIMUM:
+                case OP_PERIODIC_COPY:
+                case OP_PERIODIC_TAG:
+                case OP_GRAD_DOWN:
+                case OP_REF_CHILDREN_LEVEL:
+                    if (c.g.periodic && words <= (c.g.dim == 2 ? SOLO_WORDS_2D : SOLO_WORDS_3D))
+                    {
+                        chain.back().op |= PHASE_SOLO;
+                    }
+                    break;
+                default: break;
+            }
             if (chain.size() == CHAIN_MAX)
             {
                 flush();
@@ -1859,7 +1942,15 @@ namespace sg
     {
         if (!status && !chain.empty())
         {
-            status = chain.size() == 1 ? launch_phase_alone(c, env, chain[0]) : launch_chain(c, env, chain);
+            if (chain.size() == 1)
+            {
+                chain[0].op &= static_cast<short>(~PHASE_SOLO);
+                status = launch_phase_alone(c, env, chain[0]);
+            }
+            else
+            {
+                status = launch_chain(c, env, chain);
+            }
         }
         chain.clear();
     }

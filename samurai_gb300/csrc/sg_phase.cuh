@@ -53,7 +53,6 @@ namespace sg
         OP_REF_PERIODIC,
         OP_REF_CHILDREN,    // levels l0..l1
         OP_REF_CHILDREN_LEVEL, // level l0
-        OP_PROJ,            // levels l0..l1
         OP_SINGLE_LEVEL,
         OP_SCAN_SUMS,
         OP_SCAN_WRITE,
@@ -121,6 +120,12 @@ namespace sg
     constexpr int CHAIN_MAX     = 96;  // phases of one chain
     constexpr int CHAIN_THREADS = 512; // threads per block of a chain
 
+    constexpr short PHASE_SOLO  = 0x100; // bit of op: the phase runs in the chain's first block alone
+    // Levels whose phases do: a word per thread in 2D (levels up to 6: a few hundred cells, nine additions of 66
+    // cycles each for a predicted ghost); 3D levels up to 2, whose padded rows are mostly empty.
+    constexpr long long SOLO_WORDS_2D = 512;
+    constexpr long long SOLO_WORDS_3D = 1300;
+
     struct PhaseList
     {
         int n;
@@ -151,7 +156,7 @@ namespace sg
     void grad_pass_phases(Sequence& s, int slot, int guard);   // one graduation pass on mesh n's cells
     MeshPtrs mesh_ptrs(const DeviceMesh& m);
     int launch_phase_alone(Ctx& c, const Env& e, const Phase& p);
-    int chain_blocks(int dim);
+    int chain_blocks(const Geom& g);
     long long phase_words(const Geom& g, const Phase& p);
     const char* phase_name(int op);
 } // namespace sg

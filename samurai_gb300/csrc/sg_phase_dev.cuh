@@ -260,6 +260,17 @@ namespace sg
         return s;
     }
 
+    // Everything the launch this one depends on has written is visible after it (nothing to wait for in a launch
+    // without the programmatic attribute).  PDL: the code runs in such a launch.
+    template <bool PDL>
+    __device__ __forceinline__ void dependency_wait()
+    {
+        if constexpr (PDL)
+        {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        }
+    }
+
     // position of set bit number r (from 0) of m
     __device__ __forceinline__ int nth_bit(uint32_t m, int r)
     {
@@ -635,7 +646,7 @@ namespace sg
     // (bc/dirichlet.hpp:22-29) of a leaf and predict_bc to level l+1
     // (update_outer_ghost.hpp:195-266), or project_bc
     // (update_outer_ghost.hpp:20-155) next to a union cell.
-    template <int DIM, class A>
+    template <int DIM, bool PDL, class A>
     __device__ __forceinline__ void face_item(const Geom& g, const FaceArgs& a, long long t, const uint32_t* cells, const uint32_t* uni,
                                               const uint32_t* ref, const A& u, double value)
     {
@@ -664,12 +675,13 @@ namespace sg
         const Pos pg       = pos_of(g, l, gx, gy, gz);
         const uint32_t wg  = ref[pg.w];
         const long long eg = elem(pg);
-        const typename A::V ui = u.get(elem(pi));
         Children<DIM, 2> c2;
         if (l + 1 < g.nlev)
         {
             c2.load(g, l + 1, gx, gy, gz, ref);
         }
+        dependency_wait<PDL>();
+        const typename A::V ui = u.get(elem(pi));
         if ((a.do_dirichlet || a.do_predict) && ((wc >> pi.b) & 1u))
         {
             typename A::V v;
@@ -739,7 +751,7 @@ namespace sg
     // off-diagonal copies).  The coarse corner ghost one or two levels below takes the value of the fine one at
     // the first of its positions along the edge, the position of the thread that owns the fine one.
     // parts: 1 the corners, 2 their projection below, 3 both.
-    template <int DIM, class A>
+    template <int DIM, bool PDL, class A>
     __device__ __forceinline__ void corner_item(const Geom& g, int l, long long t, const uint32_t* cells, const uint32_t* ref, const A& u, int parts)
     {
         const int n = g.lv[l].n;
@@ -791,6 +803,7 @@ namespace sg
             }
         }
         const bool leaf       = (parts & 1) && test(cells, pc);
+        dependency_wait<PDL>();
         const typename A::V v = leaf ? u.get(elem(pc)) : u.get(eg);
         if (leaf)
         {
@@ -851,7 +864,7 @@ namespace sg
     // The items of the set bm on level l.  Every word of the level is looked at
     // when the team has a thread for it (one load to the bits); larger levels go
     // through the list of reference words.
-    template <class ItemF>
+    template <bool PDL, class ItemF>
     __device__ __forceinline__ void level_items(const Geom& g, int l, const MeshPtrs& m, const uint32_t* bm, const Team& T, int nf, ItemF item)
     {
         const LevelGeom& L = g.lv[l];
@@ -861,6 +874,7 @@ namespace sg
                     dense ? first + static_cast<int>(L.nwords) : static_cast<int>(m.lo[LO_REF + l + 1]), T, nf, [&](int w) { return bm[w]; },
                     [&](bool valid, int w, int b, int f)
                     {
+                        dependency_wait<PDL>(); // up to here nothing but the mesh's bitmaps was read
                         if (valid)
                         {
                             item(static_cast<long long>(w), b, cell_of(g, l, w, b), f);
@@ -871,18 +885,18 @@ namespace sg
     // projection of the reference cells of level l onto proj_cells[l-1]
     // (numeric/projection.hpp:15-65); the children of a projection cell are
     // reference cells by construction.  item(word, bit, cell, field)
-    template <class ItemF>
+    template <bool PDL, class ItemF>
     __device__ __forceinline__ void project_items(const Geom& g, int l, const MeshPtrs& m, const Team& T, int nf, ItemF item)
     {
-        level_items(g, l - 1, m, m.proj, T, nf, item);
+        level_items<PDL>(g, l - 1, m, m.proj, T, nf, item);
     }
 
     // prediction of the ghosts of level l from level l-1
     // (algorithm/update_ghost_mr.hpp:224-233)
-    template <class ItemF>
+    template <bool PDL, class ItemF>
     __device__ __forceinline__ void predict_items(const Geom& g, int l, const MeshPtrs& m, const Team& T, int nf, ItemF item)
     {
-        level_items(g, l, m, m.pred, T, nf, item);
+        level_items<PDL>(g, l, m, m.pred, T, nf, item);
     }
 
     // Boundary positions of level l: corners first, padded to whole warps (corner
@@ -901,7 +915,7 @@ namespace sg
     }
 
     // boundary position t of level l on accessor u
-    template <int DIM, class A>
+    template <int DIM, bool PDL, class A>
     __device__ __forceinline__ void boundary_item(const Geom& g, int l, long long t, const MeshPtrs& m, const A& u, bool has_bc, double value, int corner_parts)
     {
         const long long nc = corner_slots<DIM>(g, l);
@@ -909,13 +923,13 @@ namespace sg
         {
             if (t < corner_count<DIM>(g, l))
             {
-                corner_item<DIM>(g, l, t, m.cells, m.ref, u, corner_parts);
+                corner_item<DIM, PDL>(g, l, t, m.cells, m.ref, u, corner_parts);
             }
         }
         else
         {
             const FaceArgs a{l, l < g.max_level, l >= g.min_level && has_bc, l >= g.min_level && l < g.max_level};
-            face_item<DIM>(g, a, t - nc, m.cells, m.uni, m.ref, u, value);
+            face_item<DIM, PDL>(g, a, t - nc, m.cells, m.uni, m.ref, u, value);
         }
     }
 } // namespace sg
