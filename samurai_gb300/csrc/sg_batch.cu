@@ -391,7 +391,7 @@ extern "C"
             sg::Ctx& c = u[k]->mesh->ctx;
             b->saved_fuse.insert(b->saved_fuse.end(), {c.fuse_words_mesh, c.fuse_words_field, c.fuse_words_max, c.chain_blocks});
             b->saved_blocks.push_back(c.block);
-            c.chain_blocks = std::min(c.chain_blocks, sg::BATCH_CHAIN_BLOCKS);
+            c.chain_blocks = std::min(c.chain_blocks, sg::batch_chain_blocks(n));
             sg::set_fusion(c, sg::BATCH_FUSE_WORDS, sg::BATCH_FUSE_WORDS, sg::BATCH_FUSE_WORDS);
         }
         b->n_threads = std::min(n_threads, n);

@@ -487,7 +487,7 @@ extern "C"
         }
         st |= dalloc(c, &c.detail, static_cast<size_t>(c.capacity));
         c.n_scan_blocks = (c.g.total_words + 4095) / 4096;
-        st |= dalloc(c, &c.block_sums, 4 * static_cast<size_t>(c.n_scan_blocks) + 4);
+        st |= dalloc(c, &c.block_sums, 5 * static_cast<size_t>(c.n_scan_blocks) + 8); // pairs per 2048 words and per 64 of those
         st |= dalloc(c, &c.d_counts, static_cast<size_t>(sg::COUNTS));
         st |= dalloc(c, &c.d_flags, 8);
         st |= dalloc(c, &c.d_adapt, static_cast<size_t>(sg::A_COUNT));

@@ -618,9 +618,31 @@ namespace sg
                       });
         }
 
-        __global__ void k_fill(const int* wl, const long long* lo, int nlev, const uint32_t* ref, double* dense, double v)
+        __global__ void k_fill(const int* __restrict__ wl, const long long* __restrict__ lo, int nlev, const uint32_t* __restrict__ ref, double* dense,
+                               double v)
         {
-            warp_list(wl, lo[LO_REF], lo[LO_REF + nlev], warp_id(), warp_count(), [&](long long w) { return ref[w]; }, [&](long long w, int b) { dense[32 * w + b] = v; });
+            const int lane  = threadIdx.x & 31;
+            const int begin = static_cast<int>(lo[LO_REF]), end = static_cast<int>(lo[LO_REF + nlev]);
+            for (int c0 = begin + static_cast<int>(warp_id()) * MOVE_WORDS; c0 < end; c0 += static_cast<int>(warp_count()) * MOVE_WORDS)
+            {
+                int w      = 0;
+                uint32_t m = 0u;
+                if (lane < MOVE_WORDS && c0 + lane < end)
+                {
+                    w = wl[c0 + lane];
+                    m = ref[w];
+                }
+#pragma unroll
+                for (int k = 0; k < MOVE_WORDS; ++k)
+                {
+                    const long long e   = 32LL * __shfl_sync(FULL_MASK, w, k) + lane;
+                    const uint32_t bits = __shfl_sync(FULL_MASK, m, k);
+                    if ((bits >> lane) & 1u)
+                    {
+                        dense[e] = v;
+                    }
+                }
+            }
         }
     } // namespace
 
