@@ -389,9 +389,12 @@ extern "C"
         for (int k = 0; k < n; ++k)
         {
             sg::Ctx& c = u[k]->mesh->ctx;
-            b->saved_fuse.insert(b->saved_fuse.end(), {c.fuse_words_mesh, c.fuse_words_field, c.fuse_words_max, c.chain_blocks});
+            b->saved_fuse.insert(b->saved_fuse.end(), {c.fuse_words_mesh, c.fuse_words_field, c.fuse_words_max, c.chain_blocks, c.overlap_launches ? 1 : 0});
             b->saved_blocks.push_back(c.block);
             c.chain_blocks = std::min(c.chain_blocks, sg::batch_chain_blocks(n));
+            // waiting blocks of one instance's next launch would hold places that the others' running ones want
+            // (48 instances: 1993 us a step without overlap, 2402 with it)
+            c.overlap_launches = c.overlap_launches && n < 4;
             sg::set_fusion(c, sg::BATCH_FUSE_WORDS, sg::BATCH_FUSE_WORDS, sg::BATCH_FUSE_WORDS);
         }
         b->n_threads = std::min(n_threads, n);
@@ -416,8 +419,10 @@ extern "C"
             {
                 sg::Ctx& c = b->u[k]->mesh->ctx;
                 c.block    = b->saved_blocks[k];
-                c.chain_blocks = static_cast<int>(b->saved_fuse[4 * k + 3]);
-                sg::set_fusion(c, b->saved_fuse[4 * k], b->saved_fuse[4 * k + 1], b->saved_fuse[4 * k + 2]);
+                const long long* own = b->saved_fuse.data() + 5 * k;
+                c.chain_blocks       = static_cast<int>(own[3]);
+                c.overlap_launches   = own[4] != 0;
+                sg::set_fusion(c, own[0], own[1], own[2]);
             }
         }
         delete b;

@@ -441,7 +441,7 @@ extern "C"
         }
         c.capacity                 = 32 * c.g.total_words;
         c.fuse_words_mesh          = tuned("SG_FUSE_WORDS", sg::FUSE_WORDS);
-        c.fuse_words_field         = tuned("SG_FUSE_WORDS_FIELD", sg::FUSE_WORDS_FIELD);
+        c.fuse_words_field         = tuned("SG_FUSE_WORDS_FIELD", c.g.periodic ? sg::FUSE_WORDS_FIELD : 0);
         c.fuse_words_max           = tuned("SG_FUSE_WORDS_MAX", sg::FUSE_WORDS_MAX);
         c.max_blocks               = std::max(1LL, tuned("SG_MAX_BLOCKS", c.max_blocks));
         c.block                    = static_cast<int>(std::min(1024LL, std::max(32LL, tuned("SG_BLOCK", c.block))) / 32 * 32);
@@ -456,7 +456,7 @@ extern "C"
             return fail(SG_ERR_CUDA, "sg_mesh_create: no CUDA device");
         }
         sg::apply_tuned_launch(c); // the autotuner's choice for this device and level range, unless overridden above
-        c.overlap_levels           = tuned("SG_OVERLAP_LEVELS", 1) != 0;
+        c.overlap_launches         = tuned("SG_OVERLAP_LAUNCHES", 1) != 0;
         c.chain_blocks             = static_cast<int>(std::min<long long>(sg::chain_blocks(c.g), tuned("SG_CHAIN_BLOCKS", 16)));
         if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess)
         {

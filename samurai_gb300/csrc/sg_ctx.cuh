@@ -190,7 +190,7 @@ namespace sg
         unsigned long long mesh_version = 1; // bumped at every change of the current mesh
         long long max_blocks = 152LL * 8; // grid limit of the one-warp-per-word launches, in blocks of 8 warps (x4 for one thread per word)
         int block            = 256;       // threads per block of the FP64 list kernels
-        bool overlap_levels        = true; // levels of the ghost update as programmatic dependents of each other
+        bool overlap_launches      = true; // phases as programmatic dependents of each other
         int chain_blocks           = 0; // blocks of the cluster that runs a chain of phases (0: no chains)
         long long fuse_words_mesh  = 0; // largest phases that join a chain, in words they walk: mesh and tag phases over all levels,
         long long fuse_words_field = 0; // a level of the ghost update,
@@ -298,7 +298,7 @@ namespace sg
 
     // Limits of the phases that join a chain (sg_phase.cuh), in words
     constexpr long long FUSE_WORDS       = 16384;
-    constexpr long long FUSE_WORDS_FIELD = 5000;
+    constexpr long long FUSE_WORDS_FIELD = 5000; // with periodic axes; 0 otherwise (2D levels 2 to 8: 220 us a step against 255)
     constexpr long long FUSE_WORDS_MAX   = 12288;
     constexpr long long BATCH_FUSE_WORDS = 10000;
     // Smaller clusters in batched mode, where many meshes share the chip: 48 meshes of max_level 7..10 take

@@ -1438,14 +1438,31 @@ namespace sg
         template <int DIM, int OP>
         __global__ void k_phase(const __grid_constant__ Env E, const __grid_constant__ Phase p)
         {
-            if ((OP >= OP_GRAD_COARSEN && OP <= OP_GRAD_APPLY && guarded_off(E, p)) || (E.guard && *E.guard == 0))
+            // Launches are programmatic dependents of each other: the next one's blocks come in while this one runs and
+            // wait for its end.  A level of the ghost update that follows another (FOLLOWS) goes further: it reads
+            // nothing but the mesh's bitmaps until its items are handed out, and waits just before the first value.
+            // It may also let its successor in before its own wait, since a first level has waited for whatever
+            // wrote the bitmaps before it let anyone in.
+            constexpr bool LEVEL = OP == OP_GHOST || OP == OP_PREDICT;
+            if (!LEVEL || !(p.aux & FOLLOWS))
+            {
+                dependency_wait<true>();
+            }
+            asm volatile("griddepcontrol.launch_dependents;");
+            if ((OP >= OP_GRAD_COARSEN && OP <= OP_GRAD_APPLY && guarded_off(E, p)))
             {
                 return;
             }
-            if constexpr (OP == OP_GHOST || OP == OP_PREDICT)
+            if (E.guard)
             {
-                // the next level's launch may come in as soon as every block of this one has a place
-                asm volatile("griddepcontrol.launch_dependents;");
+                if (LEVEL)
+                {
+                    dependency_wait<true>(); // the flag may be older than the bitmaps, but never let a block end unwaited
+                }
+                if (*E.guard == 0)
+                {
+                    return;
+                }
             }
             if constexpr (OP == OP_GHOST)
             {
@@ -1470,30 +1487,40 @@ namespace sg
             }
         }
 
-        // Levels of the ghost update follow each other as programmatic dependents: a level's launch loads its bitmap
-        // words and hands out its items (nothing of that changes during the ghost update) while the level before
-        // still runs, and waits for it just before the first value.
+        template <class... Params, class... Args>
+        void launch_dependent(Ctx& c, bool overlap, void (*kernel)(Params...), int grid, int block, int cluster, Args&&... args)
+        {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim  = dim3(static_cast<unsigned>(grid));
+            cfg.blockDim = dim3(static_cast<unsigned>(block));
+            cfg.stream   = c.stream;
+            cudaLaunchAttribute at[2] = {};
+            if (cluster > 1)
+            {
+                at[cfg.numAttrs].id               = cudaLaunchAttributeClusterDimension;
+                at[cfg.numAttrs].val.clusterDim.x = static_cast<unsigned>(cluster);
+                at[cfg.numAttrs].val.clusterDim.y = at[cfg.numAttrs].val.clusterDim.z = 1;
+                ++cfg.numAttrs;
+            }
+            // not inside conditional bodies, nor where the kernel trace puts an event after every launch
+            if (overlap && c.overlap_launches && c.cap_depth == 0 && !c.trace.enabled)
+            {
+                at[cfg.numAttrs].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+                at[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+                ++cfg.numAttrs;
+            }
+            cfg.attrs = at;
+            cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...); // the caller checks the last error
+        }
+
         template <int DIM, int OP>
         void launch_one(Ctx& c, const Env& e, const Phase& p, int grid, int block)
         {
-            if constexpr (OP == OP_GHOST || OP == OP_PREDICT)
-            {
-                if (c.overlap_levels && c.cap_depth == 0 && !c.trace.enabled)
-                {
-                    cudaLaunchConfig_t cfg{};
-                    cfg.gridDim  = dim3(static_cast<unsigned>(grid));
-                    cfg.blockDim = dim3(static_cast<unsigned>(block));
-                    cfg.stream   = c.stream;
-                    cudaLaunchAttribute at{};
-                    at.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
-                    at.val.programmaticStreamSerializationAllowed = 1;
-                    cfg.attrs                                     = &at;
-                    cfg.numAttrs                                  = 1;
-                    cudaLaunchKernelEx(&cfg, k_phase<DIM, OP>, e, p);
-                    return;
-                }
-            }
-            k_phase<DIM, OP><<<grid, block, 0, c.stream>>>(e, p);
+            // The field phases over all levels stay behind a full boundary: their waiting blocks would hold the
+            // shared memory and registers that the launch before them still wants (three components, 2D levels 3
+            // to 9, relative details: 303 us a step without them, 375 with them overlapped too).
+            constexpr bool overlap = OP != OP_DETAIL && OP != OP_UPDATE_FIELDS && OP != OP_ABSMAX && OP != OP_ABSMAX_INIT;
+            launch_dependent(c, overlap, k_phase<DIM, OP>, grid, block, 1, e, p);
         }
 
         // ---------------------------------------------------------- chain
@@ -1567,7 +1594,9 @@ namespace sg
         // mesh of 8 levels (device time, warm), of which 0.9 us is the boundary
         // between two nodes and most of the rest launch, cold instructions and
         // ramp-up; a cluster barrier takes 0.25 us (16 blocks of 512 threads),
-        // a barrier over the whole grid 1.3 us.  A cluster barrier that has to
+        // a barrier over the whole grid 1.3 us.  Levels of the ghost update chain
+        // only where periodic exchanges stand between them: as overlapping launches
+        // of their own they take less (2D levels 2 to 8: 255 -> 220 us a step).  A cluster barrier that has to
         // wait for the blocks' stores takes 0.8 us, though, and every load after it
         // comes from L2 (0.2 us).  With periodic axes the exchanges between the
         // levels double the phases, most of them nearly empty: there the phases of
@@ -1578,6 +1607,8 @@ namespace sg
         template <int DIM, bool PERIODIC>
         __global__ void __launch_bounds__(CHAIN_THREADS, 1) k_chain(const __grid_constant__ Env Ep, const __grid_constant__ PhaseList L)
         {
+            dependency_wait<true>();
+            asm volatile("griddepcontrol.launch_dependents;");
             // the environment is read at every step of every phase: from shared memory, not from parameter
             // lines that each block would fetch one miss after the other
             __shared__ __align__(16) unsigned char store[sizeof(Env)];
@@ -1809,23 +1840,7 @@ namespace sg
             PhaseList list{};
             list.n = static_cast<int>(ps.size());
             std::copy(ps.begin(), ps.end(), list.p);
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim  = dim3(static_cast<unsigned>(c.chain_blocks));
-            cfg.blockDim = dim3(CHAIN_THREADS);
-            cfg.stream   = c.stream;
-            cudaLaunchAttribute at{};
-            at.id               = cudaLaunchAttributeClusterDimension;
-            at.val.clusterDim.x = static_cast<unsigned>(c.chain_blocks);
-            at.val.clusterDim.y = at.val.clusterDim.z = 1;
-            cfg.attrs    = &at;
-            cfg.numAttrs = 1;
-            const cudaError_t err = cudaLaunchKernelEx(&cfg, chain_kernel(c.g), e, list);
-            if (err != cudaSuccess)
-            {
-                cudaGetLastError();
-                c.err = std::string("chain: ") + cudaGetErrorString(err);
-                return SG_ERR_CUDA;
-            }
+            launch_dependent(c, true, chain_kernel(c.g), c.chain_blocks, CHAIN_THREADS, c.chain_blocks, e, list);
             launched(c, "chain");
             return check(c, "chain");
         }
@@ -1954,7 +1969,14 @@ namespace sg
         flush();
         if (!status)
         {
-            status = launch_phase_alone(c, env, p);
+            // a level of the ghost update right behind another one's launch
+            Phase q = p;
+            if ((op == OP_GHOST || op == OP_PREDICT) && (last_alone == OP_GHOST || last_alone == OP_PREDICT || last_alone == OP_PERIODIC_COPY))
+            {
+                q.aux = FOLLOWS;
+            }
+            last_alone = op;
+            status     = launch_phase_alone(c, env, q);
         }
     }
 
@@ -1962,6 +1984,7 @@ namespace sg
     {
         if (!status && !chain.empty())
         {
+            last_alone = -1;
             if (chain.size() == 1)
             {
                 chain[0].op &= static_cast<short>(~PHASE_SOLO);

@@ -132,6 +132,8 @@ namespace sg
         Phase p[CHAIN_MAX];
     };
 
+    constexpr short FOLLOWS = 1; // aux of a ghost-update level: launched right behind another one
+
     // Launches phases in order: small consecutive ones as one chain, the others
     // one by one.
     struct Sequence
@@ -140,6 +142,7 @@ namespace sg
         Env env;
         int status = SG_OK;
         std::vector<Phase> chain; // pending
+        int last_alone = -1;      // the phase launched last, if it was on its own
 
         Sequence(Ctx& ctx, const DeviceMesh& m, const DeviceMesh& n);
         void fields(const FieldSlot* fs, int first, int nf); // the fields of the following phases: fs[first .. first + nf)
