@@ -161,15 +161,10 @@ namespace
         }
         dfree(c.detail);
         dfree(c.block_sums);
-        dfree(c.d_counts);
         dfree(c.d_flags);
         dfree(c.d_absmax);
         dfree(c.g.err);
         dfree(h->staging);
-        if (c.h_counts)
-        {
-            cudaFreeHost(c.h_counts);
-        }
         if (c.h_flags)
         {
             cudaFreeHost(c.h_flags);
@@ -488,7 +483,6 @@ extern "C"
         st |= dalloc(c, &c.detail, static_cast<size_t>(c.capacity));
         c.n_scan_blocks = (c.g.total_words + 4095) / 4096;
         st |= dalloc(c, &c.block_sums, 5 * static_cast<size_t>(c.n_scan_blocks) + 8); // pairs per 2048 words and per 64 of those
-        st |= dalloc(c, &c.d_counts, static_cast<size_t>(sg::COUNTS));
         st |= dalloc(c, &c.d_flags, 8);
         st |= dalloc(c, &c.d_adapt, static_cast<size_t>(sg::A_COUNT));
         st |= dalloc(c, &c.d_setup, 1);
@@ -497,7 +491,6 @@ extern "C"
         if (!st)
         {
             if (cudaMallocHost(reinterpret_cast<void**>(&c.h_setup), sizeof(sg::PassSetup)) != cudaSuccess
-                || cudaMallocHost(reinterpret_cast<void**>(&c.h_counts), sg::COUNTS * sizeof(long long)) != cudaSuccess
                 || cudaMallocHost(reinterpret_cast<void**>(&c.h_flags), 8 * sizeof(int)) != cudaSuccess
                 || cudaMallocHost(reinterpret_cast<void**>(&c.h_adapt), sg::A_COUNT * sizeof(int)) != cudaSuccess)
             {

@@ -233,83 +233,6 @@ namespace sg
         return x | (x << 1);
     }
 
-    // Word of the coarsened set (parent of any member) at level l from the
-    // bitmap `fine` at level l+1.  Coarse word wi of row (yc, zc) covers the
-    // fine words 2*wi-1 and 2*wi of the fine rows 2*yc+{0,1} (x 2*zc+{0,1}).
-    __device__ __forceinline__ uint32_t coarsen_word(const Geom& g, const uint32_t* fine, int l, long long row, int wi)
-    {
-        const LevelGeom& C = g.lv[l];
-        const LevelGeom& F = g.lv[l + 1];
-        int yc, zc;
-        if (g.dim == 2)
-        {
-            yc = static_cast<int>(row) - PY;
-            zc = 0;
-        }
-        else
-        {
-            split_row(C, row, &yc, &zc);
-            yc -= PY;
-            zc -= PY;
-        }
-        uint32_t out = 0;
-        const int nz = (g.dim == 3) ? 2 : 1;
-        for (int sz = 0; sz < nz; ++sz)
-        {
-            for (int sy = 0; sy < 2; ++sy)
-            {
-                const int ry = 2 * yc + sy + PY;
-                const int rz = 2 * zc + sz + PY;
-                if (ry < 0 || ry >= F.R || (g.dim == 3 && (rz < 0 || rz >= F.R)))
-                {
-                    continue;
-                }
-                const long long frow = (g.dim == 2) ? ry : static_cast<long long>(rz) * F.R + ry;
-                const long long base = F.woff + frow * F.W;
-                const int k0         = 2 * wi - 1;
-                const uint32_t lo    = (k0 >= 0 && k0 < F.W) ? *(fine + base + k0) : 0u;
-                const uint32_t hi    = (k0 + 1 >= 0 && k0 + 1 < F.W) ? *(fine + base + k0 + 1) : 0u;
-                out |= compress_pairs(lo, hi);
-            }
-        }
-        return out;
-    }
-
-    // Word of the refined set (all children) at level l from `coarse` at
-    // level l-1.  Fine word k of row (yf, zf) reads coarse word (k+1)>>1 of
-    // row (yf>>1, zf>>1), low half when (k+1) is even, high half otherwise.
-    __device__ __forceinline__ uint32_t refine_word(const Geom& g, const uint32_t* coarse, int l, long long row, int k)
-    {
-        const LevelGeom& F = g.lv[l];
-        const LevelGeom& C = g.lv[l - 1];
-        int yf, zf;
-        if (g.dim == 2)
-        {
-            yf = static_cast<int>(row) - PY;
-            zf = 0;
-        }
-        else
-        {
-            split_row(F, row, &yf, &zf);
-            yf -= PY;
-            zf -= PY;
-        }
-        const int ry = (yf >> 1) + PY;
-        const int rz = (zf >> 1) + PY;
-        if (ry < 0 || ry >= C.R || (g.dim == 3 && (rz < 0 || rz >= C.R)))
-        {
-            return 0u;
-        }
-        const int wc = (k + 1) >> 1;
-        if (wc >= C.W)
-        {
-            return 0u;
-        }
-        const long long crow = (g.dim == 2) ? ry : static_cast<long long>(rz) * C.R + ry;
-        const uint32_t cw    = *(coarse + C.woff + crow * C.W + wc);
-        return spread16(((k + 1) & 1) ? (cw >> 16) : cw);
-    }
-
     // The word one level coarser that holds the parents of the cells of word
     // (row, wi) at level l: bit 0 of the word is x = 32 wi - PX, whose parent
     // x = 16 wi - PX/2 sits at position 16 wi + 16 of the coarse row, so the 16
@@ -375,56 +298,6 @@ namespace sg
         }
     }
 
-    // Cells of word (row, wi) at level l that lie in bm at level l or whose
-    // ancestor (levels l-1 .. lstop) lies in bm: the ancestors of the 32
-    // cells at level l - k are 32 >> k cells of one word (one cell from
-    // k = 5 on), read independently for every k and spread back.
-    __device__ __forceinline__ uint32_t self_or_ancestor(const Geom& g, const uint32_t* bm, int l, long long row, int wi, int lstop)
-    {
-        const LevelGeom& L = g.lv[l];
-        uint32_t acc       = *(bm + L.woff + row * L.W + wi);
-        int y, z;
-        if (g.dim == 2)
-        {
-            y = static_cast<int>(row) - PY;
-            z = 0;
-        }
-        else
-        {
-            split_row(L, row, &y, &z);
-            y -= PY;
-            z -= PY;
-        }
-        const int x0 = 32 * wi - PX;
-        for (int k = 1; l - k >= lstop; ++k)
-        {
-            const LevelGeom& A = g.lv[l - k];
-            const int ry = (y >> k) + PY, rz = (z >> k) + PY;
-            if (ry < 0 || ry >= A.R || (g.dim == 3 && (rz < 0 || rz >= A.R)))
-            {
-                continue;
-            }
-            const int pos        = (x0 >> (k < 31 ? k : 31)) + PX;
-            const long long arow = (g.dim == 2) ? ry : static_cast<long long>(rz) * A.R + ry;
-            const int width      = k >= 5 ? 1 : (32 >> k);
-            const uint32_t word  = __ldg(bm + A.woff + arow * A.W + (pos >> 5));
-            uint32_t bits        = (word >> (pos & 31)) & (width == 32 ? 0xFFFFFFFFu : ((1u << width) - 1u));
-            if (k >= 5)
-            {
-                acc |= bits ? 0xFFFFFFFFu : 0u;
-            }
-            else
-            {
-                for (int s = 0; s < k; ++s)
-                {
-                    bits = spread16(bits);
-                }
-                acc |= bits;
-            }
-        }
-        return acc;
-    }
-
     // x-dilation of one word by r (< 32) using its neighbours in the row
     __device__ __forceinline__ uint32_t dilate_x(uint32_t left, uint32_t mid, uint32_t right, int r)
     {
@@ -432,57 +305,6 @@ namespace sg
         for (int k = 1; k <= r; ++k)
         {
             out |= (mid << k) | (left >> (32 - k)) | (mid >> k) | (right << (32 - k));
-        }
-        return out;
-    }
-
-    // Box dilation split by axes: dilate_xy_word dilates along x and y within
-    // a z plane (the whole box dilation in 2D), dilate_z_word along z; in 3D
-    // box = z o xy reads 5 + 15 words instead of 75 for r = 2.
-    __device__ __forceinline__ uint32_t dilate_xy_word(const Geom& g, const uint32_t* src, int l, long long row, int wi, int r)
-    {
-        const LevelGeom& L = g.lv[l];
-        int ry, rz;
-        if (g.dim == 2)
-        {
-            ry = static_cast<int>(row);
-            rz = 0;
-        }
-        else
-        {
-            split_row(L, row, &ry, &rz);
-        }
-        uint32_t out = 0;
-        for (int dy = -r; dy <= r; ++dy)
-        {
-            const int y2 = ry + dy;
-            if (y2 < 0 || y2 >= L.R)
-            {
-                continue;
-            }
-            const long long base = L.woff + ((g.dim == 2) ? y2 : static_cast<long long>(rz) * L.R + y2) * L.W;
-            const uint32_t mid   = *(src + base + wi);
-            const uint32_t left  = wi > 0 ? *(src + base + wi - 1) : 0u;
-            const uint32_t right = wi + 1 < L.W ? *(src + base + wi + 1) : 0u;
-            out |= dilate_x(left, mid, right, r);
-        }
-        return out;
-    }
-
-    __device__ __forceinline__ uint32_t dilate_z_word(const Geom& g, const uint32_t* src, int l, long long row, int wi, int r)
-    {
-        const LevelGeom& L = g.lv[l];
-        int ry, rz;
-        split_row(L, row, &ry, &rz);
-        uint32_t out = 0;
-        for (int dz = -r; dz <= r; ++dz)
-        {
-            const int z2 = rz + dz;
-            if (z2 < 0 || z2 >= L.R)
-            {
-                continue;
-            }
-            out |= __ldg(src + L.woff + (static_cast<long long>(z2) * L.R + ry) * L.W + wi);
         }
         return out;
     }

@@ -35,7 +35,7 @@ namespace sg
         int* rank       = nullptr; // exclusive popcount prefix of ref
         int* wl_ref     = nullptr; // indices of the non-empty reference words, ascending
         int* wl_cells   = nullptr; // indices of the non-empty leaf-cell words, ascending
-        // Counters written by scan_rank on the device (layout below) and
+        // Counters written by the scan on the device (layout below) and
         // mirrored asynchronously into pinned host memory; kernels read the
         // device copy, so no launch waits for the host.
         long long* d_lo = nullptr;
@@ -180,9 +180,7 @@ namespace sg
         // scan scratch
         long long* block_sums = nullptr;
         long long n_scan_blocks = 0;
-        // device/host flags and counters
-        long long* d_counts = nullptr; // [0] = popcount total, [1..] misc
-        long long* h_counts = nullptr; // pinned mirror
+        // device/host flags
         int* d_flags        = nullptr;
         int* h_flags        = nullptr; // pinned mirror
         long long capacity  = 0;       // dense elements per field (32 * total_words)
@@ -298,7 +296,7 @@ namespace sg
 
     // Limits of the phases that join a chain (sg_phase.cuh), in words
     constexpr long long FUSE_WORDS       = 16384;
-    constexpr long long FUSE_WORDS_FIELD = 5000; // with periodic axes; 0 otherwise (2D levels 2 to 8: 220 us a step against 255)
+    constexpr long long FUSE_WORDS_FIELD = 5000; // with periodic axes; 0 otherwise (2D levels 2 to 8: 217 us a step, 256 in chains)
     constexpr long long FUSE_WORDS_MAX   = 12288;
     constexpr long long BATCH_FUSE_WORDS = 10000;
     // Smaller clusters in batched mode, where many meshes share the chip: 48 meshes of max_level 7..10 take
@@ -306,19 +304,6 @@ namespace sg
     inline int batch_chain_blocks(int n)
     {
         return n >= 16 ? 4 : (n >= 4 ? 8 : 16);
-    }
-
-    // blocks of 256 threads (8 warps) for a warp-per-item loop over at most
-    // max_items list entries: one wave of resident warps at most
-    inline int blocks_for_items(long long max_items)
-    {
-        long long b = (max_items + 7) / 8;
-        if (b < 1)
-        {
-            b = 1;
-        }
-        const long long cap = 152LL * 8;
-        return static_cast<int>(b > cap ? cap : b);
     }
 
     // launch helpers

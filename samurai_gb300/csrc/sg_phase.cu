@@ -1596,13 +1596,13 @@ namespace sg
         // ramp-up; a cluster barrier takes 0.25 us (16 blocks of 512 threads),
         // a barrier over the whole grid 1.3 us.  Levels of the ghost update chain
         // only where periodic exchanges stand between them: as overlapping launches
-        // of their own they take less (2D levels 2 to 8: 255 -> 220 us a step).  A cluster barrier that has to
+        // of their own they take less (2D levels 2 to 8: 256 -> 217 us a step).  A cluster barrier that has to
         // wait for the blocks' stores takes 0.8 us, though, and every load after it
         // comes from L2 (0.2 us).  With periodic axes the exchanges between the
         // levels double the phases, most of them nearly empty: there the phases of
         // the smallest levels run in the first block alone, block barriers between
         // them, and only the end of such a run is a cluster barrier (2D levels 3 to
-        // 9: 566 -> 522 us a step; without periodic axes the lone block loses what
+        // 9: 566 -> 522 us a step when it came in; without periodic axes the lone block loses what
         // the barriers save).
         template <int DIM, bool PERIODIC>
         __global__ void __launch_bounds__(CHAIN_THREADS, 1) k_chain(const __grid_constant__ Env Ep, const __grid_constant__ PhaseList L)

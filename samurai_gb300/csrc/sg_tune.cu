@@ -40,7 +40,7 @@ namespace sg
             int block;
             long long max_blocks, fuse_mesh, fuse_field, fuse_max;
             int graphed;     // the adaptation as one graph with conditional nodes (1) or pass by pass (0)
-            int level_pairs; // tag finalisation two levels per launch (1) or one (0)
+            int level_pairs; // kept in saved tunings, changes no launch
         };
 
         using TuneKey = std::tuple<std::string, int, int, int>; // device name, dim, min_level, max_level
