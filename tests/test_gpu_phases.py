@@ -16,6 +16,7 @@ SHAPES = [
     {"SG_CHAIN_BLOCKS": "2"},
     {"SG_CHAIN_BLOCKS": "16", "SG_FUSE_WORDS": "1000000", "SG_FUSE_WORDS_FIELD": "1000000", "SG_FUSE_WORDS_MAX": "1000000"},
     {"SG_BLOCK": "96", "SG_MAX_BLOCKS": "3"},
+    {"SG_OVERLAP_LAUNCHES": "0"},
 ]
 
 
@@ -49,7 +50,7 @@ def advance(sg, g, o, dim, maxl, eps, reg, steps):
     compare_meshes(g, o, maxl, "final")
 
 
-@pytest.mark.parametrize("env", SHAPES, ids=["alone", "two blocks", "all chained", "odd blocks"])
+@pytest.mark.parametrize("env", SHAPES, ids=["alone", "two blocks", "all chained", "odd blocks", "not overlapped"])
 @pytest.mark.parametrize("dim,minl,maxl,radius,pred", [(2, 1, 2, 1, 1), (2, 4, 4, 1, 1), (2, 2, 7, 2, 1), (2, 3, 9, 1, 0), (3, 1, 3, 1, 1), (3, 2, 5, 2, 1)])
 def test_phases_against_oracle(sg, monkeypatch, env, dim, minl, maxl, radius, pred):
     for k, v in env.items():
@@ -112,3 +113,29 @@ def test_more_fields_than_one_phase_takes(sg, monkeypatch, env):
     for c, k in enumerate(ks):
         assert np.array_equal(got[:, c], o.cell_values_k(k)), c
     assert np.array_equal(w.cell_values(), o.cell_values_k(kw))
+
+
+@pytest.mark.parametrize("minl,maxl", [(4, 4), (2, 6)])
+@pytest.mark.parametrize("a", [[0.9, -0.6], [0.0, 1.0]])
+def test_flux_form_of_values_that_are_not_finite(sg, minl, maxl, a):
+    """a term with a zero coefficient may be left out only where its value is finite: 0 * inf is NaN in the oracle"""
+    g, o = sg.AdvectionSim(2, minl, maxl), OracleSim(2, minl, maxl)
+    lv, co, _ = o.cells()
+    vals = shapes_2d(5, 3, 3)(lv, co)
+    g.set_cell_values(vals)
+    o.set_cell_values(vals)
+    if minl < maxl:
+        assert g.adapt(1e-3, 1.0) == o.adapt(1e-3, 1.0)
+    n = len(o.cells()[0])
+    vals = np.cos(np.arange(n))
+    vals[n // 5], vals[n // 2], vals[4 * n // 5] = np.inf, -np.inf, np.nan
+    g.set_cell_values(vals)
+    o.set_cell_values(vals)
+    g.update_ghost()
+    o.update_ghost()
+    g.upwind(a, 0.3 / (1 << maxl), 2)
+    o.upwind(a, 0.3 / (1 << maxl), 2)
+    idx = o.cells()[2]
+    got, want = g.field()[idx], o.field()[idx]
+    assert np.isnan(want).any() and np.isfinite(want).any()
+    assert np.array_equal(got, want, equal_nan=True)
