@@ -39,7 +39,7 @@ CFG_3D = dict(dim=3, min_level=3, max_level=9, a=(1.0, 1.0, 1.0), eps=1e-3, regu
 METRIC = "active cell-updates/s"
 UNIT = "cell-updates/s"
 L2_BYTES = 129 * 1024 * 1024
-UPWIND_DRAM_BYTES_PER_CELL = 8572672.0 / 511813.0
+UPWIND_DRAM_BYTES_PER_CELL = 8324352.0 / 539794.0
 
 
 def workload_config(extra=None):
@@ -155,8 +155,8 @@ UPWIND_ISSUED = {2: 10 * 2 + 3 + 2, 3: 10 * 3 + 5 + 2}
 # DRAM bytes per launch of the kernels named dominant, by (dim, max_level, kernel), from ncu captures (profiles/):
 # (bytes, how they were measured)
 DOMINANT_TRAFFIC = {
-    (2, 12, "ghost_level"): (959558.0, "ncu dram__bytes_read.sum + dram__bytes_write.sum averaged over the 22 k_ghost_level launches of one "
-                              "2D max_level-12 step (levels 12..2, twice; caches emptied by ncu before each launch)"),
+    (2, 12, "ghost_level"): (954380.0, "ncu dram__bytes_read.sum + dram__bytes_write.sum averaged over the 22 ghost level launches of one "
+                              "2D max_level-12 step on a mesh of about 540 000 leaves (caches emptied by ncu before each launch)"),
 }
 
 
@@ -231,10 +231,11 @@ def mesh_id_counts(sim, maxl):
 # bitmaps a word kernel reads or writes, per word of the levels it covers
 # (4 bytes each): the algorithmic traffic of the integer mesh kernels
 WORD_KERNEL_BITMAPS = {
-    "hc_cag": 3, "hc2_cag_on": 4, "hc2_cag_z": 4, "cag_on": 2, "union": 3, "ref0": 4, "ref0_xy": 4, "ref0_z": 4, "ref_children": 4,
-    "proj": 3, "scan_sums": 2, "scan_write": 5, "tag_flags": 3, "new_cells": 4, "grad_coarsen": 2, "grad_expand": 2, "grad_expand_xy": 2,
-    "grad_expand_z": 2, "grad_down": 5, "grad_apply": 3, "compare": 2,
+    "clear_union": 1, "hc_cag": 4, "hc2_cag": 4, "cag_on": 2, "ref0": 4, "ref0_xy": 4, "ref0_z": 4, "ref_children": 5,
+    "scan_sums": 2, "scan_write": 5, "new_cells": 5, "grad_coarsen": 3, "grad_expand": 2, "grad_expand_xy": 2,
+    "grad_expand_z": 2, "grad_down": 5, "grad_refine": 3, "grad_apply": 3, "compare": 2,
 }
+BACK_KERNELS = ("clear_union", "hc_cag", "hc2_cag", "cag_on", "ref0", "ref0_xy", "ref0_z", "ref_children", "scan_sums", "scan_write")
 
 
 def kernel_bytes(name, dim, counts, halo, words_all, words_ref, passes):
@@ -246,18 +247,16 @@ def kernel_bytes(name, dim, counts, halo, words_all, words_ref, passes):
     ch = 1 << dim
     fronts, backs = passes
     ghosts = max(nr - nc - npj, 0)
+    # word phases over the list of reference words: at least nr / 32 words
+    lw = 4 * nr // 32
     per_front = {
-        "tag_init": 9 * nr,
+        "pass_begin": 4 * lw,                        # list read, three threshold bitmaps cleared
         "ghost_level": 8 * (ch + 1) * npj,           # projection: 2^d children read, 1 written
-        "ghost_levels_small": 0,
         "ghost_corner_projection": 0,
         "predict": 8 * ghosts + 8 * ghosts // ch,    # ghost written + its coarse parent read
-        "predict_small": 0,
         "detail": 8 * (1 + 2 * ch) * npj,            # parent + children read, children's details written
-        "criteria": (8 * (ch + 1) + ch) * npj,       # details read, tags written
-        "maximum": 2 * (ch + 1) * npj,               # tags read and written
-        "maximum_small": 0,
-        "keep_boundary": 0,
+        "criteria": 11 * lw,                         # cells, thresholds and their parents' words read, tags written
+        "maximum": 8 * lw,                           # two tag bitmaps of parents and children read and written
     }
     if name == "upwind" or name == "convection":
         return 16 * nc + 8 * halo
@@ -266,10 +265,9 @@ def kernel_bytes(name, dim, counts, halo, words_all, words_ref, passes):
     if name == "update_fields":
         return 16 * nr * backs
     if name in WORD_KERNEL_BITMAPS:
-        words = words_all if name in ("tag_flags", "new_cells", "compare", "scan_sums", "scan_write") else words_ref
+        words = words_all if name in ("new_cells", "compare", "scan_sums", "scan_write", "clear_union") else words_ref
         # the scan and mesh construction run once per back half, the others once per front half
-        n = backs if name in ("hc_cag", "hc2_cag_on", "hc2_cag_z", "cag_on", "union", "ref0", "ref0_xy", "ref0_z", "ref_children", "proj",
-                              "scan_sums", "scan_write") else fronts
+        n = backs if name in BACK_KERNELS else fronts
         return 4 * WORD_KERNEL_BITMAPS[name] * words * n
     return 0
 
@@ -348,7 +346,7 @@ def run_gpu(args):
     if not args.no_tune:
         d_ms, t_ms, shape = sim.autotune(CFG["eps"], CFG["regularity"], a, dt, steps=10)
         tune = {"default_ms_per_step": d_ms, "tuned_ms_per_step": t_ms, "shape": shape,
-                "how": "sg_autotune: coordinate descent over threads per block, grid limit and one-block chain limits, "
+                "how": "sg_autotune: coordinate descent over threads per block, grid limit and chain limits, "
                        "10 steps from the same state per candidate, best of two"}
     for _ in range(args.warmup):
         step()
@@ -527,7 +525,7 @@ def run_gpu(args):
             "kernels_step": ktab,
             "upwind_roofline": {"bound": "hbm", "kernel": "k_upwind", "achieved": achieved, "peak": peak, "peak_source": peak_src, "unit": "GB/s",
                                 "frac": achieved / peak, "traffic": traffic,
-                                "traffic_source": "ncu dram__bytes of a 536 428-cell launch, scaled by leaf cells",
+                                "traffic_source": "ncu dram__bytes of a 539 794-cell launch, scaled by leaf cells",
                                 "algorithmic_bytes": int(alg_bytes), "launch_ms": upw_ms, "timing": "k_upwind alone, L2 flushed, 20 launches",
                                 "cells": int(nc), "halo": int(halo),
                                 "fp64": {"achieved_gflops": fp64_ops / (upw_ms / 1e3) / 1e9, "peak_gflops": fp64_peak,
@@ -708,7 +706,7 @@ def batch_record(args, steps, warmup, serial_steps, full=False):
     if not args.no_tune:
         d_ms, t_ms, shape = batch.autotune(eps, reg, a, dt, steps=3)
         tune = {"default_ms_per_step": d_ms, "tuned_ms_per_step": t_ms, "shape": shape,
-                "how": "sg_batch_autotune: one-block chain limit shared by the instances, then threads per block; "
+                "how": "sg_batch_autotune: chain limit shared by the instances, then threads per block; "
                        "3 batched steps from the same state per candidate"}
     for _ in range(warmup):
         batch.step(eps, reg, a, dt)

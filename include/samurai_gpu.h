@@ -123,9 +123,10 @@ int sg_mesh_set_adapt_graph(sg_mesh_t mesh, int enable);
  * chosen shape. */
 int sg_autotune(sg_field_t u, sg_field_t unp1, double eps, double regularity, const double* a, double dt, int scheme, int steps,
                 double* default_ms, double* tuned_ms);
-/* the mesh's launch shape: threads per block, grid limit (blocks of 8 warps), one-block chain limits in words per
+/* the mesh's launch shape: threads per block, grid limit (blocks of 8 warps), chain limits in words per
  * level of the mesh, field and tag-finalisation chains, 1 when the adaptation runs as one graph with conditional
- * nodes (0: pass by pass), 1 when the tag-finalisation chain takes two levels per launch; any pointer may be NULL */
+ * nodes (0: pass by pass), level_pairs is kept for callers and saved
+ * tunings and changes no launch; a chain limit is the most words a phase may walk to share a launch; any pointer may be NULL */
 int sg_launch_shape(sg_mesh_t mesh, int* block, long long* max_blocks, long long* fuse_mesh_words, long long* fuse_field_words,
                     long long* fuse_max_words, int* graphed_adapt, int* level_pairs);
 
@@ -291,7 +292,7 @@ int sg_batch_synchronize(sg_batch_t batch);
  * batched step time under the starting and the chosen shape. */
 int sg_batch_autotune(sg_batch_t batch, const double* eps, const double* regularity, const double* a, const double* dt, int scheme,
                       int steps, double* default_ms, double* tuned_ms);
-/* the batch's launch shape: one-block chain limit in words per level, threads per block (0: each instance's own) */
+/* the batch's launch shape: chain limit in words per level, threads per block (0: each instance's own) */
 int sg_batch_launch_shape(sg_batch_t batch, long long* fuse_words, int* block);
 
 /* Discrete adjoint of the time loop (no counterpart in samurai, which has no derivatives).  The loop of
