@@ -155,7 +155,7 @@ namespace
         dfree(c.t2);
         dfree(c.t3);
         dfree(c.rf);
-        for (uint32_t** bm : {&c.tk, &c.tc, &c.tr, &c.above, &c.ref_above, &c.par_above})
+        for (uint32_t** bm : {&c.tk, &c.tc, &c.tr, &c.above, &c.ref_above, &c.par_above, &c.exam})
         {
             dfree(*bm);
         }
@@ -390,13 +390,13 @@ extern "C"
             return fail(SG_ERR_CUDA, "sg_mesh_create: no CUDA device");
         }
         {
-            // device memory of the mesh (two meshes of 11 word arrays, 5 scratch and 6 tag bitmaps, the dense detail
+            // device memory of the mesh (two meshes of 11 word arrays, 5 scratch and 7 tag bitmaps, the dense detail
             // slab) and of one field with its update_fields buffer, against the free memory of the device: a
             // configuration that cannot fit is refused here rather than by a failing allocation midway
             const sg::Geom gg    = sg::make_geom(dim, min_level, max_level);
             const double words   = static_cast<double>(gg.total_words);
             const double cap     = 32.0 * words;
-            const double mesh_b  = (2.0 * 11.0 + 5.0 + 6.0) * 4.0 * words + 8.0 * cap;
+            const double mesh_b  = (2.0 * 11.0 + 5.0 + 7.0) * 4.0 * words + 8.0 * cap;
             const double field_b = 16.0 * cap;
             size_t free_b = 0, total_b = 0;
             if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess)
@@ -476,7 +476,7 @@ extern "C"
         st |= dalloc(c, &c.t2, nw);
         st |= dalloc(c, &c.t3, nw);
         st |= dalloc(c, &c.rf, nw);
-        for (uint32_t** bm : {&c.tk, &c.tc, &c.tr, &c.above, &c.ref_above, &c.par_above})
+        for (uint32_t** bm : {&c.tk, &c.tc, &c.tr, &c.above, &c.ref_above, &c.par_above, &c.exam})
         {
             st |= dalloc(c, bm, nw);
         }
@@ -516,7 +516,7 @@ extern "C"
             }
         }
         cudaMemsetAsync(c.detail, 0, static_cast<size_t>(c.capacity) * sizeof(double), c.stream);
-        for (uint32_t* bm : {c.tk, c.tc, c.tr, c.above, c.ref_above, c.par_above})
+        for (uint32_t* bm : {c.tk, c.tc, c.tr, c.above, c.ref_above, c.par_above, c.exam})
         {
             cudaMemsetAsync(bm, 0, nw * 4, c.stream);
         }
@@ -1430,6 +1430,7 @@ extern "C"
                 return from_ctx(c, SG_ERR_CUDA);
             }
             cudaMemsetAsync(c.detail, 0, static_cast<size_t>(c.capacity) * n * sizeof(double), c.stream);
+            cudaMemsetAsync(c.exam, 0, static_cast<size_t>(c.g.total_words) * 4, c.stream);
             c.detail_comps = n;
             sg::clear_graphs(c); // they hold the old detail buffer
         }

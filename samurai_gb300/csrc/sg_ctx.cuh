@@ -177,6 +177,7 @@ namespace sg
         uint32_t* above     = nullptr;
         uint32_t* ref_above = nullptr;
         uint32_t* par_above = nullptr;
+        uint32_t* exam      = nullptr; // cells whose parent was examined by the last pass that had them in its reference (details)
         // scan scratch
         long long* block_sums = nullptr;
         long long n_scan_blocks = 0;
@@ -240,8 +241,9 @@ namespace sg
     int upwind_on(Ctx& c, const DeviceMesh& m, const double* ud, double* unp1d, const double* a, double dt, int scheme);
     int step(Ctx& c, DeviceField& u, DeviceField& unp1, double eps, double regularity, const double* a, double dt, int scheme, int* n_harten);
     int gather_compact(Ctx& c, const DeviceMesh& m, const double* dense, double* compact);
-    int gather_details(Ctx& c, const DeviceMesh& m, double* compact); // the details of the last pass (first field)
-    int tag_bytes(Ctx& c, const DeviceMesh& m, uint8_t* compact);     // its tags: keep 1, coarsen 2, refine 4
+    // details (first field) and tags (keep 1, coarsen 2, refine 4) of the last pass that had a cell in its reference
+    int gather_details(Ctx& c, const DeviceMesh& m, double* compact);
+    int tag_bytes(Ctx& c, const DeviceMesh& m, uint8_t* compact);
     cudaError_t launch_gather(Ctx& c, const DeviceMesh& m, const double* dense, double* compact); // no error text
     cudaError_t read_device_error(Ctx& c, int* v);                                                  // reads and clears
     int scatter_compact(Ctx& c, const DeviceMesh& m, const double* compact, double* dense);

@@ -588,24 +588,11 @@ namespace sg
         }
 
         // details in the reference numbering: a cell whose parent the pass did not examine has none (0)
-        template <int DIM>
-        __global__ void k_gather_details(const __grid_constant__ Geom gp, MeshPtrs m, const PassSetup* setup, const double* det, double* compact)
+        __global__ void k_gather_details(MeshPtrs m, int nlev, const uint32_t* exam, const double* det, double* compact)
         {
-            const Geom& g = gp;
-            const int dl0 = max(g.min_level - 1, 0), le = g.max_level - setup->ite - 1;
-            warp_list(m.wl_ref, m.lo[LO_REF], m.lo[LO_REF + g.nlev], warp_id(), warp_count(), [&](long long w) { return m.ref[w]; },
+            warp_list(m.wl_ref, m.lo[LO_REF], m.lo[LO_REF + nlev], warp_id(), warp_count(), [&](long long w) { return m.ref[w]; },
                       [&](long long w, int b)
-                      {
-                          const int l     = level_down(g, static_cast<int>(w), 0, g.max_level);
-                          bool examined   = false;
-                          if (l - 1 >= dl0 && l - 1 <= le)
-                          {
-                              const Cell c = cell_of(g, l, w, b);
-                              const Pos p  = pos_of(g, l - 1, c.x >> 1, c.y >> 1, DIM == 3 ? c.z >> 1 : 0);
-                              examined     = test(m.ref, p) && (test(m.hc, p) || test(m.hc2, p));
-                          }
-                          compact[ref_index(m.ref, m.rank, Pos{w, b})] = examined ? det[32 * w + b] : 0.;
-                      });
+                      { compact[ref_index(m.ref, m.rank, Pos{w, b})] = ((exam[w] >> b) & 1u) ? det[32 * w + b] : 0.; });
         }
 
         __global__ void k_tag_bytes(MeshPtrs m, int nlev, const uint32_t* tk, const uint32_t* tc, const uint32_t* tr, uint8_t* compact)
@@ -684,14 +671,7 @@ namespace sg
 
     int gather_details(Ctx& c, const DeviceMesh& m, double* compact)
     {
-        if (c.g.dim == 2)
-        {
-            k_gather_details<2><<<blocks_words(c, 0, c.g.nlev - 1), c.block, 0, c.stream>>>(c.g, mesh_ptrs(m), c.d_setup, c.detail, compact);
-        }
-        else
-        {
-            k_gather_details<3><<<blocks_words(c, 0, c.g.nlev - 1), c.block, 0, c.stream>>>(c.g, mesh_ptrs(m), c.d_setup, c.detail, compact);
-        }
+        k_gather_details<<<blocks_words(c, 0, c.g.nlev - 1), c.block, 0, c.stream>>>(mesh_ptrs(m), c.g.nlev, c.exam, c.detail, compact);
         launched(c, "gather");
         return check(c, "gather_details");
     }

@@ -302,6 +302,8 @@ namespace sg
         //  - the children of a parent that is not above its own threshold and has no child above theirs are
         //    tagged coarsen (only);
         //  - the cells above the refinement threshold are tagged refine.
+        // Cells of the word outside the reference keep what an earlier pass left them, as they do in samurai's
+        // numbering: a mesh read after it changed shows the last pass that knew the cell.
         template <int DIM>
         __device__ __forceinline__ void op_criteria(const Env& E, const Team& T)
         {
@@ -312,7 +314,7 @@ namespace sg
                 [&](int w)
                 {
                     const int l = level_down(g, w, 0, g.max_level);
-                    uint32_t k = E.m.cells[w], c = 0u, r = 0u;
+                    uint32_t k = E.m.cells[w], c = 0u, r = 0u, examined = 0u;
                     if (l >= g.min_level && l <= le)
                     {
                         const Word p   = word_at<DIM>(g, l, w);
@@ -320,7 +322,9 @@ namespace sg
                         if (q.w >= 0)
                         {
                             // the 16 parents of the word's cells
-                            const uint32_t par = ((E.m.ref[q.w] & E.m.hc[q.w]) >> q.shift) & 0xFFFFu;
+                            const uint32_t pref = E.m.ref[q.w], phc = E.m.hc[q.w];
+                            const uint32_t par  = ((pref & phc) >> q.shift) & 0xFFFFu;
+                            examined            = spread16((pref & (phc | E.m.hc2[q.w])) >> q.shift);
                             if (par)
                             {
                                 if (l > g.min_level)
@@ -355,9 +359,11 @@ namespace sg
                         c &= ~edge;
                         r &= ~edge;
                     }
-                    E.tk[w] = k;
-                    E.tc[w] = c;
-                    E.tr[w] = r;
+                    const uint32_t other = ~E.m.ref[w];
+                    E.tk[w]   = (E.tk[w] & other) | k;
+                    E.tc[w]   = (E.tc[w] & other) | c;
+                    E.tr[w]   = (E.tr[w] & other) | r;
+                    E.exam[w] = (E.exam[w] & other) | examined;
                 });
         }
 
@@ -1870,6 +1876,7 @@ namespace sg
         env.above           = c.above;
         env.ref_above       = c.ref_above;
         env.par_above       = c.par_above;
+        env.exam            = c.exam;
         env.det             = c.detail;
         env.capacity        = c.capacity;
         env.setup           = c.d_setup;

@@ -99,6 +99,7 @@ namespace sg
         uint32_t *t0, *t1, *t2, *t3, *rf;
         uint32_t *tk, *tc, *tr;    // tags: keep, coarsen, refine
         uint32_t *above, *ref_above, *par_above; // |detail| over the coarsen, refine and parent thresholds
+        uint32_t* exam;            // cells with a detail
         double* det;
         long long capacity;
         PassSetup* setup;
