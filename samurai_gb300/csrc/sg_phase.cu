@@ -315,6 +315,10 @@ namespace sg
                 {
                     const int l = level_down(g, w, 0, g.max_level);
                     uint32_t k = E.m.cells[w], c = 0u, r = 0u, examined = 0u;
+                    // what the word holds outside the reference, loaded here: behind the stores the loads would wait
+                    // for each other
+                    const uint32_t other = ~E.m.ref[w];
+                    const uint32_t was_k = E.tk[w] & other, was_c = E.tc[w] & other, was_r = E.tr[w] & other, was_e = E.exam[w] & other;
                     if (l >= g.min_level && l <= le)
                     {
                         const Word p   = word_at<DIM>(g, l, w);
@@ -359,11 +363,10 @@ namespace sg
                         c &= ~edge;
                         r &= ~edge;
                     }
-                    const uint32_t other = ~E.m.ref[w];
-                    E.tk[w]   = (E.tk[w] & other) | k;
-                    E.tc[w]   = (E.tc[w] & other) | c;
-                    E.tr[w]   = (E.tr[w] & other) | r;
-                    E.exam[w] = (E.exam[w] & other) | examined;
+                    E.tk[w]   = was_k | k;
+                    E.tc[w]   = was_c | c;
+                    E.tr[w]   = was_r | r;
+                    E.exam[w] = was_e | examined;
                 });
         }
 
