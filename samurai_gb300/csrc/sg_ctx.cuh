@@ -76,6 +76,7 @@ namespace sg
         F_GRADX = 3,  // scratch for extra graduation passes
         F_ERR   = 4,  // the mesh's error word, in the host's copy
         F_DONE  = 5,  // blocks of the comparison that are through
+        F_AHEAD = 6,  // the compared cells are final (no third graduation pass) and differ
         F_COUNT = 8
     };
 

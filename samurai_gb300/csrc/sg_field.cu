@@ -1344,13 +1344,13 @@ namespace sg
         // for the adapted fields fs and the fields os carried along (their
         // ghosts are updated first, mr/adapt.hpp:383)
         // ahead: launched before the host knows whether the pass changed the mesh;
-        // the phases hang on the pass's flag.  clear: not the first time after the
-        // pass's front, which left the union of the new mesh empty.
+        // the phases hang on the pass's flag.  The pass's front left the union of the
+        // new mesh empty.
         int seq_back(Ctx& c, DeviceMesh& m, DeviceMesh& nm, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os,
-                     bool ahead = false, bool clear = false)
+                     bool ahead = false)
         {
             Sequence s(c, m, nm);
-            s.guard(ahead ? c.d_flags + F_DIFFER : nullptr);
+            s.guard(ahead ? c.d_flags + F_AHEAD : nullptr);
             if (!os.empty())
             {
                 s.timer_start(T_GHOST);
@@ -1362,7 +1362,7 @@ namespace sg
             const std::vector<FieldSlot> slots = slots_of(all);
             s.fields(slots.data(), 0, std::min(PHASE_FIELDS, static_cast<int>(slots.size())));
             s.timer_start(T_CONSTRUCTION);
-            build_mesh_phases(s, clear);
+            build_mesh_phases(s, false);
             s.timer_stop(T_CONSTRUCTION);
             s.timer_start(T_FIELDS_UPDATE);
             field_groups(s, slots, [&]() { s.add(OP_UPDATE_FIELDS); });
@@ -1446,21 +1446,21 @@ namespace sg
     namespace
     {
         // the second half of a pass, from its graph
-        int launch_back(Ctx& c, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os, bool ahead, bool clear)
+        int launch_back(Ctx& c, const std::vector<DeviceField*>& fs, const std::vector<DeviceField*>& os, bool ahead)
         {
             DeviceMesh& m  = c.m();
             DeviceMesh& nm = c.spare();
-            const unsigned long long kind = (ahead ? 1ull << 40 : 0ull) | (clear ? 1ull << 41 : 0ull);
+            const unsigned long long kind = ahead ? 1ull << 40 : 0ull;
             if (fs.size() == 1 && os.empty())
             {
                 DeviceField& f = *fs[0];
                 return run_cached(c, 3 | kind, static_cast<unsigned long long>(c.cur), ptr_key(f.data), ptr_key(f.spare),
-                                  [&]() { return seq_back(c, m, nm, fs, os, ahead, clear); });
+                                  [&]() { return seq_back(c, m, nm, fs, os, ahead); });
             }
             std::vector<DeviceField*> all(fs);
             all.insert(all.end(), os.begin(), os.end());
             return run_cached(c, (7 + 16 * fs.size()) | kind, static_cast<unsigned long long>(c.cur), fields_key(all, false), fields_key(all, true),
-                              [&]() { return seq_back(c, m, nm, fs, os, ahead, clear); });
+                              [&]() { return seq_back(c, m, nm, fs, os, ahead); });
         }
     } // namespace
 
@@ -1496,12 +1496,13 @@ namespace sg
                             [&]() { return seq_front(c, m, nm, fs); });
         }
         // The first pass of an adaptation usually changes the mesh: its second half is queued before the host
-        // hears of it (it writes only the spare mesh and the spare buffers, and hangs on the pass's flag), so
-        // the GPU does not wait for the round trip.
+        // hears of it, so the GPU does not wait for the round trip.  It hangs on a flag of the pass that is set only
+        // when the pass's cells are final and differ: a pass that keeps its mesh, or whose graduation goes on from
+        // the host, changes nothing more, the ghosts of the fields carried along included.
         c.back_ahead = !st && ite == 0;
         if (c.back_ahead)
         {
-            st = launch_back(c, fs, os, true, false);
+            st = launch_back(c, fs, os, true);
         }
         return st;
     }
@@ -1533,7 +1534,8 @@ namespace sg
         if (c.h_flags[F_GRAD1])
         {
             // graduation still refining after two passes: finish the fixed
-            // point with host-tested passes, then compare again
+            // point with host-tested passes, then compare again (a second half
+            // queued ahead did not run)
             back_queued = false;
             if ((st = graduate(c, m, nm, nullptr)))
             {
@@ -1558,7 +1560,7 @@ namespace sg
             return SG_OK;
         }
         *converged = false;
-        if (!back_queued && (st = launch_back(c, fs, os, false, c.back_ahead)))
+        if (!back_queued && (st = launch_back(c, fs, os, false)))
         {
             return st;
         }
@@ -1577,7 +1579,8 @@ namespace sg
     }
 
     // The error word of an adaptation: a last pass that kept the mesh reported it with its flags, and nothing
-    // ran after it; otherwise it is read from the device.
+    // that can raise it ran after that (further graduation and the comparison only move bits); otherwise it is
+    // read from the device.
     int pass_error(Ctx& c, bool converged)
     {
         return converged && c.h_flags[F_ERR] == 0 ? SG_OK : device_error(c);

@@ -748,7 +748,8 @@ namespace sg
             {
                 return;
             }
-            // the last block leaves the flags and the mesh's error word with the host
+            // the last block leaves the flags and the mesh's error word with the host, and settles the flag that a
+            // second half queued ahead hangs on
             __shared__ bool last;
             __threadfence();
             __syncthreads();
@@ -761,7 +762,14 @@ namespace sg
             {
                 __threadfence();
                 const int k = static_cast<int>(threadIdx.x);
-                E.report[k] = *static_cast<volatile int*>(k == F_ERR ? E.g.err : E.flags + k);
+                const int v = *static_cast<volatile int*>(k == F_ERR ? E.g.err : E.flags + k);
+                constexpr unsigned SLOTS = (1u << F_COUNT) - 1u;
+                const bool differ = __shfl_sync(SLOTS, v, F_DIFFER) != 0, final = __shfl_sync(SLOTS, v, F_GRAD1) == 0;
+                if (k == F_AHEAD)
+                {
+                    E.flags[F_AHEAD] = differ && final;
+                }
+                E.report[k] = v;
             }
         }
 

@@ -96,3 +96,29 @@ def test_every_pass_reads_as_it_was_made(sg, dim, minl, maxl, radius, per):
             g.upwind(a, dt)
             o.upwind(a, dt)
     assert changed > 4 and leftover > 0
+
+
+@pytest.mark.parametrize("dim,minl,maxl,radius", [(2, 2, 8, 1), (2, 2, 8, 2), (3, 2, 6, 1)])
+def test_a_pass_that_keeps_the_mesh_leaves_carried_fields_alone(sg, dim, minl, maxl, radius):
+    """a mesh refined along the boundary only: the criteria coarsen every ring inside, and the graduation refines them
+    again, ring after ring (with radius 2 in more than two of its passes), until the cells are the old ones.  Fields carried along
+    get new ghosts only when the mesh changes (mr/adapt.hpp:380-386)."""
+    mesh = sg.MRMesh(dim, minl, maxl, radius, 1, 1)
+    mesh.set_refine_boundary(True)
+    u, w = sg.make_scalar_field("u", mesh), sg.make_scalar_field("w", mesh)
+    for f in (u, w):
+        sg.make_bc(sg.Dirichlet(1), f, 0.0)
+    u.fill(0.0)
+    adapt = sg.make_MRAdapt(u)
+    cfg = sg.mra_config().epsilon(1e-4).regularity(0.0)
+    for _ in range(2 * maxl):
+        if adapt(cfg) == 1:
+            break
+    before = mesh.cells()
+    assert set(before[0]) >= set(range(maxl - 3, maxl + 1))
+    values = np.random.default_rng(3).uniform(1.0, 2.0, mesh.nb_cells("reference"))
+    w.set_array(values)
+    assert adapt(cfg, w) == 1
+    after = mesh.cells()
+    assert all(np.array_equal(x, y) for x, y in zip(before, after))
+    assert np.array_equal(w.array(), values)
