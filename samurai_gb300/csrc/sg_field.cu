@@ -1499,7 +1499,7 @@ namespace sg
         // hears of it, so the GPU does not wait for the round trip.  It hangs on a flag of the pass that is set only
         // when the pass's cells are final and differ: a pass that keeps its mesh, or whose graduation goes on from
         // the host, changes nothing more, the ghosts of the fields carried along included.
-        c.back_ahead = !st && ite == 0;
+        c.back_ahead = !st && ite == 0 && !c.timers.enabled; // the named timers count the halves that run
         if (c.back_ahead)
         {
             st = launch_back(c, fs, os, true);

@@ -122,3 +122,18 @@ def test_a_pass_that_keeps_the_mesh_leaves_carried_fields_alone(sg, dim, minl, m
     after = mesh.cells()
     assert all(np.array_equal(x, y) for x, y in zip(before, after))
     assert np.array_equal(w.array(), values)
+
+
+def test_timers_count_the_phases_of_the_mesh_that_changed(sg):
+    """an adaptation whose first pass keeps the mesh builds no mesh and moves no field"""
+    s = sg.AdvectionSim(2, 2, 7)
+    lv, co, _ = s.cells()
+    s.set_cell_values(shapes_2d(5, 3, 3)(lv, co))
+    while s.adapt(1e-3, 1.0) > 1:
+        pass
+    s.mesh.timers(enable=True, reset=True)
+    assert s.adapt(1e-3, 1.0) == 1
+    s.mesh.synchronize()
+    t = s.mesh.timers(enable=False)
+    assert t["mesh adaptation"][1] == 1 and t["detail computation"][1] == 1
+    assert t["mesh construction"] == (0.0, 0) and t["fields update"] == (0.0, 0)
