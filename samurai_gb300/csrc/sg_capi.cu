@@ -61,6 +61,7 @@ namespace
         {
             c.err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
             *p    = nullptr;
+            cudaGetLastError(); // reported here, not by the next launch's check
             return sg::SG_ERR_CUDA;
         }
         return sg::SG_OK;
@@ -312,6 +313,50 @@ namespace sg
             return SG_ERR_CUDA;
         }
         return SG_OK;
+    }
+
+    // Dense detail slabs and maxima for n adapted fields.  The contents are rebuilt by every pass, so the old slabs
+    // make room for the new ones; when those do not fit, the mesh gets back what it had, and where even that is gone
+    // (detail_comps 0) the next adaptation asks again.
+    int ensure_details(Ctx& c, int n)
+    {
+        if (n <= c.detail_comps)
+        {
+            return SG_OK;
+        }
+        unsigned long long* absmax = nullptr;
+        if (dalloc(c, &absmax, static_cast<size_t>(n)))
+        {
+            return SG_ERR_CUDA;
+        }
+        cudaStreamSynchronize(c.stream);
+        clear_graphs(c); // they hold the old buffers
+        const int had = c.detail_comps;
+        dfree(c.detail);
+        c.detail_comps = 0;
+        int st         = dalloc(c, &c.detail, static_cast<size_t>(c.capacity) * static_cast<size_t>(n));
+        if (st)
+        {
+            const std::string why = c.err;
+            dfree(absmax);
+            if (had > 0 && !dalloc(c, &c.detail, static_cast<size_t>(c.capacity) * static_cast<size_t>(had)))
+            {
+                c.detail_comps = had;
+            }
+            c.err = why;
+        }
+        else
+        {
+            dfree(c.d_absmax);
+            c.d_absmax     = absmax;
+            c.detail_comps = n;
+        }
+        if (c.detail)
+        {
+            cudaMemsetAsync(c.detail, 0, static_cast<size_t>(c.capacity) * static_cast<size_t>(c.detail_comps) * sizeof(double), c.stream);
+        }
+        cudaMemsetAsync(c.exam, 0, static_cast<size_t>(c.g.total_words) * 4, c.stream);
+        return st;
     }
 } // namespace sg
 
@@ -1417,22 +1462,6 @@ extern "C"
                 return from_ctx(c, SG_ERR_CUDA);
             }
             (k < n ? fs : os).push_back(&f->f);
-        }
-        if (n > c.detail_comps)
-        {
-            // one dense detail slab per adapted field; the contents are rebuilt by every pass
-            cudaStreamSynchronize(c.stream);
-            dfree(c.detail);
-            dfree(c.d_absmax);
-            if (dalloc(c, &c.detail, static_cast<size_t>(c.capacity) * static_cast<size_t>(n)) || dalloc(c, &c.d_absmax, static_cast<size_t>(n)))
-            {
-                c.detail_comps = 0;
-                return from_ctx(c, SG_ERR_CUDA);
-            }
-            cudaMemsetAsync(c.detail, 0, static_cast<size_t>(c.capacity) * n * sizeof(double), c.stream);
-            cudaMemsetAsync(c.exam, 0, static_cast<size_t>(c.g.total_words) * 4, c.stream);
-            c.detail_comps = n;
-            sg::clear_graphs(c); // they hold the old detail buffer
         }
         return from_ctx(c, sg::adapt_fields(c, fs, os, eps, regularity, relative_detail != 0, n_harten));
     }

@@ -30,6 +30,7 @@ namespace sg
     }
 
     int graduate(Ctx& c, DeviceMesh& m, DeviceMesh& nm, int* iterations);
+    int ensure_details(Ctx& c, int n);
 
     namespace
     {
@@ -1472,6 +1473,10 @@ namespace sg
             c.err = "harten: ghost widths 1 and 2 are implemented";
             return SG_ERR_ARG;
         }
+        if (int st = ensure_details(c, static_cast<int>(fs.size())))
+        {
+            return st;
+        }
         DeviceMesh& m  = c.m();
         DeviceMesh& nm = c.spare();
         // the pinned inputs staged here were consumed by the previous pass,
@@ -1783,6 +1788,10 @@ namespace sg
             {
                 c.err = "harten: ghost widths 1 and 2 are implemented";
                 return SG_ERR_ARG;
+            }
+            if (int st = ensure_details(c, static_cast<int>(fs.size())))
+            {
+                return st;
             }
             c.rel_detail = relative_detail;
             std::vector<DeviceField*> all(fs);
