@@ -1,17 +1,16 @@
 // Launch-shape autotuner (no samurai counterpart).
 //
-// The level-serial chains of the step are latency-bound and the FP64 list
-// kernels compete for the narrow FP64 pipe, so the best launch shapes depend
-// on the device and on the size of the mesh: the threads per block of the
-// FP64 list kernels, the grid limit of the one-warp-per-word launches, the
-// level sizes up to which a chain (ghost update, tag finalisation, mesh
-// construction) runs its levels in one block, whether the adaptation runs
-// as one graph with conditional nodes or pass by pass, and whether the
-// tag-finalisation chain takes two levels per launch.  sg_autotune times the time
-// step of a given problem under candidate shapes (coordinate descent, each
-// candidate from the same saved state, its graphs captured afresh), keeps the
-// fastest on the mesh and caches it per device and level range; later meshes
-// of the same device and levels start from the cached choice.  Environment
+// The phases of the step are latency-bound on small levels and the FP64 ones
+// compete for the narrow FP64 pipe, so the best launch shapes depend on the
+// device and on the size of the mesh: the threads per block of the FP64
+// phases, the grid limit of the launches, the most words that a phase may walk
+// to share a launch with its neighbours (levels of the ghost update, tag and
+// mesh phases), and whether the adaptation runs as one graph with conditional
+// nodes or pass by pass.  sg_autotune times the time step of a given problem
+// under candidate shapes (coordinate descent, each candidate from the same
+// saved state, its graphs captured afresh), keeps the fastest on the mesh and
+// caches it per device and kind of mesh (levels, periodic axes, stencil
+// radius); later meshes of the kind start from the cached choice.  Environment
 // variables (SG_BLOCK, SG_MAX_BLOCKS, SG_FUSE_WORDS, SG_FUSE_WORDS_FIELD,
 // SG_FUSE_WORDS_MAX, SG_GRAPHED_ADAPT, SG_LEVEL_PAIRS) override
 // both the defaults and the cache.  With
@@ -20,6 +19,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <fstream>
 #include <map>
 #include <mutex>
 #include <string>
@@ -38,12 +38,16 @@ namespace sg
         struct LaunchShape
         {
             int block;
-            long long max_blocks, fuse_mesh, fuse_field, fuse_max;
+            long long max_blocks, fuse_mesh, fuse_field, fuse_max; // limits below 0: the mesh's own
             int graphed;     // the adaptation as one graph with conditional nodes (1) or pass by pass (0)
             int level_pairs; // kept in saved tunings, changes no launch
         };
 
-        using TuneKey = std::tuple<std::string, int, int, int>; // device name, dim, min_level, max_level
+        // device name, dim, min_level, max_level, periodic axes (bit per axis), max_stencil_radius: with periodic axes
+        // levels of the ghost update share chains, without they do not, and the second ghost layer lengthens the
+        // phases.  ANY_MESH in place of the last two: a line from before they were recorded.
+        using TuneKey          = std::tuple<std::string, int, int, int, int, int>;
+        constexpr int ANY_MESH = -1;
 
         std::mutex g_tune_mutex;
         std::map<TuneKey, LaunchShape> g_tune_cache;
@@ -62,8 +66,40 @@ namespace sg
             return n;
         }
 
-        // SG_TUNE_FILE: lines "device dim min max block max_blocks fuse_mesh fuse_field fuse_max graphed level_pairs" (the last line of a
-        // key wins); read once, under the cache mutex
+        // SG_TUNE_FILE (the last line of a key wins; read once, under the cache mutex): lines
+        //   shape2 device dim min max periodic radius block max_blocks fuse_mesh fuse_field fuse_max graphed level_pairs
+        // and, from before the limits counted the words that a phase walks, lines
+        //   device dim min max block max_blocks fuse_mesh fuse_field fuse_max graphed level_pairs
+        // whose limits were words per level: of those, all but the limits applies, to any mesh of the levels.
+        // Other lines are skipped.
+        void read_tune_line(const std::string& line)
+        {
+            char name[256];
+            int dim, lo, hi, per = ANY_MESH, radius = ANY_MESH, block, gr, lp;
+            long long mb, fm, ff, fx;
+            const bool now = std::sscanf(line.c_str(), "shape2 %255s %d %d %d %d %d %d %lld %lld %lld %lld %d %d", name, &dim, &lo, &hi, &per, &radius,
+                                         &block, &mb, &fm, &ff, &fx, &gr, &lp) == 13;
+            if (!now)
+            {
+                if (std::sscanf(line.c_str(), "%255s %d %d %d %d %lld %lld %lld %lld %d %d", name, &dim, &lo, &hi, &block, &mb, &fm, &ff, &fx, &gr, &lp)
+                    != 11)
+                {
+                    return;
+                }
+                per = radius = ANY_MESH;
+            }
+            if (block < 32 || block > 1024 || block % 32 != 0 || mb <= 0 || fm < 0 || ff < 0 || fx < 0 || (gr != 0 && gr != 1) || (lp != 0 && lp != 1)
+                || (now && (per < 0 || radius < 1)))
+            {
+                return;
+            }
+            if (!now)
+            {
+                fm = ff = fx = -1;
+            }
+            g_tune_cache[TuneKey{name, dim, lo, hi, per, radius}] = LaunchShape{block, mb, fm, ff, fx, gr, lp};
+        }
+
         void read_tune_file()
         {
             if (g_tune_file_read)
@@ -76,23 +112,11 @@ namespace sg
             {
                 return;
             }
-            FILE* f = std::fopen(path, "r");
-            if (!f)
+            std::ifstream f(path);
+            for (std::string line; std::getline(f, line);)
             {
-                return;
+                read_tune_line(line);
             }
-            char name[256];
-            int dim, lo, hi, block, gr, lp;
-            long long mb, fm, ff, fx;
-            while (std::fscanf(f, "%255s %d %d %d %d %lld %lld %lld %lld %d %d", name, &dim, &lo, &hi, &block, &mb, &fm, &ff, &fx, &gr, &lp) == 11)
-            {
-                if (block >= 32 && block <= 1024 && block % 32 == 0 && mb > 0 && fm >= 0 && ff >= 0 && fx >= 0 && (gr == 0 || gr == 1)
-                    && (lp == 0 || lp == 1))
-                {
-                    g_tune_cache[TuneKey{name, dim, lo, hi}] = LaunchShape{block, mb, fm, ff, fx, gr, lp};
-                }
-            }
-            std::fclose(f);
         }
 
         void append_tune_file(const TuneKey& k, const LaunchShape& s)
@@ -104,15 +128,15 @@ namespace sg
             }
             if (FILE* f = std::fopen(path, "a"))
             {
-                std::fprintf(f, "%s %d %d %d %d %lld %lld %lld %lld %d %d\n", std::get<0>(k).c_str(), std::get<1>(k), std::get<2>(k), std::get<3>(k),
-                             s.block, s.max_blocks, s.fuse_mesh, s.fuse_field, s.fuse_max, s.graphed, s.level_pairs);
+                std::fprintf(f, "shape2 %s %d %d %d %d %d %d %lld %lld %lld %lld %d %d\n", std::get<0>(k).c_str(), std::get<1>(k), std::get<2>(k),
+                             std::get<3>(k), std::get<4>(k), std::get<5>(k), s.block, s.max_blocks, s.fuse_mesh, s.fuse_field, s.fuse_max, s.graphed, s.level_pairs);
                 std::fclose(f);
             }
         }
 
         TuneKey key_of(const Ctx& c)
         {
-            return TuneKey{device_name(c.device), c.g.dim, c.cfg.min_level, c.cfg.max_level};
+            return TuneKey{device_name(c.device), c.g.dim, c.cfg.min_level, c.cfg.max_level, c.g.periodic, c.cfg.max_stencil_radius};
         }
 
         bool env_set(const char* name)
@@ -137,12 +161,18 @@ namespace sg
         }
     } // namespace
 
-    // the cached shape for this device and level range, where no environment variable sets the value
+    // the cached shape for this device and kind of mesh, where no environment variable sets the value
     void apply_tuned_launch(Ctx& c)
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         read_tune_file();
-        const auto it = g_tune_cache.find(key_of(c));
+        TuneKey key = key_of(c);
+        auto it     = g_tune_cache.find(key);
+        if (it == g_tune_cache.end())
+        {
+            std::get<4>(key) = std::get<5>(key) = ANY_MESH;
+            it                                  = g_tune_cache.find(key);
+        }
         if (it == g_tune_cache.end())
         {
             return;
@@ -156,15 +186,15 @@ namespace sg
         {
             c.max_blocks = s.max_blocks;
         }
-        if (!env_set("SG_FUSE_WORDS"))
+        if (s.fuse_mesh >= 0 && !env_set("SG_FUSE_WORDS"))
         {
             c.fuse_words_mesh = s.fuse_mesh;
         }
-        if (!env_set("SG_FUSE_WORDS_FIELD"))
+        if (s.fuse_field >= 0 && !env_set("SG_FUSE_WORDS_FIELD"))
         {
             c.fuse_words_field = s.fuse_field;
         }
-        if (!env_set("SG_FUSE_WORDS_MAX"))
+        if (s.fuse_max >= 0 && !env_set("SG_FUSE_WORDS_MAX"))
         {
             c.fuse_words_max = s.fuse_max;
         }
