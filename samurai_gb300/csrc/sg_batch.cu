@@ -156,6 +156,13 @@ namespace
         return code;
     }
 
+    // The chain limit of the batch for one instance (own: its saved limits).  Where the launches overlap, levels of
+    // the ghost update keep the instance's own limit: alone they overlap, in a chain they do not.
+    void set_batch_fusion(sg::Ctx& c, const long long* own, long long words)
+    {
+        sg::set_fusion(c, words, c.overlap_launches ? own[1] : words, words);
+    }
+
     // Adapt::operator() (mr/adapt.hpp:147-195) for the instances of thread t,
     // pass by pass in lockstep; n_harten[k] as sg_adapt reports it
     void adapt_share(sg_batch_s& b, int t, const double* eps, const double* regularity, int* n_harten)
@@ -395,7 +402,7 @@ extern "C"
             // waiting blocks of one instance's next launch would hold places that the others' running ones want
             // (48 instances: 1993 us a step without overlap, 2402 with it)
             c.overlap_launches = c.overlap_launches && n < 4;
-            sg::set_fusion(c, sg::BATCH_FUSE_WORDS, sg::BATCH_FUSE_WORDS, sg::BATCH_FUSE_WORDS);
+            set_batch_fusion(c, b->saved_fuse.data() + 5 * k, sg::BATCH_FUSE_WORDS);
         }
         b->n_threads = std::min(n_threads, n);
         if (b->n_threads > 1)
@@ -618,7 +625,7 @@ extern "C"
             {
                 sg::Ctx& c = b->u[k]->mesh->ctx;
                 c.block    = block > 0 ? block : b->saved_blocks[k];
-                sg::set_fusion(c, fuse, fuse, fuse); // drops the captured graphs
+                set_batch_fusion(c, b->saved_fuse.data() + 5 * k, fuse); // drops the captured graphs
             }
             b->fuse_words = fuse;
             b->block      = block;
