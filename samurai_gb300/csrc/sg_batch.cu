@@ -157,10 +157,23 @@ namespace
     }
 
     // The chain limit of the batch for one instance (own: its saved limits).  Where the launches overlap, levels of
-    // the ghost update keep the instance's own limit: alone they overlap, in a chain they do not.
+    // the ghost update keep the instance's own limit: alone they overlap, in a chain they do not (us a step of 2 and 3
+    // instances, chained and alone: 2D levels 3 to 10 410 and 497, 329 and 350; 3D levels 2 to 6 630 and 707, 488 and
+    // 524).  With periodic axes the exchanges between the levels make the chain the faster form (2D levels 3 to 9:
+    // 553 and 577 chained, 602 and 702 with the mesh's own limit).
     void set_batch_fusion(sg::Ctx& c, const long long* own, long long words)
     {
-        sg::set_fusion(c, words, c.overlap_launches ? own[1] : words, words);
+        sg::set_fusion(c, words, c.overlap_launches && !c.g.periodic ? own[1] : words, words);
+    }
+
+    // Up to how many instances the launches of each overlap.  In larger batches the waiting blocks of one instance's
+    // next launch hold places that the others' running ones want.  us a step without and with overlap (ghost levels
+    // chained and alone): 4 instances of 2D levels 3 to 10 434 and 378, 3D 2 to 6 697 and 610; 8 instances 514 and
+    // 516, 859 and 838; 12 instances 765 and 732, 1126 and 1108 (3D 2 to 5 and 2 to 7 1 % slower); 48 instances 2283
+    // and 2343, 3063 and 3248.  With periodic axes, chained both ways, it makes no difference.
+    bool batch_overlaps(const sg::Geom& g, int n)
+    {
+        return n < (g.periodic ? 4 : 12);
     }
 
     // Adapt::operator() (mr/adapt.hpp:147-195) for the instances of thread t,
@@ -399,9 +412,7 @@ extern "C"
             b->saved_fuse.insert(b->saved_fuse.end(), {c.fuse_words_mesh, c.fuse_words_field, c.fuse_words_max, c.chain_blocks, c.overlap_launches ? 1 : 0});
             b->saved_blocks.push_back(c.block);
             c.chain_blocks = std::min(c.chain_blocks, sg::batch_chain_blocks(n));
-            // waiting blocks of one instance's next launch would hold places that the others' running ones want
-            // (48 instances: 1993 us a step without overlap, 2402 with it)
-            c.overlap_launches = c.overlap_launches && n < 4;
+            c.overlap_launches = c.overlap_launches && batch_overlaps(c.g, n);
             set_batch_fusion(c, b->saved_fuse.data() + 5 * k, sg::BATCH_FUSE_WORDS);
         }
         b->n_threads = std::min(n_threads, n);
