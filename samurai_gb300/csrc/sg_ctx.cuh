@@ -188,7 +188,7 @@ namespace sg
         long long capacity  = 0;       // dense elements per field (32 * total_words)
         bool use_graphs     = true;    // replay captured launch sequences
         unsigned long long mesh_version = 1; // bumped at every change of the current mesh
-        long long max_blocks = 152LL * 8; // grid limit of the one-warp-per-word launches, in blocks of 8 warps (x4 for one thread per word)
+        long long max_blocks = 152LL * 8; // grid limit of the launches that hand out cells, in blocks of 256 threads (x4 for one thread per word)
         int block            = 256;       // threads per block of the FP64 list kernels
         bool overlap_launches      = true; // phases as programmatic dependents of each other
         int chain_blocks           = 0; // blocks of the cluster that runs a chain of phases (0: no chains)
@@ -301,9 +301,14 @@ namespace sg
     constexpr long long FUSE_WORDS       = 16384;
     constexpr long long FUSE_WORDS_FIELD = 5000; // with periodic axes; 0 otherwise (2D levels 2 to 8: 217 us a step, 256 in chains)
     constexpr long long FUSE_WORDS_MAX   = 12288;
+    // All kinds of phases in batched mode (levels of the ghost update where launches do not overlap or exchanges stand
+    // between them).  us a step of 48 instances with limits of 0, 2500, 10000, 30000 and 100000 words: 2D levels 3 to
+    // 10 2774, 2452, 2288, 2256, 2694; the same range periodic to 9 4098, 2565, 2225, 2367, 2335; 3D 2 to 6 3430, 3412,
+    // 3078, 3089, 3786.
     constexpr long long BATCH_FUSE_WORDS = 10000;
-    // Smaller clusters in batched mode, where many meshes share the chip: 48 meshes of max_level 7..10 take
-    // 1969 us a step with 8 blocks, 1938 with 4, 2057 with 2 (1815 and 1610 with 8 and 4 on 32 hardware queues).
+    // Smaller clusters in batched mode, where many meshes share the chip.  us a step with 16, 8 and 4 blocks, 2D levels
+    // 3 to 10 (3D 2 to 7): 4 instances 372, 370, 376 (765, 776, 775), 12 instances 796, 766, 783 (1816, 1756, 1749),
+    // 16 instances 975, 892, 895 (2337, 2208, 2171), 48 instances 2741, 2401, 2287 (6307, 5885, 5721).
     inline int batch_chain_blocks(int n)
     {
         return n >= 16 ? 4 : (n >= 4 ? 8 : 16);

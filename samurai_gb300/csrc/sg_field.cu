@@ -129,9 +129,8 @@ namespace sg
                           [&](long long w, int b, const Cell& c, int) { predict_transpose<DIM>(g, u, 32 * w + b, l, c.x, c.y, c.z, order); });
         }
 
-        // update_fields (algorithm/update_fields.hpp:27-127): copy on
-        // reference ∩ new cells, projection on coarsened cells, prediction on
-        // refined cells; every other reference entry of the new field is 0.
+        // the transpose of update_fields (op_update_fields): every reference entry of the new field hands its adjoint
+        // to what it was copied, projected or predicted from
         template <int DIM, class A>
         __global__ void k_update_fields_reverse(const __grid_constant__ Geom gp, int order, const int* wl, const long long* lo, const uint32_t* nref,
                                         const uint32_t* ncells, const uint32_t* oref, const uint32_t* ocells, const uint32_t* ohc, A uo, A un)
@@ -169,10 +168,6 @@ namespace sg
         }
 
         // -------------------------------------------------------- upwind
-        // unp1 = u - dt * upwind(a, u) (stencil_field.hpp:38-44, 91-97;
-        // demos/FiniteVolume/advection_2d.cpp:144) or the README lambda
-        // (README.md:144-153).  Neighbours at the same level are reference
-        // cells, at fixed offsets in the dense slabs.
         // 2^l as a double from its exponent bits (no FP64 instruction)
         __device__ __forceinline__ double pow2(int l)
         {
@@ -636,7 +631,6 @@ namespace sg
 
     namespace
     {
-        // one warp per word of levels l0..l1, at most the mesh's block limit
         // blocks of c.block threads: one warp per word of levels l0..l1, at most
         // max_blocks blocks of 8 warps' worth of warps
         int blocks_words(const Ctx& c, int l0, int l1)

@@ -1535,7 +1535,7 @@ namespace sg
         {
             // The field phases over all levels stay behind a full boundary: their waiting blocks would hold the
             // shared memory and registers that the launch before them still wants (three components, 2D levels 3
-            // to 9, relative details: 303 us a step without them, 375 with them overlapped too).
+            // to 9, relative details: 379 us a step without them, 470 with them overlapped too).
             constexpr bool overlap = OP != OP_DETAIL && OP != OP_UPDATE_FIELDS && OP != OP_ABSMAX && OP != OP_ABSMAX_INIT;
             launch_dependent(c, overlap, k_phase<DIM, OP>, grid, block, 1, e, p);
         }
@@ -1612,8 +1612,9 @@ namespace sg
         // between two nodes and most of the rest launch, cold instructions and
         // ramp-up; a cluster barrier takes 0.25 us (16 blocks of 512 threads),
         // a barrier over the whole grid 1.3 us.  Levels of the ghost update chain
-        // only where periodic exchanges stand between them: as overlapping launches
-        // of their own they take less (2D levels 2 to 8: 256 -> 217 us a step).  A cluster barrier that has to
+        // only where periodic exchanges stand between them, or in batches whose
+        // launches do not overlap: as overlapping launches of their own they take
+        // less (2D levels 2 to 8: 256 -> 217 us a step).  A cluster barrier that has to
         // wait for the blocks' stores takes 0.8 us, though, and every load after it
         // comes from L2 (0.2 us).  With periodic axes the exchanges between the
         // levels double the phases, most of them nearly empty: there the phases of
@@ -1693,7 +1694,7 @@ namespace sg
         {
             WORDS, // a thread per bitmap word
             LIST,  // a thread per reference word
-            ITEMS, // a warp per listed word
+            ITEMS, // blocks that hand out the cells of their words
             SCAN,
             OTHER
         };
@@ -1772,7 +1773,7 @@ namespace sg
                 {
                     words = phase_words(g, p);
                 }
-                // the comparison's blocks sign off one by one at a counter (level 9 in 3D: 4864 of them took 27 us, 608 take 10)
+                // the comparison's blocks sign off one by one at a counter (level 9 in 3D: 4864 of them took 27 us, 609 take 14)
                 grid = std::min((p.op == OP_COMPARE ? c.max_blocks / 2 + 1 : 4LL * c.max_blocks), (words + block - 1) / block);
                 break;
             }

@@ -12,11 +12,7 @@ namespace sg
     // non-empty words of a superset (reference or leaf cells) in
     // ascending order; word_of(w) narrows it to the subset a kernel acts
     // on.  Consecutive cells of a word are consecutive doubles, so every
-    // field access of a warp is one 256-byte segment.  A null list means
-    // every word of [begin, end): the dense range of small levels, which
-    // a launch covers with one warp per word without loading the list
-    // or its offsets (two dependent loads fewer at the head of the
-    // launch; word_of is zero on the words the list leaves out).
+    // field access of a warp is one 256-byte segment.
     template <class WordF, class CellF>
     __device__ __forceinline__ void warp_list(const int* list, long long begin, long long end, long long warp0, long long nwarps, WordF word_of,
                                               CellF cell)
@@ -24,7 +20,7 @@ namespace sg
         const int lane = threadIdx.x & 31;
         for (long long i = begin + warp0; i < end; i += nwarps)
         {
-            const long long w = list ? list[i] : i;
+            const long long w = list[i];
             const uint32_t v  = word_of(w);
             if ((v >> lane) & 1u)
             {
