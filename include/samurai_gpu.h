@@ -112,21 +112,25 @@ int sg_mesh_set_adapt_graph(sg_mesh_t mesh, int enable);
 
 /* Without a samurai counterpart: the launch-shape autotuner.  Times sg_step(u, unp1, eps, regularity, a, dt, scheme)
  * over `steps` steps from the problem's current state under candidate launch shapes (threads per block of the FP64
- * list kernels, grid limit of the word launches, level sizes up to which the ghost-update and tag-finalisation
- * chains run in one block, the adaptation path of sg_mesh_set_adapt_graph, two levels per launch in the
- * tag-finalisation chain), each step after an untimed 256 MiB
+ * phases, grid limit of the launches, the most words that a level of the ghost update or of the tag finalisation may
+ * walk to share a launch with its neighbours, the adaptation path of sg_mesh_set_adapt_graph), each step after an
+ * untimed 256 MiB
  * write that empties the L2 (a scratch array held during the call), keeps the fastest on the mesh and caches it for
- * this device and level range (later meshes start from it; SG_TUNE_FILE names a file that keeps the cache across
- * processes; the SG_BLOCK, SG_MAX_BLOCKS, SG_FUSE_WORDS*, SG_GRAPHED_ADAPT, SG_LEVEL_PAIRS environment variables
- * override it).  The
- * problem is left in the state it had.  default_ms / tuned_ms receive the step time under the starting and the
+ * this device and kind of mesh: dimension, levels, periodic axes and stencil radius (later meshes of the kind start
+ * from it; SG_TUNE_FILE names a file that keeps the cache across processes).  The SG_BLOCK, SG_MAX_BLOCKS,
+ * SG_FUSE_WORDS (mesh and tag phases over all levels), SG_FUSE_WORDS_FIELD (levels of the ghost update),
+ * SG_FUSE_WORDS_MAX (levels of the tag finalisation) and SG_GRAPHED_ADAPT environment variables override it, read
+ * when a mesh is created.  Two more are read there and not tuned: SG_CHAIN_BLOCKS, the most blocks of the cluster
+ * that runs phases sharing a launch (default 16, as the device grants; 0: every phase launches alone), and
+ * SG_OVERLAP_LAUNCHES (default 1; 0: no launch begins before the one it follows has ended).  None changes a result.
+ * The problem is left in the state it had.  default_ms / tuned_ms receive the step time under the starting and the
  * chosen shape. */
 int sg_autotune(sg_field_t u, sg_field_t unp1, double eps, double regularity, const double* a, double dt, int scheme, int steps,
                 double* default_ms, double* tuned_ms);
-/* the mesh's launch shape: threads per block, grid limit (blocks of 8 warps), chain limits in words per
- * level of the mesh, field and tag-finalisation chains, 1 when the adaptation runs as one graph with conditional
- * nodes (0: pass by pass), level_pairs is kept for callers and saved
- * tunings and changes no launch; a chain limit is the most words a phase may walk to share a launch; any pointer may be NULL */
+/* the mesh's launch shape: threads per block, grid limit (blocks of 8 warps), chain limits (the most words a phase may
+ * walk to share a launch) of the mesh, field and tag-finalisation phases, 1 when the adaptation runs as one graph with
+ * conditional nodes (0: pass by pass); level_pairs (SG_LEVEL_PAIRS) is kept for callers and saved tunings and changes
+ * no launch; any pointer may be NULL */
 int sg_launch_shape(sg_mesh_t mesh, int* block, long long* max_blocks, long long* fuse_mesh_words, long long* fuse_field_words,
                     long long* fuse_max_words, int* graphed_adapt, int* level_pairs);
 
@@ -196,7 +200,9 @@ int sg_upwind(sg_field_t u, sg_field_t unp1, const double* a, double dt, int sch
    the four calls; the whole step is one captured CUDA graph (passes and buffers decided on the device) with one host
    synchronisation.  n_harten receives the adaptation's Harten passes. */
 int sg_step(sg_field_t u, sg_field_t unp1, double eps, double regularity, const double* a, double dt, int scheme, int* n_harten);
-/* detail and tag fields of the last Harten pass, reference numbering (n = nb_reference) */
+/* detail and tag fields of the last Harten pass, reference numbering of the current mesh (n = nb_reference).  After a
+ * pass that changed the mesh a cell reads what the last pass that had it in its reference mesh found: the detail 0
+ * where that pass examined no parent of it, and 0 where no pass ever had the cell. */
 int sg_detail_download(sg_field_t u, double* values, long long n);
 int sg_tag_download(sg_field_t u, unsigned char* values, long long n);
 
@@ -285,14 +291,15 @@ int sg_batch_step(sg_batch_t batch, const double* eps, const double* regularity,
 int sg_batch_synchronize(sg_batch_t batch);
 
 /* Without a samurai counterpart: the batch's launch-shape autotuner.  Times `steps` batched steps (sg_batch_step)
- * from the instances' current state under candidate shapes (the level size, in words, up to which every instance's
- * ghost-update, tag-finalisation and mesh chains run their levels in one block; the threads per block of their FP64
- * list kernels), each from the same saved state and each step after an untimed 256 MiB write that empties the L2;
+ * from the instances' current state under candidate shapes (the most words that a phase of any instance may walk to
+ * share a launch; the threads per block of their FP64 phases), each from the same saved state and each step after an untimed 256 MiB write that empties the L2;
  * keeps the fastest and leaves every instance's mesh and values as they were.  default_ms / tuned_ms receive the
  * batched step time under the starting and the chosen shape. */
 int sg_batch_autotune(sg_batch_t batch, const double* eps, const double* regularity, const double* a, const double* dt, int scheme,
                       int steps, double* default_ms, double* tuned_ms);
-/* the batch's launch shape: chain limit in words per level, threads per block (0: each instance's own) */
+/* the batch's launch shape: chain limit in words a phase walks (where the instances' launches overlap, batches of fewer
+ * than 12 without periodic axes, levels of the ghost update keep each instance's own), threads per block (0: each
+ * instance's own) */
 int sg_batch_launch_shape(sg_batch_t batch, long long* fuse_words, int* block);
 
 /* Discrete adjoint of the time loop (no counterpart in samurai, which has no derivatives).  The loop of
