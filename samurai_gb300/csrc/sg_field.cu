@@ -1145,6 +1145,13 @@ namespace sg
             }
         }
 
+        // threads per block of the transposed launches, whose linear forms take up to 96 (2D) and 255 (3D) registers:
+        // 65536 registers of an SM hold no larger block
+        int reverse_block(const Ctx& c)
+        {
+            return std::min(c.block, c.g.dim == 3 ? 256 : 512);
+        }
+
         // the same transposed, launch by launch in forward order (run_reversed turns the captured chain round)
         template <int DIM>
         int ghost_reverse_launches(Ctx& c, const DeviceMesh& dm, double* lam, int* overflow, bool has_bc)
@@ -1152,26 +1159,27 @@ namespace sg
             const Geom& g    = c.g;
             const MeshPtrs m = mesh_ptrs(dm);
             const RevAcc<FormCap<DIM>::value> u{lam, lam, overflow, 1};
-            const int lmin = g.min_level >= 2 ? g.min_level - 2 : 0;
+            const int lmin  = g.min_level >= 2 ? g.min_level - 2 : 0;
+            const int block = reverse_block(c);
             for (int l = g.max_level; l >= lmin; --l)
             {
-                const int nb = static_cast<int>(std::min(16384LL, (boundary_count<DIM>(g, l) + c.block - 1) / c.block));
+                const int nb = static_cast<int>(std::min(16384LL, (boundary_count<DIM>(g, l) + block - 1) / block));
                 const int np = l > lmin ? blocks_words(c, l - 1, l - 1) : 0;
                 if (nb + np > 0)
                 {
-                    k_ghost_reverse<DIM><<<nb + np, c.block, 0, c.stream>>>(c.g, l, 1, nb, has_bc ? 1 : 0, m, u);
+                    k_ghost_reverse<DIM><<<nb + np, block, 0, c.stream>>>(c.g, l, 1, nb, has_bc ? 1 : 0, m, u);
                     launched(c, "ghost_level");
                 }
                 if (l >= g.min_level)
                 {
-                    const int ncb = static_cast<int>(std::min(16384LL, (corner_count<DIM>(g, l) + c.block - 1) / c.block));
-                    k_ghost_reverse<DIM><<<ncb, c.block, 0, c.stream>>>(c.g, l, 2, ncb, has_bc ? 1 : 0, m, u);
+                    const int ncb = static_cast<int>(std::min(16384LL, (corner_count<DIM>(g, l) + block - 1) / block));
+                    k_ghost_reverse<DIM><<<ncb, block, 0, c.stream>>>(c.g, l, 2, ncb, has_bc ? 1 : 0, m, u);
                     launched(c, "ghost_corner_projection");
                 }
             }
             for (int l = std::max(lmin, 1); l <= g.max_level; ++l)
             {
-                k_predict_reverse<DIM><<<blocks_words(c, l, l), c.block, 0, c.stream>>>(c.g, l, c.cfg.prediction_radius, m, u);
+                k_predict_reverse<DIM><<<blocks_words(c, l, l), block, 0, c.stream>>>(c.g, l, c.cfg.prediction_radius, m, u);
                 launched(c, "predict");
             }
             return check(c, "update_ghost_mr (transpose)");
@@ -1640,13 +1648,13 @@ namespace sg
         if (c.g.dim == 2)
         {
             const RevAcc<FormCap<2>::value> r{lam_new, lam_old, overflow, 0};
-            k_update_fields_reverse<2><<<blocks_words(c, 0, c.g.nlev - 1), c.block, 0, c.stream>>>(c.g, c.cfg.prediction_radius, nm.wl_ref, nm.d_lo, nm.ref,
+            k_update_fields_reverse<2><<<blocks_words(c, 0, c.g.nlev - 1), reverse_block(c), 0, c.stream>>>(c.g, c.cfg.prediction_radius, nm.wl_ref, nm.d_lo, nm.ref,
                                                                                               nm.cells, m.ref, m.cells, m.hc, r, r);
         }
         else
         {
             const RevAcc<FormCap<3>::value> r{lam_new, lam_old, overflow, 0};
-            k_update_fields_reverse<3><<<blocks_words(c, 0, c.g.nlev - 1), c.block, 0, c.stream>>>(c.g, c.cfg.prediction_radius, nm.wl_ref, nm.d_lo, nm.ref,
+            k_update_fields_reverse<3><<<blocks_words(c, 0, c.g.nlev - 1), reverse_block(c), 0, c.stream>>>(c.g, c.cfg.prediction_radius, nm.wl_ref, nm.d_lo, nm.ref,
                                                                                               nm.cells, m.ref, m.cells, m.hc, r, r);
         }
         launched(c, "update_fields");
