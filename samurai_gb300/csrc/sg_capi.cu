@@ -497,7 +497,11 @@ extern "C"
         }
         sg::apply_tuned_launch(c); // the autotuner's choice for this device and level range, unless overridden above
         c.overlap_launches         = tuned("SG_OVERLAP_LAUNCHES", 1) != 0;
-        c.chain_blocks             = static_cast<int>(std::min<long long>(sg::chain_blocks(c.g), tuned("SG_CHAIN_BLOCKS", 16)));
+        c.chain_blocks             = sg::chain_blocks(c.g);
+        for (const long long most = tuned("SG_CHAIN_BLOCKS", 16); c.chain_blocks > most;)
+        {
+            c.chain_blocks /= 2; // cluster sizes were asked for in powers of two
+        }
         if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess)
         {
             cudaGetLastError();

@@ -1830,6 +1830,7 @@ namespace sg
     {
         const void* k = reinterpret_cast<const void*>(chain_kernel(g));
         const bool big = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        cudaGetLastError();
         for (int n = big ? 16 : 8; n >= 2; n /= 2)
         {
             cudaLaunchConfig_t cfg{};

@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 
 FORMS = {
     "alone": {"SG_CHAIN_BLOCKS": "0"},
+    "one block": {"SG_CHAIN_BLOCKS": "1"},
     "two blocks": {"SG_CHAIN_BLOCKS": "2"},
+    "at most twelve blocks": {"SG_CHAIN_BLOCKS": "12"},
     "all chained": {"SG_CHAIN_BLOCKS": "16", "SG_FUSE_WORDS": "1000000", "SG_FUSE_WORDS_FIELD": "1000000", "SG_FUSE_WORDS_MAX": "1000000"},
     "levels alone": {"SG_FUSE_WORDS_FIELD": "0"},
     "odd blocks": {"SG_BLOCK": "96", "SG_MAX_BLOCKS": "3"},
